@@ -186,7 +186,8 @@ struct sde_batch {
     std::vector<float *> psf, image;
     float *d_peak = nullptr;                   // PSF peak per plan
     BatchPlan *d_plans = nullptr;
-    int64_t *d_item_start = nullptr;
+    BatchItem *d_items = nullptr;  // launch list
+    int64_t nitems = 0;
     unsigned long long *d_counter = nullptr;
     FinalizeDesc *d_fin = nullptr;
     uint16_t *d_fin_blk = nullptr;             // grid of each block of the flattened finalize
@@ -249,7 +250,7 @@ int batch_grid(sde_batch *b, int psf) {
     SDE_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), ctx->stream));
     SDE_CUDA_TRY(cudaMemsetAsync(b->raw[0], 0, b->lo_clean ? b->hi_bytes : b->raw_bytes, ctx->stream));
     b->lo_clean = false;
-    SDE_TRY(launch_grid_batch(ctx, psf, b->comp, b->d_plans, b->d_item_start, b->n, b->d_counter,
+    SDE_TRY(launch_grid_batch(ctx, psf, b->comp, b->d_plans, b->d_items, b->nitems, b->d_counter,
                               ctx->d_cft, ctx->num_sms * grid_ctas_per_sm()));
     if (b->comp) {
         SDE_TRY(launch_fold_lo_batch(ctx, b->d_plans, b->d_fold, b->fold_n));
@@ -343,9 +344,9 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
     b->comp = ctx->compensated;
     int rc = SDE_OK;
     std::vector<BatchPlan> hp(n);
-    std::vector<int64_t> start(n + 1, 0);
     std::vector<FinalizeDesc> hf(n);
     std::vector<size_t> raw_off(n), img_off(n);
+    int64_t set_vis = 0;
     size_t raw_total = 0, img_total = 0;  // raw_total: the hi planes (the grids have the same layout)
     for (int i = 0; i < n; i++) {
         sde_plan *pl = plans[i];
@@ -383,7 +384,7 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
         img_off[i] = img_total;
         img_total += ((size_t)nx[i] * ny[i] * 4 + 255) & ~(size_t)255;
         b->max_cells = std::max<int64_t>(b->max_cells, (int64_t)cells);
-        start[i + 1] = start[i] + pl->nitems;
+        set_vis += pl->nvis_in;
         b->classes[std::make_tuple(fnu, nv, nx[i], ny[i], pl->pitch)].push_back(i);
     }
     char *rawmem = nullptr, *gridmem = nullptr, *imgmem = nullptr;
@@ -397,7 +398,6 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
     B_TRY(batch_alloc(b, (void **)&imgmem, 2 * img_total));
     B_TRY(batch_alloc(b, (void **)&b->d_peak, sizeof(float) * n));
     B_TRY(batch_alloc(b, (void **)&b->d_plans, sizeof(BatchPlan) * n));
-    B_TRY(batch_alloc(b, (void **)&b->d_item_start, sizeof(int64_t) * (n + 1)));
     B_TRY(batch_alloc(b, (void **)&b->d_counter, sizeof(unsigned long long)));
     B_TRY(batch_alloc(b, (void **)&b->d_fin, sizeof(FinalizeDesc) * n));
     for (int i = 0; i < n; i++)
@@ -435,6 +435,28 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
         }
         cudaStream_t st = ctx->stream;
         cudaError_t e = cudaSuccess;
+        // the launch list: the plans' items (read back once), dealt out in parts where the
+        // whole set has too few for the teams
+        std::vector<BatchItem> list;
+        std::vector<WorkItem> items;
+        const int part = part_size(set_vis);
+        for (int i = 0; i < n && e == cudaSuccess; i++) {
+            const sde_plan *pl = b->plans[i];
+            items.resize((size_t)pl->nitems);
+            if (items.empty()) continue;
+            e = cudaMemcpyAsync(items.data(), pl->items, sizeof(WorkItem) * items.size(), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) break;
+            for (WorkItem it : items) {
+                it.rstep = item_parts(it, part);
+                for (it.r0 = 0; it.r0 < it.rstep; it.r0++) list.push_back(BatchItem{it, i});
+            }
+        }
+        b->nitems = (int64_t)list.size();
+        if (e == cudaSuccess) {
+            rc = batch_alloc(b, (void **)&b->d_items, sizeof(BatchItem) * std::max<size_t>(list.size(), 1));
+            if (rc != SDE_OK) goto fail;
+        }
         // the (plan, core) pairs to fold: the plans' marked cores (read back once)
         std::vector<int2> fold;
         if (b->comp) {
@@ -462,7 +484,7 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
             e = cudaMemcpyAsync(b->d_fold, fold.data(), sizeof(int2) * fold.size(), cudaMemcpyHostToDevice, st);
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_plans, hp.data(), sizeof(BatchPlan) * n, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_item_start, start.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_items, list.data(), sizeof(BatchItem) * list.size(), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_fin, hf.data(), sizeof(FinalizeDesc) * n, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess && !fblk.empty())
             e = cudaMemcpyAsync(b->d_fin_blk, fblk.data(), sizeof(uint16_t) * fblk.size(), cudaMemcpyHostToDevice, st);

@@ -103,12 +103,36 @@ inline size_t exc_wt_off(size_t ne) { return (sizeof(DegridExc) * ne + 15) & ~(s
 inline size_t exc_rot_off(size_t ne) { return (exc_wt_off(ne) + 4 * ne + 15) & ~(size_t)15; }
 inline size_t exc_bytes(size_t ne) { return exc_rot_off(ne) + 8 * ne; }
 
-struct WorkItem {
+struct __align__(16) WorkItem {
     int32_t tile;      // tile id = tv * ntu + tu
     int32_t cbeg, cend;  // chunk range
     int32_t vbeg, vend;  // sorted visibility range
     int32_t dense;     // 1: the item's tile holds >= DENSE_TILE_VIS visibilities
+    // the rounds (of ROUND_CHUNKS chunks, one per 4-lane group of a team) that are taken:
+    // r0, r0 + rstep, ...  An item of a plan has all of them (0, 1); the launch list holds
+    // an item once, or several times with its rounds dealt out (item_parts).
+    int32_t r0, rstep;
 };
+constexpr int ROUND_CHUNKS = 64;
+// Visibilities of a launch-list entry: the power of two at or below nvis / 512, so that the
+// 456 teams of 152 SMs have about an entry each, from PART_MIN (below it an entry's tile load
+// or flush, a few us, outweighs its visibilities) to ITEM_MAX (above it there are items to
+// spare, and fewer entries flush less often).  Measured with items cut at these sizes, grid +
+// degrid us at 256 / 2048 / 8192 / 16384 visibilities: 84 240 visibilities on 512^2 39 / 75 /
+// 127 / 155; 1 347 840 on 1024^2 215 / 111 / 160 / 208; 8 087 040 on 2048^2 - / 350 / 324 /
+// 348; 16 174 080 on 4096^2 - / 681 / 588 / 569.
+constexpr int PART_MIN = 256;
+inline int part_size(int64_t nvis) {
+    int m = PART_MIN;
+    while (m < ITEM_MAX && (int64_t)m * 2 * 512 <= nvis) m *= 2;
+    return m;
+}
+// Entries of one item: ceil(visibilities / part), at most one per round.
+__host__ __device__ inline int item_parts(const WorkItem &it, int part) {
+    const int rounds = (it.cend - it.cbeg + ROUND_CHUNKS - 1) / ROUND_CHUNKS;
+    const int want = (it.vend - it.vbeg + part - 1) / part;
+    return want < rounds ? want : rounds;
+}
 // A tile this full has many work items, so its cells receive long sums across items: those
 // sums are the ones compensated (sde_ctx_set_compensated).
 constexpr int DENSE_TILE_VIS = 65536;
@@ -205,6 +229,9 @@ struct sde_plan {
     uint8_t *gconj = nullptr; // gridding-frame conjugation flag, sorted
     uint2 *chunks = nullptr;  // {first vis, cell | len << 16}
     WorkItem *items = nullptr;
+    WorkItem *parts = nullptr;  // launch list of the gridder and degridder (item_parts)
+    int64_t parts_max = 0;      // entries it has room for; their count is at nparts
+    unsigned long long *nparts = nullptr;  // after the entries, in the same allocation
     DegridExc *exc = nullptr; // exception list (includes degrid-only visibilities)
     float *wt_all = nullptr;  // caller-order weights (for user-frame degridding)
     uint8_t *core_lo = nullptr;  // (ntu+1) x (ntv+1) raw-grid cores where the compensation
@@ -249,6 +276,11 @@ struct BatchPlan {
     float2 *raw_lo;  // NULL: plain FP32 sums across items
     int pitch, ntu, nu, nv;
 };
+// A launch-list entry of a batch.
+struct __align__(16) BatchItem {
+    WorkItem it;
+    int plan;
+};
 // One grid of a batched finalize (Hermitian fold, shift by SUPP, GRDH2D normalisation).
 struct FinalizeDesc {
     const float2 *raw;
@@ -275,7 +307,7 @@ int grid_ctas_per_sm();  // resident persistent gridding CTAs per SM
 int encode_tmap_f32_2d(CUtensorMap *map, const void *base, uint64_t width, uint64_t rows,
                        uint64_t row_bytes, uint32_t box_w, uint32_t box_h);
 int launch_grid_batch(sde_ctx *ctx, int psf, int comp, const BatchPlan *d_plans,
-                      const int64_t *d_item_start, int nplans, unsigned long long *d_counter,
+                      const BatchItem *d_items, int64_t nitems, unsigned long long *d_counter,
                       const float *cft, int nctas);
 // finalize of n grids in one flattened launch: blk[b] = the grid of block b (nblk blocks)
 int launch_finalize_batch(sde_ctx *ctx, const FinalizeDesc *d_desc, const uint16_t *blk, int64_t nblk);

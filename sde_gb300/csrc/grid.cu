@@ -1,7 +1,8 @@
 // grid.cu -- tiled gridding (GRDH2D) and degridding (GRDDEH2D) over a sde_plan.
 //
 // Both kernels are persistent: one CTA per SM of TEAMS teams of 256 threads; a team takes
-// work items (<= ITEM_MAX visibilities of one 64x64-cell tile) from an atomic counter.
+// work items (<= ITEM_MAX visibilities of one 64x64-cell tile), or parts of them where there
+// are too few for the teams (item_parts), from an atomic counter.
 //
 // Gridding: a team keeps its item's tile plus a 3-cell halo in shared memory.  A 4-lane
 // group owns a chunk (<= CHUNK_MAX visibilities of one cell pair) and accumulates the
@@ -52,6 +53,7 @@ constexpr int TEAM_THREADS = 256;
 constexpr int GRID_THREADS = TEAMS * TEAM_THREADS;
 constexpr int GLANES = 4;                          // lanes per chunk
 constexpr int GGROUPS = TEAM_THREADS / GLANES;     // chunks in flight per team
+static_assert(GGROUPS == ROUND_CHUNKS, "a round of the launch list");
 constexpr int VT_ROW = 32;                         // floats per v-table row (4 copies x 8)
 static_assert(VT_ROW * 4 == TAPROW_BYTES, "the plan record's v-table offsets");
 constexpr int VT_FLOATS = 129 * VT_ROW;
@@ -109,7 +111,7 @@ __device__ __forceinline__ void grid_item(const WorkItem &it, const uint2 *__res
     const float *ucopy = ut + (grp & 3) * 8 + 2 * q;
     constexpr uint32_t FULL = 0xffffffffu;
     const int rounds = (it.cend - it.cbeg + GGROUPS - 1) / GGROUPS;
-    for (int rr = 0; rr < rounds; rr++) {
+    for (int rr = it.r0; rr < rounds; rr += it.rstep) {
         const int c = it.cbeg + rr * GGROUPS + grp;
         const bool live = c < it.cend;
         const uint2 ch = live ? chunks[c] : make_uint2(0u, 0u);
@@ -225,14 +227,50 @@ __device__ __forceinline__ void grid_item(const WorkItem &it, const uint2 *__res
     }
 }
 
-// Persistent gridding of one plan: every team takes work items from an atomic counter
-// until the list is exhausted.
+// Persistent gridding of one plan: every team takes entries of the plan's launch list (work
+// items, or parts of them) from an atomic counter until the list is exhausted.
 template <bool PSF, bool COMP>
 __global__ void __launch_bounds__(GRID_THREADS, 1)
-    k_grid(const WorkItem *__restrict__ items, int64_t nitems, unsigned long long *counter,
+    k_grid(const WorkItem *__restrict__ items, const unsigned long long *nitems_dev, unsigned long long *counter,
            const uint2 *__restrict__ chunks, const float4 *__restrict__ rec,
            const float *__restrict__ cft_g, float2 *raw, float2 *raw_lo, int pitch, int ntu, int nu,
            int nv) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float *vt = reinterpret_cast<float *>(smem_raw);
+    float *ut = vt + VT_FLOATS;
+    const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x % TEAM_THREADS;
+    float *tre = ut + UT_FLOATS + team * GTILE_FLOATS;
+    float *tim = tre + STILE * STILE;
+    __shared__ long long s_next[TEAMS];
+    for (int k = tid; k < STILE * STILE; k += TEAM_THREADS) {
+        tre[k] = 0.f;
+        tim[k] = 0.f;
+    }
+    fill_tap_tables(cft_g, vt, ut);
+    const long long nitems = (long long)*nitems_dev;
+    __syncthreads();
+    for (;;) {
+        if (tid == 0) s_next[team] = (long long)atomicAdd(counter, 1ull);
+        team_sync(team);
+        const long long n = s_next[team];
+        if (n >= nitems) break;
+        const WorkItem it = items[n];
+        if (tid == 0 && it.r0 == 0) {
+            // the item's chunk list and records stream into L2 while the first chunks run
+            prefetch_l2_range(chunks, it.cbeg, it.cend, 8);
+            prefetch_l2_range(rec, it.vbeg, it.vend, 16);
+        }
+        grid_item<PSF, COMP>(it, chunks, rec, vt, ut, tre, tim, raw, raw_lo, pitch, ntu, nu, nv, tid, team);
+        team_sync(team);
+    }
+}
+
+// Persistent gridding of many plans (a mosaic's pointings, a batch of served jobs): the
+// same, over the launch list of all plans.  One launch grids every plan.
+template <bool PSF, bool COMP>
+__global__ void __launch_bounds__(GRID_THREADS, 1)
+    k_grid_batch(const BatchPlan *__restrict__ plans, const BatchItem *__restrict__ items,
+                 int64_t nitems, unsigned long long *counter, const float *__restrict__ cft_g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *vt = reinterpret_cast<float *>(smem_raw);
     float *ut = vt + VT_FLOATS;
@@ -251,54 +289,9 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
         team_sync(team);
         const long long n = s_next[team];
         if (n >= nitems) break;
-        const WorkItem it = items[n];
-        if (tid == 0) {
-            // the item's chunk list and records stream into L2 while the first chunks run
-            prefetch_l2_range(chunks, it.cbeg, it.cend, 8);
-            prefetch_l2_range(rec, it.vbeg, it.vend, 16);
-        }
-        grid_item<PSF, COMP>(it, chunks, rec, vt, ut, tre, tim, raw, raw_lo, pitch, ntu, nu, nv, tid, team);
-        team_sync(team);
-    }
-}
-
-// Persistent gridding of many plans (a mosaic's pointings, a batch of served jobs): the
-// same, over the combined work-item list of all plans (item_start[p] = first combined index
-// of plan p).  One launch grids every plan.
-template <bool PSF, bool COMP>
-__global__ void __launch_bounds__(GRID_THREADS, 1)
-    k_grid_batch(const BatchPlan *__restrict__ plans, const int64_t *__restrict__ item_start,
-                 int nplans, unsigned long long *counter, const float *__restrict__ cft_g) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float *vt = reinterpret_cast<float *>(smem_raw);
-    float *ut = vt + VT_FLOATS;
-    const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x % TEAM_THREADS;
-    float *tre = ut + UT_FLOATS + team * GTILE_FLOATS;
-    float *tim = tre + STILE * STILE;
-    __shared__ long long s_next[TEAMS];
-    __shared__ int s_plan[TEAMS];
-    for (int k = tid; k < STILE * STILE; k += TEAM_THREADS) {
-        tre[k] = 0.f;
-        tim[k] = 0.f;
-    }
-    fill_tap_tables(cft_g, vt, ut);
-    __syncthreads();
-    const int64_t total = item_start[nplans];
-    for (;;) {
-        if (tid == 0) {
-            const long long n = (long long)atomicAdd(counter, 1ull);
-            int p = 0;
-            if (n < total)
-                while (p + 1 < nplans && item_start[p + 1] <= n) p++;
-            s_next[team] = n;
-            s_plan[team] = p;
-        }
-        team_sync(team);
-        const long long n = s_next[team];
-        if (n >= total) break;
-        const BatchPlan P = plans[s_plan[team]];
-        const WorkItem it = P.items[n - item_start[s_plan[team]]];
-        if (tid == 0) {
+        const BatchPlan P = plans[items[n].plan];
+        const WorkItem it = items[n].it;
+        if (tid == 0 && it.r0 == 0) {
             prefetch_l2_range(P.chunks, it.cbeg, it.cend, 8);
             prefetch_l2_range(P.rec, it.vbeg, it.vend, 16);
         }
@@ -554,8 +547,8 @@ static_assert(DG_TILE_STRIDE % 128 == 0 && DG_VT_OFF % 16 == 0 && DG_UT_OFF % 16
 template <int MODE>
 __global__ void __launch_bounds__(DG_THREADS, 1)
     k_degrid(const __grid_constant__ CUtensorMap tmap, const WorkItem *__restrict__ items,
-             int64_t nitems, unsigned long long *counter, const uint2 *__restrict__ chunks,
-             const uint32_t *__restrict__ gdd, const float *__restrict__ cft_g,
+             const unsigned long long *nitems_dev, unsigned long long *counter,
+             const uint2 *__restrict__ chunks, const uint32_t *__restrict__ gdd, const float *__restrict__ cft_g,
              const float2 *__restrict__ fobs, float4 *rec, const uint8_t *__restrict__ gconj,
              const float2 *__restrict__ rot, const float *__restrict__ wt, float4 *stage, int ntu,
              const float2 *__restrict__ grid, int pitch, int nv, int vorigin, int refl,
@@ -580,6 +573,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
         for (int a = 0; a < NTAP; a++) sacc += cft_g[d * 8 + a];
         rsum[d] = 1.0f / sacc;
     }
+    const long long nitems = (long long)*nitems_dev;
     __syncthreads();
     const int q = tid & 3;
     const bool hi2 = (q & 2) != 0, hi1 = (q & 1) != 0;
@@ -609,11 +603,11 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
                 " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(tile)),
                 "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(x), "r"(y), "r"(smem_u32(bar))
                 : "memory");
-            prefetch_l2_range(chunks, it.cbeg, it.cend, 8);
+            if (it.r0 == 0) prefetch_l2_range(chunks, it.cbeg, it.cend, 8);
             // the first DG_PREFETCH visibilities' words only: whole items of all resident
             // teams would not fit in L2 together (measured: the full range evicts what it
             // fetched)
-            const int pf_end = min(it.vend, it.vbeg + DG_PREFETCH);
+            const int pf_end = it.r0 == 0 ? min(it.vend, it.vbeg + DG_PREFETCH) : it.vbeg;
             prefetch_l2_range(gdd, it.vbeg, pf_end, 4);
             if (MODE == 0) prefetch_l2_range(fobs, it.vbeg, pf_end, 8);
         }
@@ -652,7 +646,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
         // Every lane of a warp runs the same number of group iterations (the loop bounds are
         // per item), so the shuffles below always see all 32 lanes.
         const int ngroups_iter = (it.cend - it.cbeg + DG_GROUPS - 1) / DG_GROUPS;
-        for (int gi = 0; gi < ngroups_iter; gi++) {
+        for (int gi = it.r0; gi < ngroups_iter; gi += it.rstep) {
             const int c = it.cbeg + gi * DG_GROUPS + grp;
             const bool live = c < it.cend;
             const uint2 ch = live ? chunks[c] : make_uint2(0u, 0u);
@@ -977,7 +971,7 @@ size_t grid_smem_bytes() { return grid_smem(); }
 int grid_ctas_per_sm() { return 1; }
 
 int launch_grid_batch(sde_ctx *ctx, int psf, int comp, const BatchPlan *d_plans,
-                      const int64_t *d_item_start, int nplans, unsigned long long *d_counter,
+                      const BatchItem *d_items, int64_t nitems, unsigned long long *d_counter,
                       const float *cft, int nctas) {
     static bool attr = false;
     if (!attr) {
@@ -994,13 +988,13 @@ int launch_grid_batch(sde_ctx *ctx, int psf, int comp, const BatchPlan *d_plans,
     KTimer kt(ctx, psf ? "grid_batch_psf" : "grid_batch");
     const dim3 g((unsigned)nctas), b(GRID_THREADS);
     if (psf && comp)
-        k_grid_batch<true, true><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_item_start, nplans, d_counter, cft);
+        k_grid_batch<true, true><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_items, nitems, d_counter, cft);
     else if (psf)
-        k_grid_batch<true, false><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_item_start, nplans, d_counter, cft);
+        k_grid_batch<true, false><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_items, nitems, d_counter, cft);
     else if (comp)
-        k_grid_batch<false, true><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_item_start, nplans, d_counter, cft);
+        k_grid_batch<false, true><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_items, nitems, d_counter, cft);
     else
-        k_grid_batch<false, false><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_item_start, nplans, d_counter, cft);
+        k_grid_batch<false, false><<<g, b, grid_smem(), ctx->stream>>>(d_plans, d_items, nitems, d_counter, cft);
     SDE_CHECK_LAUNCH();
     return SDE_OK;
 }
@@ -1045,18 +1039,18 @@ int plan_grid_raw(sde_plan *pl, int what, float2 *raw, float2 *raw_lo, bool lo_c
     SDE_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), ctx->stream));
     KTimer kt(ctx, what == SDE_GRID_PSF ? "grid_psf" : "grid");
     const int64_t want = (int64_t)ctx->num_sms;
-    const dim3 g((unsigned)(pl->nitems < want ? pl->nitems : want)), b(GRID_THREADS);
+    const dim3 g((unsigned)(pl->parts_max < want ? pl->parts_max : want)), b(GRID_THREADS);
     const size_t sm = grid_smem();
     cudaStream_t st = ctx->stream;
-    const int64_t ni = pl->nitems;
+    const unsigned long long *ni = pl->nparts;
     if (what == SDE_GRID_PSF && raw_lo)
-        k_grid<true, true><<<g, b, sm, st>>>(pl->items, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
+        k_grid<true, true><<<g, b, sm, st>>>(pl->parts, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
     else if (what == SDE_GRID_PSF)
-        k_grid<true, false><<<g, b, sm, st>>>(pl->items, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
+        k_grid<true, false><<<g, b, sm, st>>>(pl->parts, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
     else if (raw_lo)
-        k_grid<false, true><<<g, b, sm, st>>>(pl->items, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
+        k_grid<false, true><<<g, b, sm, st>>>(pl->parts, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
     else
-        k_grid<false, false><<<g, b, sm, st>>>(pl->items, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
+        k_grid<false, false><<<g, b, sm, st>>>(pl->parts, ni, counter, pl->chunks, pl->rec, pl->cft, raw, raw_lo, pl->pitch, pl->ntu, nu, nv);
     SDE_CHECK_LAUNCH();
     return SDE_OK;
 }
@@ -1113,16 +1107,16 @@ int plan_degrid(sde_plan *pl, const float *grid, int pitch, int mode, float2 *vi
         SDE_TRY(ctx_scratch(ctx, "degrid_counter", sizeof(unsigned long long), (void **)&counter));
         SDE_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), ctx->stream));
         const int64_t want = (int64_t)ctx->num_sms;
-        const unsigned nb = (unsigned)(pl->nitems < want ? pl->nitems : want);
+        const unsigned nb = (unsigned)(pl->parts_max < want ? pl->parts_max : want);
         KTimer kt(ctx, "degrid");
         if (mode == 0)
             k_degrid<0><<<nb, DG_THREADS, degrid_smem(), ctx->stream>>>(
-                map, pl->items, pl->nitems, counter, pl->chunks, pl->gdd, pl->cft, pl->fobs, pl->rec,
+                map, pl->parts, pl->nparts, counter, pl->chunks, pl->gdd, pl->cft, pl->fobs, pl->rec,
                 pl->gconj, pl->rot, pl->wt, nullptr, pl->ntu, (const float2 *)grid, pitch, nv,
                 pl->spec.vorigin, (int)(pl->spec.uorigin == 1), ctx->d_status);
         else
             k_degrid<1><<<nb, DG_THREADS, degrid_smem(), ctx->stream>>>(
-                map, pl->items, pl->nitems, counter, pl->chunks, pl->gdd, pl->cft, pl->fobs, pl->rec,
+                map, pl->parts, pl->nparts, counter, pl->chunks, pl->gdd, pl->cft, pl->fobs, pl->rec,
                 pl->gconj, pl->rot, pl->wt, stage, pl->ntu, (const float2 *)grid, pitch, nv,
                 pl->spec.vorigin, (int)(pl->spec.uorigin == 1), ctx->d_status);
         SDE_CHECK_LAUNCH();

@@ -246,6 +246,8 @@ __global__ void k_run_emit(const uint32_t *__restrict__ keys, const uint32_t *__
             wi.vbeg = (int32_t)a;
             wi.vend = 0;
             wi.dense = 0;
+            wi.r0 = 0;
+            wi.rstep = 1;
             items[nit++] = wi;
         }
         const uint64_t it = nit - 1;
@@ -338,6 +340,22 @@ __global__ void k_item_dense(WorkItem *items, int64_t nitems) {
     items[t].dense = (int64_t)items[lo - 1].vend - items[first].vbeg >= DENSE_TILE_VIS;
 }
 
+// The launch list: every item once, or once per part with its rounds dealt out.  The list's
+// order does not matter (teams take entries from a counter), so entries are appended.
+__global__ void k_item_parts(const WorkItem *__restrict__ items, int64_t nitems, int part, WorkItem *parts,
+                             unsigned long long *nparts) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nitems) return;
+    WorkItem it = items[t];
+    const int np = item_parts(it, part);
+    const unsigned long long at = atomicAdd(nparts, (unsigned long long)np);
+    it.rstep = np;
+    for (int k = 0; k < np; k++) {
+        it.r0 = k;
+        parts[at + k] = it;
+    }
+}
+
 __global__ void k_item_vend(WorkItem *items, int64_t nitems, int64_t nvalid) {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nitems) return;
@@ -377,7 +395,7 @@ int sde_plan_destroy(sde_plan *pl) {
     cudaSetDevice(ctx->device);
     // stream-ordered frees: after the plan's last use on the context's stream
     void *ptrs[] = {pl->fobs, pl->rec, pl->wt, pl->gdd, pl->orig, pl->rot, pl->gconj, pl->chunks,
-                    pl->items, pl->exc, pl->wt_all, pl->cf, pl->cft, pl->d_sums, pl->inv, pl->core_lo};
+                    pl->items, pl->parts, pl->exc, pl->wt_all, pl->cf, pl->cft, pl->d_sums, pl->inv, pl->core_lo};
     for (void *p : ptrs) ctx_free(ctx, p, 0);
     ctx->bytes -= pl->bytes;
     delete pl;
@@ -615,6 +633,14 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
             k_item_vend<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, nvalid);
             PL_CUDA(cudaGetLastError());
             k_item_dense<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems);
+            PL_CUDA(cudaGetLastError());
+            // an item has at most ceil(visibilities / part) entries
+            const int part = part_size(nvis);
+            pl->parts_max = nitems + nvalid / part;
+            PL_TRY(plan_alloc(pl, (void **)&pl->parts, sizeof(WorkItem) * (size_t)(pl->parts_max + 1)));
+            pl->nparts = reinterpret_cast<unsigned long long *>(pl->parts + pl->parts_max);
+            PL_CUDA(cudaMemsetAsync(pl->nparts, 0, sizeof(unsigned long long), st));
+            k_item_parts<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, part, pl->parts, pl->nparts);
             PL_CUDA(cudaGetLastError());
             const size_t ncore = (size_t)(pl->ntu + 1) * (pl->ntv + 1);
             PL_TRY(plan_alloc(pl, (void **)&pl->core_lo, ncore));
