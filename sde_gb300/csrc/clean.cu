@@ -9,7 +9,7 @@
 // operations (no FMA), finds its slice's first maximum, and that maximum joins a global one
 // (a packed key, one atomicMax per CTA) inside a grid barrier (bounded spin); every CTA then
 // reads the same global (max, first index), so component positions are identical to the
-// reference's.
+// reference's.  Windows that fit one thread-block cluster run in k_hogbom_cluster.
 #include <cooperative_groups.h>
 #include <math.h>
 #include <string.h>
@@ -305,6 +305,238 @@ __global__ void __launch_bounds__(CL_THREADS) k_hogbom(CleanArgs A) {
     }
 }
 
+
+// ---------------------------------------------------------------------------------------
+// Small windows: the whole minor cycle in one thread-block cluster.  A window of up to
+// HC_MAXPIX pixels is spread over the cluster's threads, PER pixels each (residual and
+// component image in registers for all iterations), so an iteration needs no grid-wide
+// barrier: every CTA sends its maximum to every CTA with one remote store that also counts
+// on the receiver's mbarrier (st.async), and waits for the others' on its own.  The
+// arithmetic and the pick (largest |RES|, then the first index) are k_hogbom's.
+// An iteration is a latency chain: PSF load, warp maximum, CTA barrier, remote store, slot
+// maximum.  Measured a component, k_hogbom -> here: 127^2 3.5 -> 0.9 us, 255^2 3.4 -> 1.1,
+// 361^2 3.5 -> 1.6, 511^2 3.7 -> 2.25.  Few warps a CTA: every warp repeats the scalar part of
+// the chain, and with 1024 threads those instructions queue for issue slots (255^2 1.3 us).
+constexpr int HC_CTAS = 16;   // cluster size (above the portable 8: opted in at launch)
+constexpr int64_t HC_MAXPIX = (int64_t)512 * HC_CTAS * 32;
+constexpr int HC_RING = 256;  // components kept before they go into CLN
+constexpr int HC_SPIN = 1 << 20;
+
+__device__ __forceinline__ uint32_t cl_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Row of pixel idx in rows of nx pixels, by the reciprocal ceil(2^32 / nx): the product can
+// only reach the next row's first pixel early.
+__device__ __forceinline__ uint32_t row_recip(int nx) { return nx > 1 ? 0xFFFFFFFFu / (uint32_t)nx + 1u : 0u; }
+__device__ __forceinline__ int row_of(int idx, int nx, uint32_t recip) {
+    if (nx == 1) return idx;
+    const int q = (int)__umulhi((uint32_t)idx, recip);
+    return q * nx > idx ? q - 1 : q;
+}
+
+// The cluster's maxima of one round: slot r holds CTA r's key.
+template <int C>
+struct ClusterMax {
+    unsigned long long slot[2][C];
+    unsigned long long bar[2];
+};
+
+template <int C>
+__device__ __forceinline__ void cluster_max_init(ClusterMax<C> *m) {
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&m->bar[p])));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(&m->bar[p])),
+                         "r"((uint32_t)(8 * C)));
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Called by the first C lanes of one warp: the CTA's key of round n to slot `rank` of CTA
+// `lane`.  A slot is written again two rounds later, by a CTA that has this CTA's key of the
+// round between, which is sent after every warp here has read the slot.
+template <int C>
+__device__ __forceinline__ void cluster_max_send(ClusterMax<C> *m, int n, int rank, int lane,
+                                                 unsigned long long key) {
+    uint32_t dst, bar;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(cl_smem(&m->slot[n & 1][rank])), "r"(lane));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(cl_smem(&m->bar[n & 1])), "r"(lane));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+                 "l"(key), "r"(bar)
+                 : "memory");
+}
+
+// Called by every thread: round n's keys of all CTAs, reduced; ok is cleared when the warp's
+// wait gave up.
+template <int C>
+__device__ __forceinline__ unsigned long long cluster_max_wait(ClusterMax<C> *m, int n, bool &ok) {
+    const uint32_t bar = cl_smem(&m->bar[n & 1]);
+    const uint32_t parity = (uint32_t)(n >> 1) & 1u;
+    uint32_t done = 0;
+    for (int spin = 0; spin < HC_SPIN && !done; spin++)
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;"
+            " selp.u32 %0, 1, 0, p; }"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    const int lane = threadIdx.x & 31;
+    ok = __all_sync(0xffffffffu, done);
+    return warp_key_max(ok && lane < C ? *(volatile unsigned long long *)&m->slot[n & 1][lane] : 0ull);
+}
+
+// One thread, after its CTA has passed round n's wait: the barrier's next phase expects C keys.
+template <int C>
+__device__ __forceinline__ void cluster_max_rearm(ClusterMax<C> *m, int n) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(&m->bar[n & 1])),
+                 "r"((uint32_t)(8 * C))
+                 : "memory");
+}
+
+// PSF peak (1-based) from PIXISAMA's index (pix/pix2drcl.f:73-80)
+__host__ __device__ inline void psf_peak(int64_t ip1, int pnx, int pny, int *pmpx, int *pmpy) {
+    const int ipeak = (int)((ip1 > 0 ? ip1 : 1) - 1);  // PIXISAMA's default I = 1
+    int px = 1 + ipeak % pnx;
+    int py = 1 + (ipeak - px + 1) / pnx;
+    if (px >= pnx) px = pnx / 2;
+    if (py >= pny) py = pny / 2;
+    *pmpx = px;
+    *pmpy = py;
+}
+
+// Every shift of the window by a component lies inside the PSF array, axis by axis: no PSF
+// read is out of range or wraps into another row.
+__host__ __device__ inline bool psf_covers(int pmpx, int pmpy, int nx, int ny, int pnx, int pny) {
+    return pmpx - (nx - 1) >= 1 && pmpx + (nx - 1) <= pnx && pmpy - (ny - 1) >= 1 && pmpy + (ny - 1) <= pny;
+}
+
+// A.psf_ip: the PSF's peak index on the device (k_isamax_final).  When the PSF does not cover
+// every shift nothing is done and A.out[3] is HC_NOTCOVERED (the caller runs k_hogbom).
+constexpr int HC_NOTCOVERED = 3;
+template <int T, int PER>
+__global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int64_t *psf_ip) {
+    __shared__ __align__(16) ClusterMax<HC_CTAS> cm;
+    __shared__ unsigned long long skey[T / 32];
+    __shared__ int ring_idx[HC_RING];
+    __shared__ float ring_f[HC_RING];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint32_t rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    int pmpx, pmpy;
+    psf_peak(*psf_ip, A.pnx, A.pny, &pmpx, &pmpy);
+    if (!psf_covers(pmpx, pmpy, A.nx, A.ny, A.pnx, A.pny)) {
+        if (rank == 0 && t == 0) A.out[3] = __int_as_float(HC_NOTCOVERED);
+        return;
+    }
+    cluster_max_init(&cm);
+    const int npix = A.nx * A.ny, base = (int)rank * PER * T;
+    float r[PER];
+    int rel[PER];  // the pixel's PSF offset from the component's: -ix - iy * pnx
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int k = base + j * T + t;
+        const bool in = k < npix;
+        const int iy = in ? k / A.nx : 0, ix = in ? k - iy * A.nx : 0;
+        rel[j] = -ix - iy * A.pnx;
+        r[j] = in ? __fmul_rn(A.drt[k], A.box ? A.box[k] : 1.0f) : 0.f;
+    }
+    // NaN pixels (and the padding past the window) never win
+    auto best = [&]() {
+        float la = -1.0f, lv = 0.f;
+        int li = 0;
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int k = base + j * T + t;
+            if (k < npix && fabsf(r[j]) > la) {
+                la = fabsf(r[j]);
+                li = k;
+                lv = r[j];
+            }
+        }
+        return warp_key_max(la >= 0.0f ? cand_key(Cand{la, li, lv}) : 0ull);
+    };
+    // n components of the ring into CLN, each by its pixel's thread in order
+    auto drain = [&](int n) {
+        __syncthreads();
+        for (int i = 0; i < n; i++) {
+            const int own = ring_idx[i] - base - t;
+            if (own >= 0 && own < PER * T && own % T == 0)
+                A.cln[ring_idx[i]] = __fadd_rn(A.cln[ring_idx[i]], ring_f[i]);
+        }
+        __syncthreads();
+    };
+    float tflux = A.tflux_in, maxres = 0.f;
+    const int nabs = A.nsub < 0 ? -A.nsub : A.nsub;
+    const uint32_t rnx = row_recip(A.nx);
+    int isub = A.bsub, stopped = 0;
+    bool ok = true;
+    for (int n = 0;; n++) {
+        const unsigned long long wk = best();
+        if (lane == 0) skey[warp] = wk;
+        if (__syncthreads_or(!ok)) {  // some warp's wait gave up: the whole CTA leaves
+            if (t == 0) atomicExch(&A.status[STATUS_TIMEOUT], 1);
+            break;
+        }
+        if (warp == 0) {
+            const unsigned long long ck = warp_key_max(lane < T / 32 ? skey[lane] : 0ull);
+            if (lane < HC_CTAS) cluster_max_send(&cm, n, (int)rank, lane, ck);
+        }
+        const unsigned long long gk = cluster_max_wait(&cm, n, ok);
+        if (!ok) continue;
+        if (t == 0) cluster_max_rearm(&cm, n);
+        const Cand g = key_cand(gk);
+        maxres = g.v;
+        if (isub > nabs) break;
+        // (a key of 0: no pixel is a number, so there is nothing to subtract)
+        if ((A.nsub < 0 && maxres < 0.0f) || fabsf(maxres) <= A.flux || gk == 0ull) {
+            stopped = 1;
+            break;
+        }
+        const float pntsub = __fmul_rn(A.gain, maxres);
+        tflux = __fadd_rn(tflux, pntsub);
+        const int gy = row_of(g.idx, A.nx, rnx), gx = g.idx - gy * A.nx;
+        // PSF(OFFX-IX, OFFY-IY), flat: (pmpx-1 + gx - ix) + (pmpy-1 + gy - iy) * pnx
+        const float *p0 = A.psf + (pmpx - 1 + gx) + (int64_t)(pmpy - 1 + gy) * A.pnx;
+        float p[PER];
+#pragma unroll
+        for (int j = 0; j < PER; j++) p[j] = __ldg(p0 + rel[j]);
+        const int nring = (isub - A.bsub) % HC_RING;
+        if (t == 0) {
+            ring_idx[nring] = g.idx;
+            ring_f[nring] = pntsub;
+            if (rank == 0) {
+                A.cflux[isub - 1] = pntsub;
+                A.cx[isub - 1] = gx + 1;
+                A.cy[isub - 1] = gy + 1;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const float sub = __fmul_rn(pntsub, p[j]);
+            r[j] = __fsub_rn(r[j], A.box ? __fmul_rn(sub, A.box[min(base + j * T + t, npix - 1)]) : sub);
+        }
+        isub++;
+        if (nring == HC_RING - 1) drain(HC_RING);
+    }
+    drain((isub - A.bsub) % HC_RING);
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int k = base + j * T + t;
+        if (k < npix) A.res[k] = r[j];
+    }
+    if (rank == 0 && t == 0) {
+        A.out[0] = maxres;
+        A.out[1] = tflux;
+        A.out[2] = __int_as_float(stopped ? isub - 1 : A.nsub);
+        A.out[3] = __int_as_float(stopped);
+    }
+    // no CTA leaves while another's stores to it may be in flight
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // first strictly-largest |a| (PIXISAMA), two-level
 __global__ void __launch_bounds__(CL_THREADS) k_isamax_part(const float *a, int64_t n, Cand *part) {
     Cand c{-1.0f, INT32_MAX, 0.0f};
@@ -360,8 +592,9 @@ int sde_isamax(sde_ctx *ctx, const float *a, int64_t n, int64_t *index_out) {
     return SDE_OK;
 }
 
-int sde_isamax0(sde_ctx *ctx, const float *a, int64_t n, int64_t *index_out) {
-    if (!ctx || !a || n <= 0 || !index_out || n > INT32_MAX) return SDE_EINVAL;
+// PIXISAMA's index (0 when no |a| exceeds 0) left on the device
+static int isamax_dev(sde_ctx *ctx, const float *a, int64_t n, int64_t **dev) {
+    if (!ctx || !a || n <= 0 || n > INT32_MAX) return SDE_EINVAL;
     SDE_CUDA_TRY(cudaSetDevice(ctx->device));
     int nb = ctx->num_sms * 2;
     Cand *part;
@@ -372,9 +605,15 @@ int sde_isamax0(sde_ctx *ctx, const float *a, int64_t n, int64_t *index_out) {
     SDE_CHECK_LAUNCH();
     k_isamax_final<<<1, CL_THREADS, 0, ctx->stream>>>(part, nb, d);
     SDE_CHECK_LAUNCH();
-    SDE_CUDA_TRY(cudaMemcpyAsync(index_out, d, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    SDE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    *dev = d;
     return SDE_OK;
+}
+
+int sde_isamax0(sde_ctx *ctx, const float *a, int64_t n, int64_t *index_out) {
+    if (!index_out) return SDE_EINVAL;
+    int64_t *d;
+    SDE_TRY(isamax_dev(ctx, a, n, &d));
+    return ctx_read_small(ctx, ctx->stream, index_out, d, sizeof(int64_t));
 }
 
 int sde_image_max(sde_ctx *ctx, const float *image, int64_t n, float *max_dev) {
@@ -413,6 +652,77 @@ int clean_preload(sde_ctx *ctx) {
     ctx->hogbom_per_sm = per_sm;
     SDE_CUDA_TRY(cudaFuncSetAttribute(k_hogbom<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)CL_SMEM_SLICE_MAX));
+    // the cluster kernels: larger clusters than the portable size, if they can be resident
+    struct {
+        const void *k;
+        int threads;
+    } hc[] = {{(const void *)k_hogbom_cluster<256, 4>, 256},
+              {(const void *)k_hogbom_cluster<256, 16>, 256},
+              {(const void *)k_hogbom_cluster<256, 32>, 256},
+              {(const void *)k_hogbom_cluster<512, 32>, 512}};
+    ctx->hogbom_cluster = true;
+    for (const auto &h : hc) {
+        SDE_CUDA_TRY(cudaFuncSetAttribute(h.k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = HC_CTAS;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(HC_CTAS);
+        cfg.blockDim = dim3(h.threads);
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        SDE_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, h.k, &cfg));
+        if (n < 1) ctx->hogbom_cluster = false;
+    }
+    return SDE_OK;
+}
+
+// a minor cycle's scalars after the work queued on the context's stream
+static int clean_result(sde_ctx *ctx, const float *dout, sde_clean_result *out, int *stopped) {
+    float *h = reinterpret_cast<float *>(ctx->h_small);
+    SDE_CUDA_TRY(cudaMemcpyAsync(h, dout, 4 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+    SDE_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int) * STATUS_COUNT,
+                                 cudaMemcpyDeviceToHost, ctx->stream));
+    SDE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (ctx->h_status[STATUS_TIMEOUT]) {
+        sde_set_error("sde_hogbom: a device wait timed out");
+        return SDE_ETIMEDOUT;
+    }
+    memcpy(stopped, &h[3], 4);
+    if (*stopped == HC_NOTCOVERED) return SDE_OK;
+    out->maxres = h[0];
+    out->tflux = h[1];
+    memcpy(&out->ansub, &h[2], 4);
+    return SDE_OK;
+}
+
+static int launch_hogbom_cluster(const CleanArgs &A, const int64_t *psf_ip, cudaStream_t st) {
+    const int64_t npix = (int64_t)A.nx * A.ny;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = HC_CTAS;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(HC_CTAS);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const int64_t per = ceil_div(npix, (int64_t)256 * HC_CTAS);
+    cudaError_t e;
+    if (per <= 4) {
+        e = cudaLaunchKernelEx(&cfg, k_hogbom_cluster<256, 4>, A, psf_ip);
+    } else if (per <= 16) {
+        e = cudaLaunchKernelEx(&cfg, k_hogbom_cluster<256, 16>, A, psf_ip);
+    } else if (per <= 32) {
+        e = cudaLaunchKernelEx(&cfg, k_hogbom_cluster<256, 32>, A, psf_ip);
+    } else {
+        cfg.blockDim = dim3(512);
+        e = cudaLaunchKernelEx(&cfg, k_hogbom_cluster<512, 32>, A, psf_ip);
+    }
+    SDE_CUDA_TRY(e);
     return SDE_OK;
 }
 
@@ -431,14 +741,31 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
         return SDE_EINVAL;
     }
     SDE_CUDA_TRY(cudaSetDevice(ctx->device));
+    float *dout;
+    SDE_TRY(ctx_scratch(ctx, "cl_out", 4 * sizeof(float), (void **)&dout));
+    SDE_CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, sizeof(int) * STATUS_COUNT, ctx->stream));
+    CleanArgs A;
+    A.drt = drt; A.psf = psf; A.box = box; A.cln = cln; A.res = res; A.cflux = cflux;
+    A.cx = cx; A.cy = cy; A.nx = nx; A.ny = ny; A.pnx = pnx; A.pny = pny;
+    A.pmpx = A.pmpy = 0; A.gain = gain; A.flux = flux; A.tflux_in = tflux_in;
+    A.nsub = nsub; A.bsub = bsub; A.cancel = cancel_flag; A.bar = nullptr;
+    A.status = ctx->d_status; A.out = dout;
     // PSF peak (pix/pix2drcl.f:73-80)
+    int64_t *psf_ip;
+    SDE_TRY(isamax_dev(ctx, psf, (int64_t)pnx * pny, &psf_ip));
+    // a window that one cluster holds, and no interrupt flag to poll
+    if (ctx->hogbom_cluster && !cancel_flag && (int64_t)nx * ny <= HC_MAXPIX) {
+        {
+            KTimer kt(ctx, "hogbom");
+            SDE_TRY(launch_hogbom_cluster(A, psf_ip, ctx->stream));
+        }
+        int stopped;
+        SDE_TRY(clean_result(ctx, dout, out, &stopped));
+        if (stopped != HC_NOTCOVERED) return SDE_OK;
+    }
     int64_t ip1;
-    SDE_TRY(sde_isamax(ctx, psf, (int64_t)pnx * pny, &ip1));
-    int ipeak = (int)(ip1 - 1);
-    int pmpx = 1 + ipeak % pnx;
-    int pmpy = 1 + (ipeak - pmpx + 1) / pnx;
-    if (pmpx >= pnx) pmpx = pnx / 2;
-    if (pmpy >= pny) pmpy = pny / 2;
+    SDE_TRY(ctx_read_small(ctx, ctx->stream, &ip1, psf_ip, sizeof ip1));
+    psf_peak(ip1, pnx, pny, &A.pmpx, &A.pmpy);
     int per_sm = ctx->hogbom_per_sm;
     if (per_sm < 1) SDE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hogbom<false>, CL_THREADS, 0));
     if (per_sm < 1) {
@@ -458,18 +785,8 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
         SDE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_hogbom<true>, CL_THREADS, slice));
         smem_res = (int64_t)fit * ctx->num_sms >= nblocks;
     }
-    Barrier *bar;
-    float *dout;
-    SDE_TRY(ctx_scratch(ctx, "cl_bar", sizeof(Barrier), (void **)&bar));
-    SDE_TRY(ctx_scratch(ctx, "cl_out", 4 * sizeof(float), (void **)&dout));
-    SDE_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(Barrier), ctx->stream));
-    SDE_CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, sizeof(int) * STATUS_COUNT, ctx->stream));
-    CleanArgs A;
-    A.drt = drt; A.psf = psf; A.box = box; A.cln = cln; A.res = res; A.cflux = cflux;
-    A.cx = cx; A.cy = cy; A.nx = nx; A.ny = ny; A.pnx = pnx; A.pny = pny;
-    A.pmpx = pmpx; A.pmpy = pmpy; A.gain = gain; A.flux = flux; A.tflux_in = tflux_in;
-    A.nsub = nsub; A.bsub = bsub; A.cancel = cancel_flag; A.bar = bar;
-    A.status = ctx->d_status; A.out = dout;
+    SDE_TRY(ctx_scratch(ctx, "cl_bar", sizeof(Barrier), (void **)&A.bar));
+    SDE_CUDA_TRY(cudaMemsetAsync(A.bar, 0, sizeof(Barrier), ctx->stream));
     void *args[] = {&A};
     KTimer kt(ctx, "hogbom");
     if (smem_res)
@@ -478,21 +795,8 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
     else
         SDE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_hogbom<false>, dim3(nblocks), dim3(CL_THREADS),
                                                  args, 0, ctx->stream));
-    float h[4];
-    SDE_CUDA_TRY(cudaMemcpyAsync(h, dout, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-    SDE_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int) * STATUS_COUNT,
-                                 cudaMemcpyDeviceToHost, ctx->stream));
-    SDE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (ctx->h_status[STATUS_TIMEOUT]) {
-        sde_set_error("sde_hogbom: grid barrier timed out");
-        return SDE_ETIMEDOUT;
-    }
-    int ansub, stopped;
-    memcpy(&ansub, &h[2], 4);
-    memcpy(&stopped, &h[3], 4);
-    out->maxres = h[0];
-    out->tflux = h[1];
-    out->ansub = ansub;
+    int stopped;
+    SDE_TRY(clean_result(ctx, dout, out, &stopped));
     if (stopped == 2) return SDE_ECANCELLED;
     return SDE_OK;
 }
