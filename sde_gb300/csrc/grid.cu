@@ -110,9 +110,8 @@ __device__ __forceinline__ void grid_item(const WorkItem &it, const uint2 *__res
     const float *vcopy = vt + (grp & 3) * 8;
     const float *ucopy = ut + (grp & 3) * 8 + 2 * q;
     constexpr uint32_t FULL = 0xffffffffu;
-    const int rounds = (it.cend - it.cbeg + GGROUPS - 1) / GGROUPS;
-    for (int rr = it.r0; rr < rounds; rr += it.rstep) {
-        const int c = it.cbeg + rr * GGROUPS + grp;
+    for (int c0 = it.cbeg + it.r0 * GGROUPS; c0 < it.cend; c0 += it.rstep * GGROUPS) {
+        const int c = c0 + grp;
         const bool live = c < it.cend;
         const uint2 ch = live ? chunks[c] : make_uint2(0u, 0u);
         const int start = (int)ch.x, cell = (int)(ch.y & 4095u), len = live ? (int)(ch.y >> 16) : 0;
@@ -241,25 +240,32 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
     const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x % TEAM_THREADS;
     float *tre = ut + UT_FLOATS + team * GTILE_FLOATS;
     float *tim = tre + STILE * STILE;
-    __shared__ long long s_next[TEAMS];
+    // the team's item, read from here where it is used: the accumulators leave no registers
+    __shared__ WorkItem s_item[TEAMS];
     for (int k = tid; k < STILE * STILE; k += TEAM_THREADS) {
         tre[k] = 0.f;
         tim[k] = 0.f;
     }
     fill_tap_tables(cft_g, vt, ut);
-    const long long nitems = (long long)*nitems_dev;
     __syncthreads();
+    const WorkItem &it = s_item[team];
     for (;;) {
-        if (tid == 0) s_next[team] = (long long)atomicAdd(counter, 1ull);
-        team_sync(team);
-        const long long n = s_next[team];
-        if (n >= nitems) break;
-        const WorkItem it = items[n];
-        if (tid == 0 && it.r0 == 0) {
-            // the item's chunk list and records stream into L2 while the first chunks run
-            prefetch_l2_range(chunks, it.cbeg, it.cend, 8);
-            prefetch_l2_range(rec, it.vbeg, it.vend, 16);
+        if (tid == 0) {
+            const unsigned long long n = atomicAdd(counter, 1ull);
+            if (n < *nitems_dev) {
+                const WorkItem w = items[n];
+                s_item[team] = w;
+                if (w.r0 == 0) {
+                    // the item's chunk list and records stream into L2 while the first chunks run
+                    prefetch_l2_range(chunks, w.cbeg, w.cend, 8);
+                    prefetch_l2_range(rec, w.vbeg, w.vend, 16);
+                }
+            } else {
+                s_item[team].tile = -1;
+            }
         }
+        team_sync(team);
+        if (it.tile < 0) break;
         grid_item<PSF, COMP>(it, chunks, rec, vt, ut, tre, tim, raw, raw_lo, pitch, ntu, nu, nv, tid, team);
         team_sync(team);
     }
@@ -277,24 +283,33 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
     const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x % TEAM_THREADS;
     float *tre = ut + UT_FLOATS + team * GTILE_FLOATS;
     float *tim = tre + STILE * STILE;
-    __shared__ long long s_next[TEAMS];
+    __shared__ WorkItem s_item[TEAMS];  // the team's item and its plan, as in k_grid
+    __shared__ BatchPlan s_plan[TEAMS];
     for (int k = tid; k < STILE * STILE; k += TEAM_THREADS) {
         tre[k] = 0.f;
         tim[k] = 0.f;
     }
     fill_tap_tables(cft_g, vt, ut);
     __syncthreads();
+    const WorkItem &it = s_item[team];
+    const BatchPlan &P = s_plan[team];
     for (;;) {
-        if (tid == 0) s_next[team] = (long long)atomicAdd(counter, 1ull);
-        team_sync(team);
-        const long long n = s_next[team];
-        if (n >= nitems) break;
-        const BatchPlan P = plans[items[n].plan];
-        const WorkItem it = items[n].it;
-        if (tid == 0 && it.r0 == 0) {
-            prefetch_l2_range(P.chunks, it.cbeg, it.cend, 8);
-            prefetch_l2_range(P.rec, it.vbeg, it.vend, 16);
+        if (tid == 0) {
+            const unsigned long long n = atomicAdd(counter, 1ull);
+            if (n < (unsigned long long)nitems) {
+                const WorkItem w = items[n].it;
+                s_item[team] = w;
+                s_plan[team] = plans[items[n].plan];
+                if (w.r0 == 0) {
+                    prefetch_l2_range(P.chunks, w.cbeg, w.cend, 8);
+                    prefetch_l2_range(P.rec, w.vbeg, w.vend, 16);
+                }
+            } else {
+                s_item[team].tile = -1;
+            }
         }
+        team_sync(team);
+        if (it.tile < 0) break;
         grid_item<PSF, COMP>(it, P.chunks, P.rec, vt, ut, tre, tim, P.raw, P.raw_lo, P.pitch, P.ntu,
                              P.nu, P.nv, tid, team);
         team_sync(team);
