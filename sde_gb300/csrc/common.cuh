@@ -349,13 +349,8 @@ int sde_isamax0(sde_ctx *ctx, const float *a, int64_t n, int64_t *index_out);
 
 // ---------------------------------------------------------------------------------------
 // Kernels shared across translation units (host-side launchers).
-int launch_radix_sort_u32(sde_ctx *ctx, uint32_t *keys, uint32_t *vals, int64_t n, int bits,
-                          uint32_t *keys_tmp, uint32_t *vals_tmp);
-int launch_radix_sort_u64(sde_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, int bits,
-                          uint64_t *keys_tmp, uint32_t *vals_tmp);
-int launch_exclusive_scan_u32(sde_ctx *ctx, const uint32_t *in, uint32_t *out, int64_t n,
-                              uint32_t *total_dev);
-int launch_inclusive_max_scan_i32(sde_ctx *ctx, const int32_t *in, int32_t *out, int64_t n);
+int launch_radix_sort_u32(sde_ctx *ctx, uint32_t **keys, const uint32_t *first_vals, uint32_t **vals, int64_t n,
+                          int bits, uint32_t *keys_tmp, uint32_t *vals_tmp, unsigned long long *fail);
 
 
 // host restatement of the 'SF' tables (grd/grdcf.f, grd/grdsf.f, grd/grdccf.f)

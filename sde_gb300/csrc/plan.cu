@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "geom.cuh"
+#include "lookback.cuh"
 
 namespace {
 
@@ -39,24 +40,60 @@ struct __align__(32) PlanRecU {
     uint32_t exc_slot;  // the visibility's place in the exception list (exceptions only)
 };
 
+// What the build reads back and what must start at zero: the visibility counts, the control
+// words of the two scans below, and (following this) their tiles' look-back words.
+struct ScanCtl {
+    unsigned long long total;
+    uint32_t next, pad;
+};
+struct PlanCounts {
+    unsigned long long ngrid, nexc, npos, exc_next;  // gridded, exceptions, WT > 0, list slots taken
+    unsigned long long fail;                         // a device wait gave up
+    ScanCtl runs, emit;                              // totals: runs; chunks | items << 31
+    unsigned long long pad;
+};
+constexpr int SC_T = 256, SC_R = 4;  // 1024 entries a scan tile
+int64_t scan_tiles(int64_t n) { return n / (SC_T * SC_R) + 1; }
+
 // Per visibility (caller order): gridding key, the PlanRecU sector and, for an exception, its
-// entry in the exception list,
-// from both routines' geometry (geom_vis).
-__global__ void k_plan_geom(GParams p, const float *__restrict__ u, const float *__restrict__ v,
+// entry in the exception list, from both routines' geometry (geom_vis).  GE_PER visibilities a
+// thread, their loads in flight together (64.7 million: one a thread, its value and coordinates
+// read once its weight was known, 1.19 ms; here 0.91).
+constexpr int GE_T = 256, GE_PER = 2;
+__device__ __forceinline__ void store_rec(PlanRecU *r, const PlanRecU &v) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(r), "f"(v.rec.x), "f"(v.rec.y),
+                 "f"(v.rec.z), "f"(v.rec.w), "r"(v.gdd), "f"(v.rc), "f"(v.rs), "r"(v.exc_slot)
+                 : "memory");
+}
+__global__ void __launch_bounds__(GE_T) k_plan_geom(GParams p, const float *__restrict__ u, const float *__restrict__ v,
                             const float *__restrict__ w, const float2 *__restrict__ vis,
                             const float *__restrict__ wt, int64_t n, uint32_t *keys,
-                            uint32_t *vals, PlanRecU *rec_u, uint32_t *exc_list,
-                            unsigned long long *counts) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t nvalid = 0, nexc = 0;
-    const float wi = i < n ? wt[i] : 0.0f;
-    if (i < n) {
+                            PlanRecU *rec_u, uint32_t *exc_list,
+                            PlanCounts *counts) {
+    const int64_t i0 = (int64_t)blockIdx.x * (GE_T * GE_PER) + threadIdx.x;
+    uint32_t nvalid = 0, nexc = 0, npos = 0;
+    float wts[GE_PER], us[GE_PER], vs[GE_PER], ws[GE_PER];
+    float2 vals[GE_PER];
+#pragma unroll
+    for (int j = 0; j < GE_PER; j++) {
+        const int64_t i = min(i0 + j * GE_T, n - 1);
+        wts[j] = wt[i];
+        us[j] = u[i];
+        vs[j] = v[i];
+        ws[j] = w[i];
+        vals[j] = vis[i];
+    }
+#pragma unroll
+    for (int j = 0; j < GE_PER; j++) {
+        const int64_t i = i0 + j * GE_T;
+        if (i >= n) break;
+        const float wi = wts[j];
         uint32_t key = KEY_INVALID, pdd = 0, tw = 0;
         float2 f = make_float2(0.f, 0.f), r = make_float2(1.f, 0.f);
         uint8_t gc = 0;
         if (wi > 0.0f) {
-            const float2 vv = vis[i];
-            const GGeo g = geom_vis(p, u[i], v[i], w[i], vv.x, vv.y);
+            npos++;
+            const GGeo g = geom_vis(p, us[j], vs[j], ws[j], vals[j].x, vals[j].y);
             const DGeo &dg = g.dg;
             gc = g.gc ? 1 : 0;
             r = make_float2(g.rc, g.rs);
@@ -80,15 +117,14 @@ __global__ void k_plan_geom(GParams p, const float *__restrict__ u, const float 
                 const uint32_t off = (uint32_t)lu & 1u;
                 tw = taps_word(dug, dvg, off);
                 pdd = exc ? (taps_word(0, 0, off) | GDD_EXCEPTION) : taps_word(dg.dui, dg.dvi, off);
-                nvalid = 1;
-                nexc = exc;
+                nvalid++;
+                nexc += exc;
                 f = make_float2(g.fr, g.fi);
             } else {
-                nexc = 1;  // degrid-only or degrid-invalid: exception path
+                nexc++;  // degrid-only or degrid-invalid: exception path
             }
         }
         keys[i] = key;
-        vals[i] = (uint32_t)i;
         PlanRecU pr;
         pr.rec = make_float4(wi, __uint_as_float(tw), f.x, f.y);
         pr.gdd = pdd | (gc ? GDD_GCONJ_U : 0u);
@@ -99,55 +135,99 @@ __global__ void k_plan_geom(GParams p, const float *__restrict__ u, const float 
         // whose degridding cell is not the gridding cell: appended to the list (a few in 10^4;
         // the list's order does not matter, each is degridded on its own)
         if (wi > 0.0f && (key == KEY_INVALID || (pdd & GDD_EXCEPTION) != 0)) {
-            pr.exc_slot = (uint32_t)atomicAdd(&counts[3], 1ull);
+            pr.exc_slot = (uint32_t)atomicAdd(&counts->exc_next, 1ull);
             exc_list[pr.exc_slot] = (uint32_t)i;
         }
-        rec_u[i] = pr;
+        store_rec(rec_u + i, pr);
     }
     // block-aggregated counters (one atomic per block and counter: per-warp atomics on three
     // addresses serialise in L2 at this visibility count)
-    const int cv = __syncthreads_count(nvalid), ce = __syncthreads_count(nexc);
-    const int ct = __syncthreads_count(i < n && wi > 0.0f);
+    __shared__ uint32_t sum[3];
+    if (threadIdx.x < 3) sum[threadIdx.x] = 0;
+    __syncthreads();
+    nvalid = __reduce_add_sync(0xffffffffu, nvalid);
+    nexc = __reduce_add_sync(0xffffffffu, nexc);
+    npos = __reduce_add_sync(0xffffffffu, npos);
+    if ((threadIdx.x & 31) == 0) {
+        if (nvalid) atomicAdd(&sum[0], nvalid);
+        if (nexc) atomicAdd(&sum[1], nexc);
+        if (npos) atomicAdd(&sum[2], npos);
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        if (cv) atomicAdd(&counts[0], (unsigned long long)cv);
-        if (ce) atomicAdd(&counts[1], (unsigned long long)ce);
-        if (ct) atomicAdd(&counts[2], (unsigned long long)ct);
+        if (sum[0]) atomicAdd(&counts->ngrid, (unsigned long long)sum[0]);
+        if (sum[1]) atomicAdd(&counts->nexc, (unsigned long long)sum[1]);
+        if (sum[2]) atomicAdd(&counts->npos, (unsigned long long)sum[2]);
     }
 }
 
 // Gather the per-visibility data into the plan's order (one 32-byte sector read per
-// visibility), one warp per chunk: chunk c's visibilities, at [st, st + length) in the sort's
-// order, go to [cpos[c], cpos[c] + length) -- the chunk order, the order the kernels take
-// them -- and the chunk's start moves there.  An exception that also grids learns its
+// visibility): a block takes GA_CHUNKS consecutive chunks, whose visibilities are one
+// contiguous range of the output, and its threads take the range's positions, finding the
+// chunk of a position by bisection of the chunks' starts; the reads of GA_BATCH positions are
+// in flight together (64.7 million visibilities: 1.80 ms by a warp per chunk, whose 27
+// visibilities are one round, here 1.61).  An exception that also grids learns its
 // position here.
-__global__ void __launch_bounds__(256) k_plan_gather(const uint32_t *__restrict__ perm,
-                                                     const uint32_t *__restrict__ cpos, int64_t nchunks,
-                                                     uint2 *chunks, const PlanRecU *__restrict__ rec_u,
-                                                     float2 *fobs,
-                                                     float4 *rec, float *wt, uint32_t *gdd, uint32_t *orig,
-                                                     float2 *rot, uint8_t *gconj, DegridExc *exc) {
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (c >= nchunks) return;
-    const uint2 ch = chunks[c];
-    const uint32_t st = ch.x, len = ch.y >> 16, to = cpos[c];
-    for (uint32_t k = lane; k < len; k += 32) {
-        const uint32_t i = perm[st + k];
-        const int64_t p = (int64_t)to + k;
-        const PlanRecU pr = rec_u[i];
-        const float4 r = pr.rec;
-        const uint32_t d = pr.gdd;
-        rec[p] = r;
-        fobs[p] = make_float2(r.z, r.w);
-        wt[p] = r.x;
-        gdd[p] = d & ~GDD_GCONJ_U;
-        orig[p] = i;
-        gconj[p] = (d & GDD_GCONJ_U) ? 1 : 0;
-        if (rot) rot[p] = make_float2(pr.rc, pr.rs);
-        if ((d & GDD_EXCEPTION) && exc) exc[pr.exc_slot].pos = (int32_t)p;
+__device__ __forceinline__ PlanRecU load_rec(const PlanRecU *r) {
+    PlanRecU v;  // one 32-byte load
+    asm("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v.rec.x), "=f"(v.rec.y), "=f"(v.rec.z), "=f"(v.rec.w), "=r"(v.gdd), "=f"(v.rc), "=f"(v.rs),
+          "=r"(v.exc_slot)
+        : "l"(r));
+    return v;
+}
+constexpr int GA_CHUNKS = 64, GA_BATCH = 4, GA_T = 256;
+__global__ void __launch_bounds__(GA_T) k_plan_gather(const uint32_t *__restrict__ perm,
+                                                      const uint2 *__restrict__ chunks,
+                                                      const uint32_t *__restrict__ csrc, int64_t nchunks,
+                                                      const PlanRecU *__restrict__ rec_u, float2 *fobs,
+                                                      float4 *rec, float *wt, uint32_t *gdd, uint32_t *orig,
+                                                      float2 *rot, uint8_t *gconj, DegridExc *exc) {
+    __shared__ uint32_t to[GA_CHUNKS + 1], from[GA_CHUNKS];
+    const int t = threadIdx.x;
+    const int64_t c0 = (int64_t)blockIdx.x * GA_CHUNKS;
+    const int nc = (int)min((int64_t)GA_CHUNKS, nchunks - c0);
+    if (t < nc) {
+        const uint2 ch = chunks[c0 + t];
+        to[t] = ch.x;
+        from[t] = csrc[c0 + t];
+        if (t == nc - 1) to[nc] = ch.x + (ch.y >> 16);
     }
-    __syncwarp();  // every lane has read the chunk record
-    if (lane == 0) chunks[c] = make_uint2(to, ch.y);
+    __syncthreads();
+    const uint32_t end = to[nc];
+    for (uint32_t p0 = to[0] + t; p0 < end; p0 += GA_BATCH * GA_T) {
+        uint32_t src[GA_BATCH];
+#pragma unroll
+        for (int j = 0; j < GA_BATCH; j++) {
+            const uint32_t p = p0 + j * GA_T;
+            if (p >= end) break;
+            int lo = 0, hi = nc;  // the last chunk that starts at or before p
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (to[mid] <= p) lo = mid; else hi = mid;
+            }
+            src[j] = perm[from[lo] + (p - to[lo])];
+        }
+        PlanRecU pr[GA_BATCH];
+#pragma unroll
+        for (int j = 0; j < GA_BATCH; j++)
+            if (p0 + j * GA_T < end) pr[j] = load_rec(rec_u + src[j]);
+#pragma unroll
+        for (int j = 0; j < GA_BATCH; j++) {
+            const uint32_t p = p0 + j * GA_T;
+            if (p >= end) break;
+            const float4 r = pr[j].rec;
+            const uint32_t d = pr[j].gdd;
+            rec[p] = r;
+            fobs[p] = make_float2(r.z, r.w);
+            wt[p] = r.x;
+            gdd[p] = d & ~GDD_GCONJ_U;
+            orig[p] = src[j];
+            gconj[p] = (d & GDD_GCONJ_U) ? 1 : 0;
+            if (rot) rot[p] = make_float2(pr[j].rc, pr[j].rs);
+            if ((d & GDD_EXCEPTION) && exc) exc[pr[j].exc_slot].pos = (int32_t)p;
+        }
+    }
 }
 
 // The exception list's entries, one thread per exception (pos is set by k_plan_gather for the
@@ -180,149 +260,185 @@ __global__ void k_exc_write(GParams p, const float *__restrict__ u, const float 
 // (equal key >> 1); a tile's visibilities split into work items at every item_max from the
 // tile's first one; a run's part within one item (a piece) splits into chunks of chunk_max
 // from the piece's start.  Chunks and items are numbered in position order.
-__global__ void k_run_heads(const uint32_t *__restrict__ keys, const unsigned long long *counts,
-                            int64_t n, uint32_t *head) {
-    const int64_t nv = (int64_t)counts[0];
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    head[q] = q < nv && (q == 0 || (keys[q - 1] >> 1) != (keys[q] >> 1));
-}
-
-__global__ void k_run_compact(const uint32_t *__restrict__ head, const uint32_t *__restrict__ ridx,
-                              const unsigned long long *counts, uint32_t *rstart) {
-    const int64_t nv = (int64_t)counts[0];
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < nv && head[q]) rstart[ridx[q]] = (uint32_t)q;
-}
-
-// a run that starts a tile: its start (the tile's first visibility), else -1, for a max-scan
-__global__ void k_run_tilehead(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ rstart,
-                               int64_t nruns, int32_t *tstart) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nruns) return;
-    const uint32_t rs = rstart[r];
-    const bool th = r == 0 || (keys[rstart[r - 1]] >> 12) != (keys[rs] >> 12);
-    tstart[r] = th ? (int32_t)rs : -1;
-}
-
-// the run's chunks and item heads (an item head is a position ts + k*item_max of the run)
-__global__ void k_run_counts(const uint32_t *__restrict__ rstart, const int32_t *__restrict__ tstart,
-                             int64_t nruns, int64_t nvalid, int item_max, int chunk_max, uint32_t *nch,
-                             uint32_t *nih) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nruns) return;
-    const int64_t rs = rstart[r], re = r + 1 < nruns ? (int64_t)rstart[r + 1] : nvalid, ts = tstart[r];
-    uint32_t c = 0, h = 0;
-    for (int64_t a = rs; a < re;) {
-        const int64_t is = ts + (a - ts) / item_max * item_max;
-        h += is == a;
-        const int64_t b = min(re, is + item_max);
-        c += (uint32_t)((b - a + chunk_max - 1) / chunk_max);
-        a = b;
+//
+// The runs' starts, compacted, and the first visibility of every tile that has one.  A warp
+// takes RU_R rounds of 32 consecutive keys; heads are counted by ballots, so the keys stay in
+// registers.
+constexpr int RU_T = 512, RU_R = 16;  // 8192 keys a scan tile
+__global__ void __launch_bounds__(RU_T) k_runs(const uint32_t *__restrict__ keys, PlanCounts *counts, int64_t n,
+                                               unsigned long long *words, uint32_t *rstart, uint32_t *tstart) {
+    __shared__ uint32_t wsum[RU_T / 32];
+    __shared__ unsigned long long before;
+    __shared__ uint32_t stile;
+    const int64_t nv = (int64_t)counts->ngrid;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t == 0) stile = atomicAdd(&counts->runs.next, 1u);
+    __syncthreads();
+    const int64_t tile = stile, base = tile * (RU_T * RU_R), w0 = base + (int64_t)warp * 32 * RU_R;
+    uint32_t key[RU_R], mask[RU_R];
+#pragma unroll
+    for (int r = 0; r < RU_R; r++) {
+        const int64_t q = w0 + r * 32 + lane;
+        key[r] = q < nv ? keys[q] : 0u;
     }
-    nch[r] = c;
-    nih[r] = h;
+    uint32_t prev = w0 > 0 && w0 <= nv ? keys[w0 - 1] : 0u;  // (lane 0's) the key before the round
+    uint32_t sum = 0;
+#pragma unroll
+    for (int r = 0; r < RU_R; r++) {
+        const int64_t q = w0 + r * 32 + lane;
+        uint32_t p = __shfl_up_sync(0xffffffffu, key[r], 1);
+        if (lane == 0) p = prev;
+        prev = __shfl_sync(0xffffffffu, key[r], 31);
+        mask[r] = __ballot_sync(0xffffffffu, q < nv && (q == 0 || (p >> 1) != (key[r] >> 1)));
+        sum += __popc(mask[r]);
+    }
+    if (lane == 0) wsum[warp] = sum;
+    __syncthreads();
+    uint32_t pre = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < RU_T / 32; w++) {
+        pre += w < warp ? wsum[w] : 0u;
+        all += wsum[w];
+    }
+    if (t == 0) {
+        unsigned long long b = 0;
+        if (tile > 0) {
+            lb_publish(&words[tile], LB_AGG, all);
+            b = lb_sum_before(words, tile, 1, &counts->fail);
+        }
+        lb_publish(&words[tile], LB_PREFIX, b + all);
+        before = b;
+        if (base + RU_T * RU_R >= n) counts->runs.total = b + all;
+    }
+    __syncthreads();
+    uint32_t at = (uint32_t)before + pre;
+#pragma unroll
+    for (int r = 0; r < RU_R; r++) {
+        const int64_t q = w0 + r * 32 + lane;
+        if ((mask[r] >> lane) & 1u) {
+            const uint32_t o = at + __popc(mask[r] & ((1u << lane) - 1u));
+            if (o < (uint64_t)n) rstart[o] = (uint32_t)q;
+            if (q == 0 || (keys[q - 1] >> 12) != (key[r] >> 12)) tstart[key[r] >> 12] = (uint32_t)q;
+        }
+        at += __popc(mask[r]);
+    }
 }
 
-// the run's chunk records (sort key, index, start) and the items that start in it
-__global__ void k_run_emit(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ rstart,
-                           const int32_t *__restrict__ tstart, int64_t nruns, int64_t nvalid,
-                           const uint32_t *__restrict__ cbase, const uint32_t *__restrict__ ibase,
-                           int item_max, int chunk_max, int lbits, int jbits, uint64_t *ckey,
-                           uint32_t *cval, uint32_t *cstart, WorkItem *items) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nruns) return;
-    const int64_t rs = rstart[r], re = r + 1 < nruns ? (int64_t)rstart[r + 1] : nvalid, ts = tstart[r];
-    const uint32_t k = keys[rs];
-    const uint32_t cell = k & 4094u, lu = cell & 63u, lv = cell >> 6;  // pair's even cell
-    const uint32_t color = ((lu >> 1) & 3u) * 7u + (lv % 7u);
-    uint32_t c = cbase[r], nit = ibase[r];  // items started before the run's current piece
+// A run's pieces: piece(a, b, starts_item) for each.
+template <class F>
+__device__ __forceinline__ void run_pieces(int64_t rs, int64_t re, int64_t ts, int item_max, F piece) {
     for (int64_t a = rs; a < re;) {
         const int64_t is = ts + (a - ts) / item_max * item_max;
-        if (is == a) {
-            WorkItem wi;
-            wi.tile = (int32_t)(k >> 12);
-            wi.cbeg = wi.cend = 0;
-            wi.vbeg = (int32_t)a;
-            wi.vend = 0;
-            wi.dense = 0;
-            wi.r0 = 0;
-            wi.rstep = 1;
-            items[nit++] = wi;
-        }
-        const uint64_t it = nit - 1;
         const int64_t b = min(re, is + item_max);
-        uint32_t j = 0;
-        for (int64_t q = a; q < b; q += chunk_max, j++, c++) {
-            ckey[c] = (it << (LENBIN_BITS + 6 + lbits + jbits + 12)) |
-                      ((uint64_t)color << (lbits + jbits + 12)) | ((uint64_t)j << 12) | cell;
-            cval[c] = c;
-            cstart[c] = (uint32_t)q;
-        }
+        piece(a, b, is == a);
         a = b;
     }
 }
 
-// Length class (CHUNK_MAX - length) of each chunk, above the chunk index in its sort key,
-// and a coarse length bin (LENBIN_BITS, longest first) above the colour class: the 8 chunks
-// a warp of the gridder or degridder takes together have similar lengths (the warp runs to
-// its longest), and mostly one colour.  On the large single field the lanes do useful work
-// in 94% of the warps' visibility slots with 8 bins, 81% with the colour class alone above
-// the length (a simulation of both orders on its chunks; measured: gridder 0.82 -> 0.75 ms).
-__global__ void k_chunk_len(const uint32_t *__restrict__ cstart, int64_t nchunks, int64_t nvalid,
-                            int chunk_max, int lshift, int bshift, uint64_t *ckey) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    const uint32_t en = c + 1 < nchunks ? cstart[c + 1] : (uint32_t)nvalid;
-    const uint32_t len = en - cstart[c];
-    const int cls = chunk_max - (int)len;
-    const int nbin = 1 << LENBIN_BITS;
-    const int bin = min(cls * nbin / chunk_max, nbin - 1);
-    ckey[c] |= ((uint64_t)cls << lshift) | ((uint64_t)bin << bshift);
+// The runs' chunks and the items that start in them, numbered by a scan of both counts (31
+// bits each).  A chunk's entry: where its visibilities are in the sort's order, its even cell
+// and length, and its sort key within the item, in bits from the top: a coarse length bin
+// (LENBIN_BITS, longest first), the colour class, the length class, the chunk index and (16
+// bits) its number in the item.  The 8 chunks that a warp of the gridder or degridder takes
+// together then have similar lengths (the warp runs to its longest) and mostly one colour.  On
+// the large single field the lanes do useful work in 94% of the warps' visibility slots with 8
+// bins, 81% with the colour class alone above the length (a simulation of both orders on its
+// chunks; measured: gridder 0.82 -> 0.75 ms).
+__global__ void __launch_bounds__(SC_T) k_run_emit(const uint32_t *__restrict__ keys, PlanCounts *counts,
+                                                   const uint32_t *__restrict__ rstart,
+                                                   const uint32_t *__restrict__ tstart, int64_t nruns,
+                                                   int item_max, int chunk_max, int lbits, int jbits,
+                                                   int64_t max_items, int64_t max_chunks, unsigned long long *words,
+                                                   uint64_t *ckey, uint2 *craw, WorkItem *items) {
+    const int64_t nvalid = (int64_t)counts->ngrid;
+    auto run_end = [&](int64_t r) { return r + 1 < nruns ? (int64_t)rstart[r + 1] : nvalid; };
+    auto in = [&](int64_t r) -> unsigned long long {
+        const int64_t rs = rstart[r];
+        unsigned long long c = 0, h = 0;
+        run_pieces(rs, run_end(r), tstart[keys[rs] >> 12], item_max, [&](int64_t a, int64_t b, bool starts) {
+            h += starts;
+            c += (unsigned long long)((b - a + chunk_max - 1) / chunk_max);
+        });
+        return c | (h << 31);
+    };
+    // a piece's chunks step threads at a time from the first-th; bits above the chunk index
+    auto piece_chunks = [&](uint32_t cell, int64_t c, int64_t a, int64_t b, int first, int step) {
+        const uint32_t lu = cell & 63u, lv = cell >> 6;
+        const uint64_t color = ((lu >> 1) & 3u) * 7u + (lv % 7u);
+        const int nc = (int)((b - a + chunk_max - 1) / chunk_max);
+        for (int j = first; j < nc; j += step) {
+            const int64_t q = a + (int64_t)j * chunk_max;
+            const int len = (int)min((int64_t)chunk_max, b - q), cls = chunk_max - len;
+            const int bin = min(cls * (1 << LENBIN_BITS) / chunk_max, (1 << LENBIN_BITS) - 1);
+            ckey[c + j] = ((((((uint64_t)bin << 6) | color) << lbits) | (uint64_t)cls) << jbits) | (uint64_t)j;
+            craw[c + j] = make_uint2((uint32_t)q, cell | ((uint32_t)len << 16));
+        }
+        return nc;
+    };
+    // A run of more than EM_LONG chunks is left to a warp (a dense cell's has thousands).
+    constexpr int EM_LONG = 4;
+    struct LongRun {
+        uint32_t rs, re, ts, cell, chunk;
+    };
+    __shared__ LongRun lrun[SC_T * SC_R];
+    __shared__ int nlong;
+    if (threadIdx.x == 0) nlong = 0;
+    auto out = [&](int64_t r, unsigned long long cnt, unsigned long long before) {
+        const int64_t rs = rstart[r];
+        const uint32_t k = keys[rs];
+        int64_t c = (int64_t)(before & 0x7FFFFFFFull), nit = (int64_t)(before >> 31);
+        const int64_t nc = (int64_t)(cnt & 0x7FFFFFFFull);
+        // (sums of a look-back that gave up: nothing is written outside the arrays)
+        if (c + nc > max_chunks || nit + (int64_t)(cnt >> 31) > max_items) return;
+        const bool is_long = nc > EM_LONG;
+        const int64_t re = run_end(r), ts = tstart[k >> 12];
+        if (is_long)
+            lrun[atomicAdd(&nlong, 1)] = LongRun{(uint32_t)rs, (uint32_t)re, (uint32_t)ts, k & 4094u, (uint32_t)c};
+        run_pieces(rs, re, ts, item_max, [&](int64_t a, int64_t b, bool starts) {
+            if (starts) {
+                WorkItem wi;
+                wi.tile = (int32_t)(k >> 12);
+                wi.cbeg = (int32_t)c;
+                wi.vbeg = (int32_t)a;
+                wi.cend = wi.vend = wi.dense = wi.r0 = 0;
+                wi.rstep = 1;
+                items[nit++] = wi;
+            }
+            c += is_long ? (b - a + chunk_max - 1) / chunk_max : piece_chunks(k & 4094u, c, a, b, 0, 1);
+        });
+    };
+    lb_scan_tile<SC_T, SC_R>(nruns, words, &counts->emit.next, &counts->emit.total, &counts->fail, in, out);
+    __syncthreads();
+    for (int e = threadIdx.x >> 5; e < nlong; e += SC_T / 32) {
+        const LongRun r = lrun[e];
+        int64_t c = r.chunk;
+        run_pieces(r.rs, r.re, r.ts, item_max,
+                   [&](int64_t a, int64_t b, bool) { c += piece_chunks(r.cell, c, a, b, threadIdx.x & 31, 32); });
+    }
 }
 
-__global__ void k_chunk_final(const uint64_t *__restrict__ ckey, const uint32_t *__restrict__ cval,
-                              const uint32_t *__restrict__ cstart, const uint32_t *__restrict__ keys,
-                              int64_t nchunks, int64_t nvalid, int shift_item, uint2 *chunks,
-                              uint32_t *clen, WorkItem *items) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    uint32_t orig = cval[c];
-    uint32_t st = cstart[orig];
-    uint32_t en = (int64_t)orig + 1 < nchunks ? cstart[orig + 1] : (uint32_t)nvalid;
-    uint32_t cell = keys[st] & 4094u;
-    chunks[c] = make_uint2(st, cell | ((en - st) << 16));
-    clen[c] = en - st;
-    uint32_t it = (uint32_t)(ckey[c] >> shift_item);
-    if (c == 0 || (uint32_t)(ckey[c - 1] >> shift_item) != it) items[it].cbeg = (int32_t)c;
-    if (c == nchunks - 1 || (uint32_t)(ckey[c + 1] >> shift_item) != it) items[it].cend = (int32_t)(c + 1);
-}
-
-// a work item's first visibility: its first chunk's (new) start
-__global__ void k_item_vbeg(const uint2 *__restrict__ chunks, int64_t nitems, WorkItem *items) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nitems) return;
-    items[t].vbeg = (int32_t)chunks[items[t].cbeg].x;
-}
-
-// dense flag of each work item: its tile's items (contiguous, sorted by tile) together
-// hold >= DENSE_TILE_VIS visibilities
 // Raw-grid cores of the compensation plane: the footprint of a tile (tu, tv) (its 64x64
 // cells and 3-cell halo, raw rows [64 tv - 3, 64 tv + 67), raw indices [64 tu - 2,
 // 64 tu + 68)) lies in cores (tu, tv), (tu+1, tv), (tu, tv+1), (tu+1, tv+1), where core
 // (cu, cv) is raw rows [64 cv - 3, 64 cv + 61) x raw indices [64 cu - 2, 64 cu + 62).
-__global__ void k_core_lo(const WorkItem *items, int64_t nitems, int ntu, uint8_t *core) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nitems || !items[t].dense) return;
-    const int tu = items[t].tile % ntu, tv = items[t].tile / ntu, ncu = ntu + 1;
+__device__ __forceinline__ void mark_cores(int tile, int ntu, uint8_t *core) {
+    const int tu = tile % ntu, tv = tile / ntu, ncu = ntu + 1;
     core[tv * ncu + tu] = 1;
     core[tv * ncu + tu + 1] = 1;
     core[(tv + 1) * ncu + tu] = 1;
     core[(tv + 1) * ncu + tu + 1] = 1;
 }
 
-__global__ void k_item_dense(WorkItem *items, int64_t nitems) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Each item's ends, its dense flag (its tile's items, contiguous, hold >= DENSE_TILE_VIS
+// visibilities together), the cores of a dense tile, and its entries of the launch list:
+// every item once, or once per part with its rounds dealt out.  Where no item is larger than a
+// part the list is the items in their own order, neighbouring tiles together (64.7 million
+// visibilities, gridding in an order that the blocks' timing made: 700 -> 727 us); smaller
+// plans' entries are appended in any order.
+__global__ void k_item_finish(WorkItem *items, int64_t nitems, int64_t nchunks, int64_t nvalid, int ntu, uint8_t *core,
+                              int item_max, int part, WorkItem *parts,
+                              unsigned long long *nparts) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nitems) return;
     const int32_t tile = items[t].tile;
     int64_t lo = 0, hi = t;  // first item of the tile
@@ -337,18 +453,19 @@ __global__ void k_item_dense(WorkItem *items, int64_t nitems) {
         const int64_t mid = (lo + hi) / 2;
         if (items[mid].tile <= tile) lo = mid + 1; else hi = mid;
     }
-    items[t].dense = (int64_t)items[lo - 1].vend - items[first].vbeg >= DENSE_TILE_VIS;
-}
-
-// The launch list: every item once, or once per part with its rounds dealt out.  The list's
-// order does not matter (teams take entries from a counter), so entries are appended.
-__global__ void k_item_parts(const WorkItem *__restrict__ items, int64_t nitems, int part, WorkItem *parts,
-                             unsigned long long *nparts) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nitems) return;
+    const int64_t end = lo < nitems ? items[lo].vbeg : nvalid;
     WorkItem it = items[t];
-    const int np = item_parts(it, part);
-    const unsigned long long at = atomicAdd(nparts, (unsigned long long)np);
+    it.cend = t + 1 < nitems ? items[t + 1].cbeg : (int32_t)nchunks;
+    it.vend = t + 1 < nitems ? items[t + 1].vbeg : (int32_t)nvalid;
+    it.dense = end - items[first].vbeg >= DENSE_TILE_VIS;
+    items[t].cend = it.cend;
+    items[t].vend = it.vend;
+    items[t].dense = it.dense;
+    if (it.dense) mark_cores(tile, ntu, core);
+    const int np = item_max <= part ? 1 : item_parts(it, part);
+    const unsigned long long at =
+        item_max <= part ? (unsigned long long)t : atomicAdd(nparts, (unsigned long long)np);
+    if (item_max <= part && t == 0) *nparts = (unsigned long long)nitems;
     it.rstep = np;
     for (int k = 0; k < np; k++) {
         it.r0 = k;
@@ -356,10 +473,68 @@ __global__ void k_item_parts(const WorkItem *__restrict__ items, int64_t nitems,
     }
 }
 
-__global__ void k_item_vend(WorkItem *items, int64_t nitems, int64_t nvalid) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nitems) return;
-    items[t].vend = t + 1 < nitems ? items[t + 1].vbeg : (int32_t)nvalid;
+// One block per work item: its chunks sorted by their keys in shared memory (bitonic), and
+// their places in the plan, which follow one another from the item's first visibility.  An
+// item has at most 2048 cell pairs and item_max / chunk_max longer runs' chunks, so with the
+// default sizes every item fits; one with more than OR_MAX chunks keeps position order.  The
+// device-wide radix sort of 64-bit keys that this replaces took 7 passes of 5 launches.
+constexpr int OR_MAX = 4096, OR_T = 256;
+__global__ void __launch_bounds__(OR_T) k_item_order(const WorkItem *__restrict__ items, int64_t nitems,
+                                                     const uint64_t *__restrict__ ckey,
+                                                     const uint2 *__restrict__ craw, uint2 *chunks, uint32_t *csrc) {
+    __shared__ uint64_t sk[OR_MAX];
+    __shared__ uint32_t wsum[OR_T / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const WorkItem it = items[blockIdx.x];
+    const int m = it.cend - it.cbeg;
+    const bool sorted = m <= OR_MAX;
+    if (sorted) {
+        int n = 2;
+        while (n < m) n <<= 1;
+        for (int i = t; i < n; i += OR_T) sk[i] = i < m ? (ckey[it.cbeg + i] << 16) | (uint32_t)i : ~0ull;
+        __syncthreads();
+        for (int k = 2; k <= n; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int i = t; i < n / 2; i += OR_T) {
+                    const int a = 2 * i - (i & (j - 1)), b = a + j;  // the pair (a, a ^ j), a's bit j clear
+                    const uint64_t x = sk[a], y = sk[b];
+                    if ((x > y) == ((a & k) == 0)) {
+                        sk[a] = y;
+                        sk[b] = x;
+                    }
+                }
+                // pairs closer than a warp's span stay in the warp's own stretch
+                if (j > 32 || (j == 1 && k < n)) __syncthreads(); else __syncwarp();
+            }
+        __syncthreads();
+    }
+    uint32_t at = (uint32_t)it.vbeg;
+    for (int base = 0; base < m; base += OR_T) {
+        const int p = base + t;
+        uint2 c = make_uint2(0u, 0u);
+        if (p < m) c = craw[it.cbeg + (sorted ? (int)(sk[p] & 0xFFFFu) : p)];
+        const uint32_t len = c.y >> 16;
+        uint32_t x = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        uint32_t pre = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < OR_T / 32; w++) {
+            pre += w < warp ? wsum[w] : 0u;
+            all += wsum[w];
+        }
+        if (p < m) {
+            chunks[it.cbeg + p] = make_uint2(at + pre + x - len, c.y);
+            csrc[it.cbeg + p] = c.x;
+        }
+        at += all;
+        __syncthreads();
+    }
 }
 
 int bits_for(int64_t maxval) {
@@ -399,6 +574,16 @@ int sde_plan_destroy(sde_plan *pl) {
     for (void *p : ptrs) ctx_free(ctx, p, 0);
     ctx->bytes -= pl->bytes;
     delete pl;
+    return SDE_OK;
+}
+
+static int read_counts(sde_ctx *ctx, const PlanCounts *dev, PlanCounts *host) {
+    static_assert(sizeof(PlanCounts) <= H_SMALL_BYTES, "counts fit the pinned buffer");
+    SDE_TRY(ctx_read_small(ctx, ctx->stream, host, dev, sizeof *host));
+    if (host->fail) {
+        sde_set_error("plan: a device wait timed out");
+        return SDE_ETIMEDOUT;
+    }
     return SDE_OK;
 }
 
@@ -498,53 +683,44 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
         gp.ntu = pl->ntu;
         gp.twopi = (double)(8.0f * atanf(1.0f));  // TWOPI = 8 * ATAN(1.0), REAL (grdh2d.f:91)
 
-        uint32_t *keys, *vals, *ktmp, *vtmp, *exc_list;
+        uint32_t *keys, *vals, *ktmp, *vtmp, *exc_list, *rstart, *tstart;
         PlanRecU *rec_u;
-        unsigned long long *counts;
+        PlanCounts *counts;
         PL_TRY(ctx_scratch(ctx, "pl_keys", 4 * n, (void **)&keys));
         PL_TRY(ctx_scratch(ctx, "pl_vals", 4 * n, (void **)&vals));
         PL_TRY(ctx_scratch(ctx, "pl_ktmp", 4 * n, (void **)&ktmp));
         PL_TRY(ctx_scratch(ctx, "pl_vtmp", 4 * n, (void **)&vtmp));
         PL_TRY(ctx_scratch(ctx, "pl_exclist", 4 * n, (void **)&exc_list));
         PL_TRY(ctx_scratch(ctx, "pl_rec", sizeof(PlanRecU) * n, (void **)&rec_u));
-        PL_TRY(ctx_scratch(ctx, "pl_counts", 64, (void **)&counts));
-        PL_CUDA(cudaMemsetAsync(counts, 0, 64, st));
+        const int64_t ntiles = (int64_t)pl->ntu * pl->ntv, nscan = scan_tiles((int64_t)n);
+        const size_t count_bytes = sizeof(PlanCounts) + 2 * 8 * (size_t)nscan;
+        PL_TRY(ctx_scratch(ctx, "pl_counts", count_bytes, (void **)&counts));
+        unsigned long long *words = reinterpret_cast<unsigned long long *>(counts + 1);
+        PL_TRY(ctx_scratch(ctx, "pl_rstart", 4 * n, (void **)&rstart));
+        PL_TRY(ctx_scratch(ctx, "pl_tstart", 4 * (size_t)ntiles, (void **)&tstart));
+        PL_CUDA(cudaMemsetAsync(counts, 0, count_bytes, st));
         const int T = 256;
         if (nvis > 0) {
-            k_plan_geom<<<ceil_div(nvis, T), T, 0, st>>>(gp, du, dv, dw, dvis, dwt, nvis, keys, vals,
-                                                       rec_u, exc_list, counts);
+            k_plan_geom<<<ceil_div(nvis, GE_T * GE_PER), GE_T, 0, st>>>(gp, du, dv, dw, dvis, dwt, nvis, keys, rec_u, exc_list,
+                                                       counts);
             PL_CUDA(cudaGetLastError());
         }
-        int64_t ntiles = (int64_t)pl->ntu * pl->ntv;
         int kbits = bits_for((ntiles << 12) + 1);
         if (kbits > 32) {
             sde_set_error("plan: grid too large for 32-bit tile keys");
             rc = SDE_EINVAL;
             goto fail;
         }
-        if (nvis > 0) PL_TRY(launch_radix_sort_u32(ctx, keys, vals, nvis, kbits, ktmp, vtmp));
-        // run heads of the sorted keys (0 past the gridded visibilities) and their count, read
-        // back with the visibility counts: one wait for both
-        uint32_t *head, *ridx, *tot;
-        PL_TRY(ctx_scratch(ctx, "pl_runhead", 4 * n, (void **)&head));
-        PL_TRY(ctx_scratch(ctx, "pl_runidx", 4 * n, (void **)&ridx));
-        PL_TRY(ctx_scratch(ctx, "pl_tot", 16, (void **)&tot));
         if (nvis > 0) {
-            k_run_heads<<<ceil_div(nvis, T), T, 0, st>>>(keys, counts, nvis, head);
+            PL_TRY(launch_radix_sort_u32(ctx, &keys, nullptr, &vals, nvis, kbits, ktmp, vtmp, &counts->fail));
+            k_runs<<<ceil_div(nvis, RU_T * RU_R), RU_T, 0, st>>>(keys, counts, nvis, words, rstart, tstart);
             PL_CUDA(cudaGetLastError());
-            PL_TRY(launch_exclusive_scan_u32(ctx, head, ridx, nvis, tot));
-        } else {
-            PL_CUDA(cudaMemsetAsync(tot, 0, 16, st));
         }
-        unsigned long long hc[3] = {0, 0, 0};
-        uint32_t hruns = 0;
-        PL_CUDA(cudaMemcpyAsync(ctx->h_small, counts, sizeof hc, cudaMemcpyDeviceToHost, st));
-        PL_CUDA(cudaMemcpyAsync(ctx->h_small + sizeof hc, tot, sizeof hruns, cudaMemcpyDeviceToHost, st));
-        PL_CUDA(cudaStreamSynchronize(st));
-        memcpy(hc, ctx->h_small, sizeof hc);
-        memcpy(&hruns, ctx->h_small + sizeof hc, sizeof hruns);
-        const int64_t nvalid = (int64_t)hc[0], nexc = (int64_t)hc[1];
-        pl->nuntouched = nvis - (int64_t)hc[2];
+        // the counts and the number of runs: one wait for both
+        PlanCounts hc;
+        PL_TRY(read_counts(ctx, counts, &hc));
+        const int64_t nvalid = (int64_t)hc.ngrid, nexc = (int64_t)hc.nexc;
+        pl->nuntouched = nvis - (int64_t)hc.npos;
         pl->nvis = nvalid;
         pl->nexc = nexc;
         const size_t nv1 = (size_t)(nvalid > 0 ? nvalid : 1);
@@ -569,83 +745,47 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
         }
         // runs, chunks, work items
         if (nvalid > 0) {
-            const int64_t nruns = hruns;
-            uint32_t *rstart, *nch, *nih, *cbase, *ibase;
-            int32_t *tstart;
-            PL_TRY(ctx_scratch(ctx, "pl_rstart", 4 * (size_t)nruns, (void **)&rstart));
-            PL_TRY(ctx_scratch(ctx, "pl_tstart", 4 * (size_t)nruns, (void **)&tstart));
-            PL_TRY(ctx_scratch(ctx, "pl_nch", 4 * (size_t)nruns, (void **)&nch));
-            PL_TRY(ctx_scratch(ctx, "pl_nih", 4 * (size_t)nruns, (void **)&nih));
-            PL_TRY(ctx_scratch(ctx, "pl_cbase", 4 * (size_t)nruns, (void **)&cbase));
-            PL_TRY(ctx_scratch(ctx, "pl_ibase", 4 * (size_t)nruns, (void **)&ibase));
-            k_run_compact<<<ceil_div(nvalid, T), T, 0, st>>>(head, ridx, counts, rstart);
-            PL_CUDA(cudaGetLastError());
-            k_run_tilehead<<<ceil_div(nruns, T), T, 0, st>>>(keys, rstart, nruns, tstart);
-            PL_CUDA(cudaGetLastError());
-            PL_TRY(launch_inclusive_max_scan_i32(ctx, tstart, tstart, nruns));
-            k_run_counts<<<ceil_div(nruns, T), T, 0, st>>>(rstart, tstart, nruns, nvalid, pl->item_max,
-                                                         pl->chunk_max, nch, nih);
-            PL_CUDA(cudaGetLastError());
-            PL_TRY(launch_exclusive_scan_u32(ctx, nih, ibase, nruns, tot + 1));
-            PL_TRY(launch_exclusive_scan_u32(ctx, nch, cbase, nruns, tot + 2));
-            uint32_t htot[2];
-            PL_TRY(ctx_read_small(ctx, st, htot, tot + 1, sizeof htot));
-            const int64_t nitems = htot[0], nchunks = htot[1];
-            pl->nitems = nitems;
-            pl->nchunks = nchunks;
-            PL_TRY(plan_alloc(pl, (void **)&pl->items, sizeof(WorkItem) * (size_t)nitems));
-            PL_TRY(plan_alloc(pl, (void **)&pl->chunks, sizeof(uint2) * (size_t)nchunks));
-            uint64_t *ckey, *cktmp;
-            uint32_t *cval, *cvtmp, *cstart;
-            PL_TRY(ctx_scratch(ctx, "pl_ckey", 8 * (size_t)nchunks, (void **)&ckey));
-            PL_TRY(ctx_scratch(ctx, "pl_cktmp", 8 * (size_t)nchunks, (void **)&cktmp));
-            PL_TRY(ctx_scratch(ctx, "pl_cval", 4 * (size_t)nchunks, (void **)&cval));
-            PL_TRY(ctx_scratch(ctx, "pl_cvtmp", 4 * (size_t)nchunks, (void **)&cvtmp));
-            PL_TRY(ctx_scratch(ctx, "pl_cstart", 4 * (size_t)nchunks, (void **)&cstart));
+            // at most one item per tile that has a run and one more per item_max visibilities; a
+            // chunk per run, per item inside a run, and per chunk_max visibilities
+            const int64_t nruns = (int64_t)hc.runs.total;
+            const int64_t max_items = std::min(ntiles, nruns) + nvalid / pl->item_max;
+            const int64_t max_chunks = nruns + max_items + nvalid / pl->chunk_max;
+            uint64_t *ckey;
+            uint2 *craw;
+            uint32_t *csrc;
+            PL_TRY(ctx_scratch(ctx, "pl_ckey", 8 * (size_t)max_chunks, (void **)&ckey));
+            PL_TRY(ctx_scratch(ctx, "pl_craw", 8 * (size_t)max_chunks, (void **)&craw));
+            PL_TRY(ctx_scratch(ctx, "pl_csrc", 4 * (size_t)max_chunks, (void **)&csrc));
+            PL_TRY(plan_alloc(pl, (void **)&pl->items, sizeof(WorkItem) * (size_t)max_items));
             const int jbits = bits_for(pl->item_max / pl->chunk_max);
             const int lbits = bits_for(pl->chunk_max - 1);
-            k_run_emit<<<ceil_div(nruns, T), T, 0, st>>>(keys, rstart, tstart, nruns, nvalid, cbase, ibase,
-                                                       pl->item_max, pl->chunk_max, lbits, jbits, ckey,
-                                                       cval, cstart, pl->items);
+            k_run_emit<<<ceil_div(nruns, SC_T * SC_R), SC_T, 0, st>>>(
+                keys, counts, rstart, tstart, nruns, pl->item_max, pl->chunk_max, lbits, jbits, max_items, max_chunks,
+                words + nscan, ckey, craw, pl->items);
             PL_CUDA(cudaGetLastError());
-            k_chunk_len<<<ceil_div(nchunks, T), T, 0, st>>>(cstart, nchunks, nvalid, pl->chunk_max,
-                                                          jbits + 12, 6 + lbits + jbits + 12, ckey);
-            PL_CUDA(cudaGetLastError());
-            const int shift_item = LENBIN_BITS + 6 + lbits + jbits + 12;
-            const int cbits = shift_item + bits_for(nitems);
-            PL_TRY(launch_radix_sort_u64(ctx, ckey, cval, nchunks, cbits, cktmp, cvtmp));
-            uint32_t *clen, *cpos;
-            PL_TRY(ctx_scratch(ctx, "pl_clen", 4 * (size_t)nchunks, (void **)&clen));
-            PL_TRY(ctx_scratch(ctx, "pl_cpos", 4 * (size_t)nchunks, (void **)&cpos));
-            k_chunk_final<<<ceil_div(nchunks, T), T, 0, st>>>(ckey, cval, cstart, keys, nchunks,
-                                                            nvalid, shift_item, pl->chunks, clen,
-                                                            pl->items);
-            PL_CUDA(cudaGetLastError());
-            // chunk order: each chunk's new start, then one gather of the caller-order sectors
-            PL_TRY(launch_exclusive_scan_u32(ctx, clen, cpos, nchunks, nullptr));
-            k_plan_gather<<<ceil_div(nchunks, T / 32), T, 0, st>>>(vals, cpos, nchunks, pl->chunks, rec_u,
-                                                                 pl->fobs, pl->rec, pl->wt, pl->gdd,
-                                                                 pl->orig, pl->rot, pl->gconj,
-                                                                 nexc > 0 ? pl->exc : nullptr);
-            PL_CUDA(cudaGetLastError());
-            k_item_vbeg<<<ceil_div(nitems, T), T, 0, st>>>(pl->chunks, nitems, pl->items);
-            PL_CUDA(cudaGetLastError());
-            k_item_vend<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, nvalid);
-            PL_CUDA(cudaGetLastError());
-            k_item_dense<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems);
-            PL_CUDA(cudaGetLastError());
+            PL_TRY(read_counts(ctx, counts, &hc));
+            const int64_t nitems = (int64_t)(hc.emit.total >> 31), nchunks = (int64_t)(hc.emit.total & 0x7FFFFFFFull);
+            pl->nitems = nitems;
+            pl->nchunks = nchunks;
+            PL_TRY(plan_alloc(pl, (void **)&pl->chunks, sizeof(uint2) * (size_t)nchunks));
             // an item has at most ceil(visibilities / part) entries
             const int part = part_size(nvis);
             pl->parts_max = nitems + nvalid / part;
             PL_TRY(plan_alloc(pl, (void **)&pl->parts, sizeof(WorkItem) * (size_t)(pl->parts_max + 1)));
             pl->nparts = reinterpret_cast<unsigned long long *>(pl->parts + pl->parts_max);
             PL_CUDA(cudaMemsetAsync(pl->nparts, 0, sizeof(unsigned long long), st));
-            k_item_parts<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, part, pl->parts, pl->nparts);
-            PL_CUDA(cudaGetLastError());
             const size_t ncore = (size_t)(pl->ntu + 1) * (pl->ntv + 1);
             PL_TRY(plan_alloc(pl, (void **)&pl->core_lo, ncore));
             PL_CUDA(cudaMemsetAsync(pl->core_lo, 0, ncore, st));
-            k_core_lo<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, pl->ntu, pl->core_lo);
+            k_item_finish<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, nchunks, nvalid, pl->ntu, pl->core_lo,
+                                                           pl->item_max, part, pl->parts, pl->nparts);
+            PL_CUDA(cudaGetLastError());
+            k_item_order<<<(unsigned)nitems, OR_T, 0, st>>>(pl->items, nitems, ckey, craw, pl->chunks, csrc);
+            PL_CUDA(cudaGetLastError());
+            k_plan_gather<<<ceil_div(nchunks, GA_CHUNKS), GA_T, 0, st>>>(vals, pl->chunks, csrc, nchunks, rec_u,
+                                                                       pl->fobs, pl->rec, pl->wt, pl->gdd, pl->orig,
+                                                                       pl->rot, pl->gconj,
+                                                                       nexc > 0 ? pl->exc : nullptr);
             PL_CUDA(cudaGetLastError());
         }
         // gridding function: the context's 'SF' table
