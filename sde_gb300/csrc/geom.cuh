@@ -104,6 +104,15 @@ GEOM_HD float bits_f(int i) {
     return x;
 #endif
 }
+GEOM_HD long long d_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return __double_as_longlong(x);
+#else
+    long long i;
+    memcpy(&i, &x, 8);
+    return i;
+#endif
+}
 GEOM_HD void dsincos(double x, double *s, double *c) {
 #ifdef __CUDA_ARCH__
     sincos(x, s, c);
@@ -345,19 +354,53 @@ GEOM_HD bool axis_near_identity(float x, float scale, float sgn, int origin, flo
     return true;
 }
 
+constexpr float TWOPI_R = 6.2831855f;  // TWOPI = 8 * ATAN(1.0), REAL (grd/grdh2d.f:91)
+
+// The REAL SIN of GRDH2D/GRDDEH2D's phase, SNGL(TWOPI*(S*W - W)) in DOUBLE, for a diagonal
+// entry S = 1 + k 2^-53 of SHIFT with |k| <= 8, by integers: W has 24 significant bits, M, so
+// in units of W's spacing as a DOUBLE, S*W = W + M k / 2^24 before rounding, and S*W - W is
+// that quotient rounded to nearest (its ties to even, as W is an even number of units).  Where
+// W is a power of two and k < 0, S*W lies in the binade below, of half the spacing, and k/2
+// is exact.  The difference times TWOPI, a REAL, fits a DOUBLE, so the phase is the REAL
+// product TWOPI * (difference in units), scaled.  False for other S, and for W so small or
+// large that the scaling leaves the REALs or the phase is not below 2^-27 (where COS is 1 and
+// SIN the phase itself).
+GEOM_HD bool tiny_phase(double s, float w, float &sn) {
+    const long long ulps = d_bits(s) - 0x3FF0000000000000ll;  // 2^-52 above 1, 2^-53 below
+    const long long kl = ulps > 0 ? 2 * ulps : ulps;
+    sn = 0.0f;
+    if (kl == 0 || w == 0.0f) return true;
+    if (kl < -8 || kl > 8) return false;
+    const float aw = fabsf(w);
+    if (!(aw >= 0x1p-60f && aw < 0x1p21f)) return false;
+    const int k = (int)kl, b = f_bits(aw);
+    const int m = (b & 0x007FFFFF) | 0x00800000;
+    const int a = m * (k < 0 ? -k : k), rem = a & 0x00FFFFFF;
+    int n = a >> 24;
+    n += rem > 0x00800000 || (rem == 0x00800000 && (n & 1));
+    float units = (float)n;
+    if (m == 0x00800000 && k < 0) units = 0.5f * (float)(-k);
+    if ((k < 0) != (w < 0.0f)) units = -units;
+    // TWOPI * units, times 2^(E - 52) for aw in [2^E, 2^(E+1))
+    sn = fmul(fmul(TWOPI_R, units), bits_f((((b >> 23) - 52) << 23)));
+    return fabsf(sn) < 0x1p-27f;
+}
+
 // geom_dd's results from FP32 arithmetic for a SHIFT within 2^-50 of the identity on the u
 // and v axes (the identity, and CRDSHIFT's matrix for a phase centre at the tangent point,
 // whose diagonal sin^2 + cos^2 misses 1 by an ulp) and zero offsets; false when some value
 // lies too close to a rounding boundary to decide (axis_near_identity) or the phase is not
-// tiny.  The phase keeps its two DOUBLE products.
+// tiny.
 GEOM_HD bool geom_near_identity(const GParams &p, float uf, float vf, float wf, float vr, float vi, GGeo &g) {
-    double cd = 1.0, sd = 0.0;
+    float rs = 0.0f;  // COS is 1
     if (!p.identity) {
-        const double wg = (double)wf;
-        const double wl = p.diagonal ? dmul(p.s[8], wg) : wg;
-        const double ph = dmul(p.twopi, dsub(wl, wg));
-        if (!(fabs(ph) < 0x1p-27)) return false;
-        sd = ph;
+        if (!p.diagonal) return false;
+        if (!tiny_phase(p.s[8], wf, rs)) {
+            const double wg = (double)wf;
+            const double ph = dmul(p.twopi, dsub(dmul(p.s[8], wg), wg));
+            if (!(fabs(ph) < 0x1p-27)) return false;
+            rs = d2f(ph);
+        }
     }
     const bool conj = fmul(p.uscale, uf) > 0.0f;  // sign of USCALE*U, exact
     const float sgn = conj ? 1.0f : -1.0f;
@@ -366,10 +409,10 @@ GEOM_HD bool geom_near_identity(const GParams &p, float uf, float vf, float wf, 
     if (!axis_near_identity(vf, p.vscale, sgn, p.vorigin, (float)p.osamp, g.nvc, g.dvg, cv)) return false;
     g.sane = true;
     g.gc = conj;
-    const float rc = d2f(cd), rs = d2f(sd);
+    const float rc = 1.0f;
     g.dg = degrid_cell_r(p, cu, cv, conj, rc, rs);
     if (p.doshift) {
-        const float c = rc, s = d2f(-sd);
+        const float c = rc, s = -rs;
         g.fr = fsub(fmul(vr, c), fmul(vi, s));
         g.fi = fadd(fmul(vr, s), fmul(vi, c));
         g.rc = rc;
