@@ -555,19 +555,32 @@ struct StPasses<LOGN, LOGN, INV, NT, T> {
 
 // Shapes: columns per CTA and threads for a column transform of length 2^LOGN, rows per CTA
 // and threads for a row transform of half-length 2^LOGH.
-template <int LOGN>
+//
+// Two shapes per length.  The wide one puts 4096 elements on a CTA; a single 256^2 or 512^2
+// image is then 8 to 33 CTAs, and each pass waits for one SM's chain of loads, butterflies
+// and divisions.  FEW takes 512 elements of rows or 1024 of columns (whole 32-byte sectors of
+// a grid row where the length leaves four columns); the butterflies and their order are the
+// same, so are the results.  512^2 grids, wide -> FEW: row c2r 17.8 -> 7.6 us, row r2c 13.4 ->
+// 6.2, columns 7.0 -> 6.4; 256^2: 18.7 -> 7.5 and 6.9 -> 5.7.
+// FEW is taken while the wide shape has fewer CTAs than two per SM: 8 grids of 256^2 (64
+// wide CTAs) 18.4 -> 7.9 us for the rows, but batches that fill the chip lose by it (1024^2
+// rows, 16 grids: 70 -> 83 us; columns 43 -> 57).
+constexpr int FEW_CTAS = 2 * 152, ROW_FEW = 512, COL_FEW = 1024;
+constexpr bool few_ctas(int ctas, int nbatch) { return ctas * nbatch < FEW_CTAS; }
+template <int LOGN, bool FEW>
 struct ColShape {
     static constexpr int N = 1 << LOGN;
-    static constexpr int CC = N >= 4096 ? 2 : (4096 / N > 64 ? 64 : 4096 / N);  // columns
+    static constexpr int E = FEW ? COL_FEW : 4096;  // elements per CTA
+    static constexpr int CC = 2 * N >= E ? 2 : (E / N > 64 ? 64 : E / N);  // columns
     static constexpr int T0 = CC * N / 16;
     static constexpr int T = T0 < 128 ? 128 : (T0 > 1024 ? 1024 : T0);
     static constexpr size_t SMEM = sizeof(float2) * (size_t)CC * N;
     static constexpr int MINB = 1024 / T;  // resident CTAs the kernel is built for (64 regs)
 };
-template <int LOGH>
+template <int LOGH, bool FEW>
 struct RowShape {
     static constexpr int H = 1 << LOGH;
-    static constexpr int ROWS = H >= 2048 ? 2 : 4096 / H;
+    static constexpr int ROWS = FEW ? (H >= ROW_FEW ? 1 : ROW_FEW / H) : (H >= 2048 ? 2 : 4096 / H);
     static constexpr int T0 = ROWS * H / 16;
     static constexpr int T = T0 < 128 ? 128 : (T0 > 1024 ? 1024 : T0);
     static constexpr size_t SMEM = sizeof(float2) * (size_t)ROWS * H + 16;  // + an mbarrier
@@ -575,12 +588,12 @@ struct RowShape {
 };
 
 // Column pass along v (as k_col_fft), CC columns per CTA read as 16-byte column pairs.
-template <int LOGN, bool INV>
-__global__ void __launch_bounds__(ColShape<LOGN>::T, ColShape<LOGN>::MINB)
+template <int LOGN, bool INV, bool FEW>
+__global__ void __launch_bounds__(ColShape<LOGN, FEW>::T, ColShape<LOGN, FEW>::MINB)
     k_col_fft_t(const __grid_constant__ FftBatch bt, int pitch, int nu, const float2 *__restrict__ tw,
                 int r0, int r1) {
     float2 *grid = bt.grid[blockIdx.y];
-    using S = ColShape<LOGN>;
+    using S = ColShape<LOGN, FEW>;
     constexpr int N = S::N, CC = S::CC, T = S::T;
     constexpr int LP = __builtin_ctz(CC) - 1;           // log2(column pairs per row)
     constexpr int TOTAL = N * CC / 2;                   // (row, pair) items
@@ -630,14 +643,14 @@ __global__ void __launch_bounds__(ColShape<LOGN>::T, ColShape<LOGN>::MINB)
 }
 
 // Row pass grid -> image (as k_row_c2r), ROWS rows per CTA, half-length 2^LOGH.
-template <int LOGH>
-__global__ void __launch_bounds__(RowShape<LOGH>::T, RowShape<LOGH>::MINB)
+template <int LOGH, bool FEW>
+__global__ void __launch_bounds__(RowShape<LOGH, FEW>::T, RowShape<LOGH, FEW>::MINB)
     k_row_c2r_t(const __grid_constant__ FftBatch bt, int pitch, int nx, int ny, int ibegy,
                 const float2 *__restrict__ tw, CorrParams cp) {
     const float2 *__restrict__ grid = bt.grid[blockIdx.y];
     const float *__restrict__ scale_dev = bt.scale[blockIdx.y];
     float *image = bt.image[blockIdx.y];
-    using S = RowShape<LOGH>;
+    using S = RowShape<LOGH, FEW>;
     constexpr int H = S::H, ROWS = S::ROWS, T = S::T, FNU = 2 * H;
     constexpr int TOTAL = ROWS * H;
     constexpr int PER = (TOTAL + T - 1) / T;
@@ -669,8 +682,15 @@ __global__ void __launch_bounds__(RowShape<LOGH>::T, RowShape<LOGH>::MINB)
     const float inv = 1.0f / (float)H;
     const int cu = (FNU + 1) / 2 - 1, ioff = (FNU - nx) / 2;
     const float sc = scale_dev ? 1.0f / *scale_dev : 1.0f;
-    for (int t = threadIdx.x; t < ROWS * nx; t += T) {
-        const int rr = t / nx, ix = t - rr * nx;
+    // (row, pixel) of t = threadIdx.x + k T by steps: no division inside the loop
+    const int dr = T / nx, dx = T - dr * nx;
+    int rr = (int)threadIdx.x / nx, ix = (int)threadIdx.x - rr * nx;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < ROWS * nx; t += T, rr += dr, ix += dx) {
+        if (ix >= nx) {
+            ix -= nx;
+            rr++;
+        }
         const int iy = iy0 + rr;
         if (iy >= ny) break;
         int n = ix + ioff - cu;
@@ -684,20 +704,20 @@ __global__ void __launch_bounds__(RowShape<LOGH>::T, RowShape<LOGH>::MINB)
 }
 
 // Row pass image -> grid (as k_row_r2c), ROWS rows per CTA, half-length 2^LOGH.
-template <int LOGH>
-__global__ void __launch_bounds__(RowShape<LOGH>::T, RowShape<LOGH>::MINB)
+template <int LOGH, bool FEW>
+__global__ void __launch_bounds__(RowShape<LOGH, FEW>::T, RowShape<LOGH, FEW>::MINB)
     k_row_r2c_t(const __grid_constant__ FftBatch bt, int nx, int ny, int ibegy,
                 const float2 *__restrict__ tw, CorrParams cp, int pitch, int *status) {
     const float *__restrict__ image = bt.image[blockIdx.y];
     float2 *grid = bt.grid[blockIdx.y];
-    using S = RowShape<LOGH>;
+    using S = RowShape<LOGH, FEW>;
     constexpr int H = S::H, ROWS = S::ROWS, T = S::T, FNU = 2 * H;
     constexpr int TOTAL = ROWS * H;
     constexpr int PER = (TOTAL + T - 1) / T;
     extern __shared__ __align__(16) float2 s[];
     const int cu = (FNU + 1) / 2 - 1, ioff = (FNU - nx) / 2;
     const int iy0 = blockIdx.x * ROWS;
-    if (ROWS == 2 && status) {
+    if (!FEW && ROWS == 2 && status) {
         // the CTA's image rows come in by bulk copy (row rr at floats [rr*FNU, rr*FNU+nx) of
         // s); every thread reads its inputs from there, then the FFT layout overwrites it
         // (measured: 0.099 -> 0.088 ms at 4096^2 against the L2-prefetch path below)
@@ -1267,47 +1287,69 @@ static bool row_pair_ok(int logh, const FftBatch &bt, int nbatch, int pitch, int
 }
 
 // Launchers for the compile-time shapes: false if the size has no instance.
+template <int LOGN, bool INV, bool FEW>
+cudaError_t launch_col_shape(const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw, int r0,
+                             int r1, cudaStream_t st) {
+    using S = ColShape<LOGN, FEW>;
+    cudaError_t e = cudaFuncSetAttribute(k_col_fft_t<LOGN, INV, FEW>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e != cudaSuccess) return e;
+    k_col_fft_t<LOGN, INV, FEW><<<dim3((unsigned)((nu + S::CC - 1) / S::CC), (unsigned)nbatch), S::T,
+                                  S::SMEM, st>>>(bt, pitch, nu, tw, r0, r1);
+    return cudaGetLastError();
+}
 template <int LOGN>
 cudaError_t launch_col_t(const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw,
                          bool inverse, int r0, int r1, cudaStream_t st) {
-    using S = ColShape<LOGN>;
-    const dim3 nb((unsigned)((nu + S::CC - 1) / S::CC), (unsigned)nbatch);
-    if (inverse) {
-        cudaError_t e = cudaFuncSetAttribute(k_col_fft_t<LOGN, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-        if (e != cudaSuccess) return e;
-        k_col_fft_t<LOGN, true><<<nb, S::T, S::SMEM, st>>>(bt, pitch, nu, tw, r0, r1);
-    } else {
-        cudaError_t e = cudaFuncSetAttribute(k_col_fft_t<LOGN, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-        if (e != cudaSuccess) return e;
-        k_col_fft_t<LOGN, false><<<nb, S::T, S::SMEM, st>>>(bt, pitch, nu, tw, r0, r1);
-    }
-    return cudaGetLastError();
+    const int cc = ColShape<LOGN, false>::CC;
+    if constexpr (LOGN < 12)
+        if (few_ctas((nu + cc - 1) / cc, nbatch))
+            return inverse ? launch_col_shape<LOGN, true, true>(bt, nbatch, pitch, nu, tw, r0, r1, st)
+                           : launch_col_shape<LOGN, false, true>(bt, nbatch, pitch, nu, tw, r0, r1, st);
+    return inverse ? launch_col_shape<LOGN, true, false>(bt, nbatch, pitch, nu, tw, r0, r1, st)
+                   : launch_col_shape<LOGN, false, false>(bt, nbatch, pitch, nu, tw, r0, r1, st);
 }
 
+template <int LOGH, bool FEW>
+cudaError_t launch_c2r_shape(const FftBatch &bt, int nbatch, int pitch, int nx, int ny, int ibegy,
+                             const float2 *tw, CorrParams cp, cudaStream_t st) {
+    using S = RowShape<LOGH, FEW>;
+    cudaError_t e = cudaFuncSetAttribute(k_row_c2r_t<LOGH, FEW>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e != cudaSuccess) return e;
+    k_row_c2r_t<LOGH, FEW><<<dim3((unsigned)((ny + S::ROWS - 1) / S::ROWS), (unsigned)nbatch), S::T,
+                             S::SMEM, st>>>(bt, pitch, nx, ny, ibegy, tw, cp);
+    return cudaGetLastError();
+}
 template <int LOGH>
 cudaError_t launch_c2r_t(const FftBatch &bt, int nbatch, int pitch, int nx, int ny, int ibegy,
                          const float2 *tw, CorrParams cp, cudaStream_t st) {
-    using S = RowShape<LOGH>;
-    cudaError_t e = cudaFuncSetAttribute(k_row_c2r_t<LOGH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)S::SMEM);
-    if (e != cudaSuccess) return e;
-    k_row_c2r_t<LOGH><<<dim3((unsigned)((ny + S::ROWS - 1) / S::ROWS), (unsigned)nbatch), S::T, S::SMEM,
-                        st>>>(bt, pitch, nx, ny, ibegy, tw, cp);
-    return cudaGetLastError();
+    const int rows = RowShape<LOGH, false>::ROWS;
+    if constexpr (LOGH < 12)
+        if (few_ctas((ny + rows - 1) / rows, nbatch))
+            return launch_c2r_shape<LOGH, true>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, st);
+    return launch_c2r_shape<LOGH, false>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, st);
 }
 
+template <int LOGH, bool FEW>
+cudaError_t launch_r2c_shape(const FftBatch &bt, int nbatch, int nx, int ny, int ibegy, const float2 *tw,
+                             CorrParams cp, int pitch, int *status, cudaStream_t st) {
+    using S = RowShape<LOGH, FEW>;
+    cudaError_t e = cudaFuncSetAttribute(k_row_r2c_t<LOGH, FEW>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e != cudaSuccess) return e;
+    k_row_r2c_t<LOGH, FEW><<<dim3((unsigned)((ny + S::ROWS - 1) / S::ROWS), (unsigned)nbatch), S::T,
+                             S::SMEM, st>>>(bt, nx, ny, ibegy, tw, cp, pitch, status);
+    return cudaGetLastError();
+}
 template <int LOGH>
 cudaError_t launch_r2c_t(const FftBatch &bt, int nbatch, int nx, int ny, int ibegy, const float2 *tw,
                          CorrParams cp, int pitch, int *status, cudaStream_t st) {
-    using S = RowShape<LOGH>;
-    cudaError_t e = cudaFuncSetAttribute(k_row_r2c_t<LOGH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)S::SMEM);
-    if (e != cudaSuccess) return e;
-    k_row_r2c_t<LOGH><<<dim3((unsigned)((ny + S::ROWS - 1) / S::ROWS), (unsigned)nbatch), S::T, S::SMEM,
-                        st>>>(bt, nx, ny, ibegy, tw, cp, pitch, status);
-    return cudaGetLastError();
+    const int rows = RowShape<LOGH, false>::ROWS;
+    if constexpr (LOGH < 11)  // two-row CTAs from H = 2048 on stage their rows by bulk copy
+        if (few_ctas((ny + rows - 1) / rows, nbatch))
+            return launch_r2c_shape<LOGH, true>(bt, nbatch, nx, ny, ibegy, tw, cp, pitch, status, st);
+    return launch_r2c_shape<LOGH, false>(bt, nbatch, nx, ny, ibegy, tw, cp, pitch, status, st);
 }
 
 #define SDE_LOG_CASES(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13)
