@@ -38,7 +38,8 @@ def _stale(lib, deps):
 def build(verbose=False, force=False, ptxas_info=False):
     os.makedirs(OUT, exist_ok=True)
     deps = [os.path.join(SRC, s) for s in SOURCES] + [
-        os.path.join(SRC, h) for h in ("common.cuh", "geom.cuh", "lookback.cuh")] + [os.path.join(HERE, "..", "include", "sde_gpu.h"),
+        os.path.join(SRC, h) for h in ("common.cuh", "geom.cuh", "lookback.cuh", "cluster_max.cuh")] + [
+        os.path.join(HERE, "..", "include", "sde_gpu.h"),
         os.path.abspath(__file__)]
     if not force and not _stale(LIB, deps):
         return LIB

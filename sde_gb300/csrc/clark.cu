@@ -5,33 +5,30 @@
 //   |residual| histogram of 1024 bins (PIXRABSH)               k_clark_hist
 //   the list limit (PIXFLIM, ARRFLIM, EXTSIDE)                 k_clark_limit
 //   the list of pixels above it, in storage order (PIX2DRLI)   k_clark_count / _scan / _emit
-//   the minor cycle on the list (PIX2DRCC)                     k_clark_minor: one cluster
-//   the components into the model image (PIX2DRMA)             k_clark_addcomp
+//   the minor cycle on the list and the components into the
+//   model image (PIX2DRCC, PIX2DRMA)                           k_clark_minor: one cluster
 //   residual = dirty - IFFT(FFT(model) * XFR) (IMGRESID)       FFTR2D passes + k_clark_cmul/_sub
 // The host reads back the cycle's scalars once per major cycle for IMGCCLEA's stop test.
 #include <string.h>
 
-#include <cooperative_groups.h>
-
+#include "cluster_max.cuh"
 #include "common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace {
 
 constexpr int CL_NB = 1024;        // histogram bins (arr/arrabshi.f:34 NB = 1024)
-constexpr int CL_T = 1024;         // minor-cycle threads per CTA
 constexpr int CL_CTAS = 8;         // minor-cycle CTAs: one thread-block cluster
-constexpr int CL_PER = 4;          // list entries per thread held in registers
-constexpr int CL_SLICE = CL_T * CL_PER;           // entries per CTA
-constexpr int CL_MAXNL = CL_CTAS * CL_SLICE;      // 32768
+constexpr int CL_T = 512;          // and their threads
+constexpr int CL_PER = 8;          // list entries per minor-cycle thread, at most
+constexpr int CL_MAXNL = CL_CTAS * CL_T * CL_PER;  // 32768
+constexpr int CL_ERR_WAIT = 4;     // ClarkState::err: a wait between the minor cycle's CTAs gave up
 constexpr int CL_CHUNK = 4096;     // pixels per block of the list compaction (256 x 16)
 
 struct ClarkState {
     unsigned int smax, smin;       // ordered encodings of the signed max / min (ARRSTAT)
     unsigned int amax, amin;       // |residual| max / min (non-negative float bits)
     float base, incr, slim;
-    int err;                       // 1 zero range, 2 too many points, 3 negative limit
+    int err;                       // 1 zero range, 2 too many points, 3 negative limit, CL_ERR_WAIT
     int anl, total;                // list length, pixels above the limit
     int pmpx, pmpy;                // beam-patch peak (1-based)
     float extside;
@@ -245,66 +242,48 @@ __global__ void __launch_bounds__(256) k_clark_emit(const float *__restrict__ re
     }
 }
 
-// PIXISAMA key: larger |v| first, then the smaller list index (pix/pixisama.f: the first
-// index whose |A| is strictly greater than every earlier one; 1 when all are zero)
-__device__ __forceinline__ unsigned long long isama_key(float v, int i) {
-    return ((unsigned long long)__float_as_uint(fabsf(v)) << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)i);
-}
-
-// pix/pix2drcc.f:66-140 with SPEED = 1 and GSUB = BSUB on a cluster of CL_CTAS CTAs.  CTA r
-// holds list entries r*CL_SLICE ..; its thread t holds CL_PER consecutive ones (storage order,
-// so spatially compact) in registers, their positions in shared memory (entry (t, j) at
-// spos[j*CL_T + t]), the beam patch in shared memory when it fits, and the bounding box of
-// its entries: an iteration whose beam patch misses the box leaves them alone, and a thread
-// rescans its local maximum only after one of its entries changed.  An iteration's argmax
-// (PIXISAMA: the largest |v|, then the first index): warp shuffles, one __syncthreads, the
-// CTA's best into its slot in CTA 0's shared memory, one cluster barrier, every warp reduces
-// the CL_CTAS slots.  Slots alternate between two sets, so no second barrier is needed.
-struct ClSlot {
-    unsigned long long key;
-    float val;
-    int pos;
-};
-
-__device__ __forceinline__ void slot_max(unsigned long long &k, float &v, int &p, int width) {
-    for (int d = width / 2; d > 0; d >>= 1) {
-        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, d);
-        const float ov = __shfl_xor_sync(0xffffffffu, v, d);
-        const int op = __shfl_xor_sync(0xffffffffu, p, d);
-        if (ok > k) {
-            k = ok;
-            v = ov;
-            p = op;
-        }
-    }
-}
-
+// pix/pix2drcc.f:66-140 with SPEED = 1 and GSUB = BSUB, and PIX2DRMA (pix/pix2drma.f:17-21), on
+// one cluster of CL_CTAS CTAs.  The list is spread over the threads, the same number of consecutive
+// entries each (storage order, so spatially compact), neighbouring warps' entries on different
+// CTAs: a beam patch touches a few rows of the list and its work spreads over the cluster.
+// Values, positions and the pixels' component sums stay in registers, the beam patch in shared
+// memory when it fits.  A thread whose entries' bounding box misses the patch skips the update;
+// a warp that changed nothing keeps its maximum.  Entries come in storage order, so PIXISAMA's
+// first index is the smallest flat pixel: the key of ClusterMax carries the position itself.
+// The pixel's thread adds its components to COMP's value in list order, as PIX2DRMA would.
+// An iteration is a latency chain (warp maximum, CTA barrier, remote store, slot maximum, patch
+// reads).  Measured an iteration on a 1024^2 window with 300 components: 0.98 us (0.93 with 16
+// CTAs of 256 threads, which need an opt-in cluster size); with 1024 threads a CTA, a cluster
+// barrier an iteration and the maximum by 64-bit shuffles it was 2.5 us, and one thread's
+// PIX2DRMA took another 52 us.
 template <bool PSF_SMEM>
-__global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_T, 1)
+__global__ void __launch_bounds__(CL_T, 1)
     k_clark_minor(const float *__restrict__ al, const int *__restrict__ pl, ClarkState *st,
-                  const float *__restrict__ psf_g, int pw, int ph, float gain, int nsub, int bsub,
-                  float flux, float *cl, int *cx, int *cy) {
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    extern __shared__ __align__(16) unsigned char smem[];
-    int *spos = reinterpret_cast<int *>(smem);
-    float *spsf = reinterpret_cast<float *>(smem + sizeof(int) * CL_SLICE);
-    __shared__ unsigned long long skey[2][32];
-    __shared__ float sval[2][32];
-    __shared__ int spo[2][32];
-    __shared__ ClSlot cslot[2][CL_CTAS];  // CTA 0's copy is the cluster's
+                  const float *__restrict__ psf_g, int pw, float gain, int nsub, int bsub,
+                  float flux, float *cl, int *cx, int *cy, float *comp, int logw) {
+    constexpr int C = CL_CTAS, T = CL_T;
+    extern __shared__ float spsf[];
+    __shared__ __align__(16) ClusterMax<C> cm;
+    __shared__ unsigned long long skey[T / 32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int anl = st->anl, base = rank * CL_SLICE;
-    float v[CL_PER];
+    uint32_t rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    cluster_max_init(&cm);
+    const int anl = st->anl, per = (anl + C * T - 1) / (C * T);
+    const int i0 = ((warp * C + (int)rank) * 32 + lane) * per;
+    float v[CL_PER], c[CL_PER];
+    int q[CL_PER];
+    unsigned mine = 0;  // entries with components
     int bx0 = 0x7FFF, bx1 = -1, by0 = 0x7FFF, by1 = -1;
 #pragma unroll
     for (int j = 0; j < CL_PER; j++) {
-        const int i = base + t * CL_PER + j;
-        const int q = i < anl ? pl[i] : (0x7FFF | (0x7FFF << 16));  // never inside the patch
-        v[j] = i < anl ? al[i] : 0.f;
-        spos[j * CL_T + t] = q;
-        if (i < anl) {
-            const int x = q & 0xFFFF, y = q >> 16;
+        v[j] = c[j] = 0.f;
+        q[j] = 0x7FFF | (0x7FFF << 16);  // no entry: never inside the patch
+        if (j < per && i0 + j < anl) {
+            q[j] = pl[i0 + j];
+            v[j] = al[i0 + j];
+            const int x = q[j] & 0xFFFF, y = q[j] >> 16;
+            c[j] = comp[((size_t)(y - 1) << logw) + (x - 1)];
             bx0 = min(bx0, x);
             bx1 = max(bx1, x);
             by0 = min(by0, y);
@@ -313,73 +292,50 @@ __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_T, 1)
     }
     const float *psf = psf_g;
     if (PSF_SMEM) {
-        for (int k = t; k < pw * ph; k += CL_T) spsf[k] = psf_g[k];
+        for (int k = t; k < pw * pw; k += T) spsf[k] = psf_g[k];
         psf = spsf;
     }
-    ClSlot *c0 = cluster.map_shared_rank(&cslot[0][0], 0);
-    cluster.sync();
+    __syncthreads();
     const float slim = st->slim;
     const int pmpx = st->pmpx, pmpy = st->pmpy;
     float tflux = st->tflux, smn = 0.f, maxres = 0.f;
-    int ansub = nsub, buf = 0;
-    unsigned long long lbest = 0ull;
-    float lbv = 0.f;
-    int lpos = 0;
-    bool rescan = true;
-    // the cluster's argmax: value into *val, packed position into *pos
-    auto argmax = [&](float *val, int *pos) {
-        if (rescan) {
-            lbest = 0ull;
-            lbv = 0.f;
-            lpos = 0;
+    int isub = bsub, ansub = nsub;
+    const int nabs = abs(nsub);
+    unsigned long long wk = 0ull;
+    bool changed = true, ok = true, gave_up = false;
+    for (int n = 0;; n++) {
+        if (__any_sync(0xffffffffu, changed)) {
+            // |v| compared by its bits: the order of the values, a NaN above all
+            unsigned la = 0u, lo = 0u;
 #pragma unroll
             for (int j = 0; j < CL_PER; j++) {
-                const unsigned long long k = isama_key(v[j], base + t * CL_PER + j);
-                if (k > lbest) {
-                    lbest = k;
-                    lbv = v[j];
-                    lpos = spos[j * CL_T + t];
+                const unsigned bits = __float_as_uint(v[j]), a = bits & 0x7FFFFFFFu;
+                const int idx = (((q[j] >> 16) - 1) << logw) + (q[j] & 0xFFFF) - 1;
+                const bool in = j < per && i0 + j < anl;
+                if (in && (lo == 0u || a > la)) {
+                    la = a;
+                    lo = ((unsigned)(INT32_MAX - idx) << 1) | (bits >> 31);
                 }
             }
-            rescan = false;
+            wk = warp_key_max(((unsigned long long)la << 32) | lo);
+            changed = false;
         }
-        unsigned long long k = lbest;
-        float bv = lbv;
-        int bp = lpos;
-        slot_max(k, bv, bp, 32);
-        if (lane == 0) {
-            skey[buf][warp] = k;
-            sval[buf][warp] = bv;
-            spo[buf][warp] = bp;
+        if (lane == 0) skey[warp] = wk;
+        if (__syncthreads_or(!ok)) {  // some warp's wait gave up: the whole CTA leaves
+            gave_up = true;
+            break;
         }
-        __syncthreads();
         if (warp == 0) {
-            k = skey[buf][lane];
-            bv = sval[buf][lane];
-            bp = spo[buf][lane];
-            slot_max(k, bv, bp, 32);
-            if (lane == 0) c0[buf * CL_CTAS + rank] = ClSlot{k, bv, bp};
+            const unsigned long long ck = warp_key_max(lane < T / 32 ? skey[lane] : 0ull);
+            if (lane < C) cluster_max_send(&cm, n, (int)rank, lane, ck);
         }
-        cluster.sync();
-        if (lane < CL_CTAS) {
-            const ClSlot c = c0[buf * CL_CTAS + lane];
-            k = c.key;
-            bv = c.val;
-            bp = c.pos;
-        } else {
-            k = 0ull;
-            bv = 0.f;
-            bp = 0;
-        }
-        slot_max(k, bv, bp, 32);
-        buf ^= 1;
-        *val = bv;
-        *pos = bp;
-    };
-    int isub, pp = 0;
-    for (isub = bsub; isub <= abs(nsub); isub++) {
         smn = __fadd_rn(smn, __fdiv_rn(1.0f, (float)isub));
-        argmax(&maxres, &pp);
+        const unsigned long long gk = cluster_max_wait(&cm, n, ok);
+        if (!ok) continue;
+        if (t == 0) cluster_max_rearm(&cm, n);
+        const Cand g = key_cand(gk);
+        maxres = g.v;
+        if (isub > nabs) break;  // pix/pix2drcc.f:133-135
         if ((flux < 0.f && maxres < 0.f) || (nsub < 0 && maxres < 0.f) ||
             fabsf(maxres) <= fmaxf(__fmul_rn(slim, smn), fabsf(flux))) {
             ansub = isub - 1;
@@ -387,46 +343,44 @@ __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_T, 1)
         }
         const float pntsub = __fmul_rn(gain, maxres);
         tflux = __fadd_rn(tflux, pntsub);
-        const int pmx = pp & 0xFFFF, pmy = pp >> 16;
+        const int pmx = (g.idx & ((1 << logw) - 1)) + 1, pmy = (g.idx >> logw) + 1;
         if (rank == 0 && t == 0) {
             cl[isub - 1] = pntsub;
             cx[isub - 1] = pmx;
             cy[isub - 1] = pmy;
         }
-        // entry (x, y) is updated when 1 <= offx - x <= pw and 1 <= offy - y <= ph
+        // entry (x, y) is updated when 1 <= offx - x <= pw and 1 <= offy - y <= pw
         const int offx = pmpx + pmx, offy = pmpy + pmy;
-        if (bx1 >= offx - pw && bx0 <= offx - 1 && by1 >= offy - ph && by0 <= offy - 1) {
+        if (bx1 >= offx - pw && bx0 <= offx - 1 && by1 >= offy - pw && by0 <= offy - 1) {
 #pragma unroll
             for (int j = 0; j < CL_PER; j++) {
-                const int q = spos[j * CL_T + t];
-                const int px = offx - (q & 0xFFFF), py = offy - (q >> 16);
-                if (px >= 1 && px <= pw && py >= 1 && py <= ph) {
-                    v[j] = __fsub_rn(v[j], __fmul_rn(pntsub, psf[(py - 1) * pw + (px - 1)]));
-                    rescan = true;
+                const int px = offx - 1 - (q[j] & 0xFFFF), py = offy - 1 - (q[j] >> 16);
+                if ((unsigned)px < (unsigned)pw && (unsigned)py < (unsigned)pw) {
+                    v[j] = __fsub_rn(v[j], __fmul_rn(pntsub, psf[py * pw + px]));
+                    if (px == pmpx - 1 && py == pmpy - 1) {  // the component's own pixel
+                        c[j] = __fadd_rn(c[j], pntsub);
+                        mine |= 1u << j;
+                    }
+                    changed = true;
                 }
             }
         }
+        isub++;
     }
-    if (isub > abs(nsub)) argmax(&maxres, &pp);  // pix/pix2drcc.f:133-135
-    cluster.sync();  // no CTA leaves while another may still read CTA 0's slots
-    if (rank == 0 && t == 0) {
-        st->aniter = ansub;
-        st->maxres = maxres;
-        st->tflux = tflux;
-    }
-}
-
-// pix/pix2drma.f:17-21: components RITER..ANITER added in list order (one thread keeps it)
-__global__ void k_clark_addcomp(const float *cl, const int *cx, const int *cy, int riter, const ClarkState *st,
-                                float *comp, int nx, int ny) {
-    const int aniter = st->aniter;
-    for (int i = riter; i <= aniter; i++) {
-        const int ix = cx[i - 1], iy = cy[i - 1];
-        if (ix >= 1 && ix <= nx && iy >= 1 && iy <= ny) {
-            float *a = comp + (size_t)(iy - 1) * nx + (ix - 1);
-            *a = __fadd_rn(*a, cl[i - 1]);
+    if (gave_up) {
+        if (t == 0) st->err = CL_ERR_WAIT;
+    } else {
+#pragma unroll
+        for (int j = 0; j < CL_PER; j++)
+            if (mine >> j & 1u) comp[((size_t)((q[j] >> 16) - 1) << logw) + (q[j] & 0xFFFF) - 1] = c[j];
+        if (rank == 0 && t == 0) {
+            st->aniter = ansub;
+            st->maxres = maxres;
+            st->tflux = tflux;
         }
     }
+    // no CTA leaves while another's stores to it may be in flight
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // pix/pixxmult.f: MVIS = MVIS * XFR, the complex product in REAL
@@ -444,6 +398,12 @@ __global__ void k_clark_cmul(float2 *g, const float2 *__restrict__ x, int nu, in
 __global__ void k_clark_sub(const float *__restrict__ drt, float *res, int64_t n) {
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
         res[k] = __fsub_rn(drt[k], res[k]);
+}
+
+// PIXISAMA key: larger |v| first, then the smaller list index (pix/pixisama.f: the first
+// index whose |A| is strictly greater than every earlier one; 1 when all are zero)
+__device__ __forceinline__ unsigned long long isama_key(float v, int i) {
+    return ((unsigned long long)__float_as_uint(fabsf(v)) << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)i);
 }
 
 // beam-patch peak (PIXISAMA over the patch, pix/pix2drcc.f:63-66), one block; clears the
@@ -489,6 +449,31 @@ __global__ void __launch_bounds__(256) k_clark_ext(const float *__restrict__ psf
         atomicMax(reinterpret_cast<unsigned int *>(&st->extside), __float_as_uint(ext));
 }
 
+int launch_minor(const float *al, const int *pl, ClarkState *dst, const float *spsf, int pw,
+                    const sde_clark_params *p, int riter, float *cl, int *cx, int *cy, float *comp, int w,
+                    cudaStream_t st) {
+    const size_t sm_psf = sizeof(float) * (size_t)pw * pw;
+    const bool in_smem = sm_psf <= 200u * 1024u;
+    auto *k = in_smem ? &k_clark_minor<true> : &k_clark_minor<false>;
+    if (in_smem)
+        SDE_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_psf));
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = CL_CTAS;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CL_CTAS);
+    cfg.blockDim = dim3(CL_T);
+    cfg.dynamicSmemBytes = in_smem ? sm_psf : 0;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int logw = 0;
+    while ((1 << logw) < w) logw++;
+    SDE_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, al, pl, dst, spsf, pw, p->gain, p->niter, riter, p->flux, cl, cx, cy,
+                                    comp, logw));
+    return SDE_OK;
+}
 int fail(const char *m) {
     sde_set_error("%s", m);
     return SDE_EINVAL;
@@ -560,14 +545,6 @@ extern "C" int sde_clark(sde_ctx *ctx, const float *dirty, const float *psf, int
     k_clark_patch<<<1, 1024, 0, st>>>(spsf, pw, dst);
     k_clark_ext<<<std::min(n, ctx->num_sms * 8), 256, 0, st>>>(psf, n, b0, b1, dst);
     SDE_CHECK_LAUNCH();
-    // minor-cycle kernel: positions (+ beam patch when it fits) in shared memory
-    const size_t sm_pos = sizeof(int) * CL_SLICE, sm_psf = sizeof(float) * (size_t)pw * pw;
-    const bool psf_smem = sm_pos + sm_psf <= 200u * 1024u;
-    const size_t sm = sm_pos + (psf_smem ? sm_psf : 0);
-    if (psf_smem)
-        SDE_CUDA_TRY(cudaFuncSetAttribute(k_clark_minor<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    else
-        SDE_CUDA_TRY(cudaFuncSetAttribute(k_clark_minor<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     ClarkState h{};
     int riter = biter, aniter = biter - 1, rc = SDE_OK;
     float tflux = 0.f;
@@ -596,22 +573,16 @@ extern "C" int sde_clark(sde_ctx *ctx, const float *dirty, const float *psf, int
         if (h.anl == 0) break;  // PIX2DRCC would read DRTL(1), never written: nothing to subtract
         {
             KTimer kt(ctx, "clark_minor");
-            ClarkState *d = dst;
-            // TFLUX carries over the cycles (img/imgcclea.f:251)
-            SDE_CUDA_TRY(cudaMemcpyAsync(&d->tflux, &tflux, sizeof(float), cudaMemcpyHostToDevice, st));
-            if (psf_smem)
-                k_clark_minor<true><<<CL_CTAS, CL_T, sm, st>>>(al, pl, dst, spsf, pw, pw, p->gain, p->niter, riter, p->flux,
-                                                         lcl, lcx, lcy);
-            else
-                k_clark_minor<false><<<CL_CTAS, CL_T, sm, st>>>(al, pl, dst, spsf, pw, pw, p->gain, p->niter, riter,
-                                                          p->flux, lcl, lcx, lcy);
-            SDE_CHECK_LAUNCH();
-            k_clark_addcomp<<<1, 1, 0, st>>>(lcl, lcx, lcy, riter, dst, comp, w, w);
-            SDE_CHECK_LAUNCH();
+            // TFLUX carries over the cycles in *dst (img/imgcclea.f:251)
+            SDE_TRY(launch_minor(al, pl, dst, spsf, pw, p, riter, lcl, lcx, lcy, comp, w, st));
         }
         SDE_TRY(clark_resid(ctx, comp, drt, xfr, mvis, pitch, resid, w, n));
         SDE_CUDA_TRY(cudaMemcpyAsync(&h, dst, sizeof h, cudaMemcpyDeviceToHost, st));
         SDE_CUDA_TRY(cudaStreamSynchronize(st));
+        if (h.err == CL_ERR_WAIT) {
+            sde_set_error("sde_clark: a device wait timed out");
+            return SDE_ETIMEDOUT;
+        }
         aniter = h.aniter;
         tflux = h.tflux;
         if (out->ncycles < SDE_CLARK_TRACE) {

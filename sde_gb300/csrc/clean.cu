@@ -16,6 +16,7 @@
 
 #include <mutex>
 
+#include "cluster_max.cuh"
 #include "common.cuh"
 
 namespace {
@@ -24,12 +25,6 @@ constexpr int CL_THREADS = 512;
 constexpr size_t CL_SMEM_SLICE_MAX = 100 * 1024;  // largest RES slice kept in shared memory
 constexpr int CL_BATCH = 4;                        // pixels per thread with PSF loads in flight
 constexpr unsigned SPIN_LIMIT = 1u << 26;
-
-struct Cand {
-    float a;      // |value|
-    int32_t idx;  // flat 0-based index, INT32_MAX if none
-    float v;      // signed value
-};
 
 __device__ __forceinline__ Cand better(Cand x, Cand y) {
     // larger |a| wins; ties go to the smaller index (first occurrence)
@@ -72,29 +67,6 @@ struct Barrier {
     int stopreq[2];  // cancel requests published by CTA 0 before each barrier
     unsigned long long best[3];  // each iteration's maximum, as a packed key (cand_key)
 };
-
-// A candidate as a 64-bit key whose unsigned order is better()'s: |value| bits (|value| >= 0
-// and not NaN here, so the bits order as the values do), then INT32_MAX - index (the first
-// index wins a tie), then the value's sign bit.  One atomicMax per CTA finds the maximum.
-__device__ __forceinline__ unsigned long long cand_key(Cand c) {
-    return ((unsigned long long)__float_as_uint(c.a) << 32) |
-           ((unsigned long long)(uint32_t)(INT32_MAX - c.idx) << 1) | (__float_as_uint(c.v) >> 31);
-}
-// the largest key of a warp's lanes: the largest high word, then the largest low word among
-// the lanes that hold it
-__device__ __forceinline__ unsigned long long warp_key_max(unsigned long long k) {
-    const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
-    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    return ((unsigned long long)mhi << 32) | mlo;
-}
-__device__ __forceinline__ Cand key_cand(unsigned long long k) {
-    Cand c;
-    c.a = __uint_as_float((uint32_t)(k >> 32));
-    c.idx = INT32_MAX - (int32_t)((uint32_t)k >> 1);
-    c.v = (k & 1ull) ? -c.a : c.a;
-    return c;
-}
 
 // Grid-wide barrier on a monotonic arrival count: barrier number `epoch` (0, 1, ...) is passed
 // when the count reaches (epoch + 1) * nblocks, so the last CTA's arrival releases the others
@@ -320,9 +292,6 @@ __global__ void __launch_bounds__(CL_THREADS) k_hogbom(CleanArgs A) {
 constexpr int HC_CTAS = 16;   // cluster size (above the portable 8: opted in at launch)
 constexpr int64_t HC_MAXPIX = (int64_t)512 * HC_CTAS * 32;
 constexpr int HC_RING = 256;  // components kept before they go into CLN
-constexpr int HC_SPIN = 1 << 20;
-
-__device__ __forceinline__ uint32_t cl_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Row of pixel idx in rows of nx pixels, by the reciprocal ceil(2^32 / nx): the product can
 // only reach the next row's first pixel early.
@@ -331,69 +300,6 @@ __device__ __forceinline__ int row_of(int idx, int nx, uint32_t recip) {
     if (nx == 1) return idx;
     const int q = (int)__umulhi((uint32_t)idx, recip);
     return q * nx > idx ? q - 1 : q;
-}
-
-// The cluster's maxima of one round: slot r holds CTA r's key.
-template <int C>
-struct ClusterMax {
-    unsigned long long slot[2][C];
-    unsigned long long bar[2];
-};
-
-template <int C>
-__device__ __forceinline__ void cluster_max_init(ClusterMax<C> *m) {
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int p = 0; p < 2; p++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&m->bar[p])));
-        asm volatile("fence.mbarrier_init.release.cluster;");
-#pragma unroll
-        for (int p = 0; p < 2; p++)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(&m->bar[p])),
-                         "r"((uint32_t)(8 * C)));
-    }
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Called by the first C lanes of one warp: the CTA's key of round n to slot `rank` of CTA
-// `lane`.  A slot is written again two rounds later, by a CTA that has this CTA's key of the
-// round between, which is sent after every warp here has read the slot.
-template <int C>
-__device__ __forceinline__ void cluster_max_send(ClusterMax<C> *m, int n, int rank, int lane,
-                                                 unsigned long long key) {
-    uint32_t dst, bar;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(cl_smem(&m->slot[n & 1][rank])), "r"(lane));
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(cl_smem(&m->bar[n & 1])), "r"(lane));
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
-                 "l"(key), "r"(bar)
-                 : "memory");
-}
-
-// Called by every thread: round n's keys of all CTAs, reduced; ok is cleared when the warp's
-// wait gave up.
-template <int C>
-__device__ __forceinline__ unsigned long long cluster_max_wait(ClusterMax<C> *m, int n, bool &ok) {
-    const uint32_t bar = cl_smem(&m->bar[n & 1]);
-    const uint32_t parity = (uint32_t)(n >> 1) & 1u;
-    uint32_t done = 0;
-    for (int spin = 0; spin < HC_SPIN && !done; spin++)
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;"
-            " selp.u32 %0, 1, 0, p; }"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-    const int lane = threadIdx.x & 31;
-    ok = __all_sync(0xffffffffu, done);
-    return warp_key_max(ok && lane < C ? *(volatile unsigned long long *)&m->slot[n & 1][lane] : 0ull);
-}
-
-// One thread, after its CTA has passed round n's wait: the barrier's next phase expects C keys.
-template <int C>
-__device__ __forceinline__ void cluster_max_rearm(ClusterMax<C> *m, int n) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(&m->bar[n & 1])),
-                 "r"((uint32_t)(8 * C))
-                 : "memory");
 }
 
 // PSF peak (1-based) from PIXISAMA's index (pix/pix2drcl.f:73-80)

@@ -1,0 +1,100 @@
+// cluster_max.cuh -- the argmax of CLEAN's minor cycles: candidates as 64-bit keys, their maximum
+// over a warp, and over a thread-block cluster by remote stores.
+#pragma once
+#include <stdint.h>
+
+struct Cand {
+    float a;      // |value|
+    int32_t idx;  // flat 0-based index, INT32_MAX if none
+    float v;      // signed value
+};
+
+// A candidate as a 64-bit key whose unsigned order is better()'s: |value| bits (|value| >= 0
+// and not NaN here, so the bits order as the values do), then INT32_MAX - index (the first
+// index wins a tie), then the value's sign bit.  One atomicMax per CTA finds the maximum.
+__device__ __forceinline__ unsigned long long cand_key(Cand c) {
+    return ((unsigned long long)__float_as_uint(c.a) << 32) |
+           ((unsigned long long)(uint32_t)(INT32_MAX - c.idx) << 1) | (__float_as_uint(c.v) >> 31);
+}
+// the largest key of a warp's lanes: the largest high word, then the largest low word among
+// the lanes that hold it
+__device__ __forceinline__ unsigned long long warp_key_max(unsigned long long k) {
+    const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+    return ((unsigned long long)mhi << 32) | mlo;
+}
+__device__ __forceinline__ Cand key_cand(unsigned long long k) {
+    Cand c;
+    c.a = __uint_as_float((uint32_t)(k >> 32));
+    c.idx = INT32_MAX - (int32_t)((uint32_t)k >> 1);
+    c.v = (k & 1ull) ? -c.a : c.a;
+    return c;
+}
+
+constexpr int CM_SPIN = 1 << 20;  // polls of a cluster wait before it gives up
+
+__device__ __forceinline__ uint32_t cl_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// The cluster's maxima of one round: slot r holds CTA r's key.
+template <int C>
+struct ClusterMax {
+    unsigned long long slot[2][C];
+    unsigned long long bar[2];
+};
+
+template <int C>
+__device__ __forceinline__ void cluster_max_init(ClusterMax<C> *m) {
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&m->bar[p])));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(&m->bar[p])),
+                         "r"((uint32_t)(8 * C)));
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Called by the first C lanes of one warp: the CTA's key of round n to slot `rank` of CTA
+// `lane`.  A slot is written again two rounds later, by a CTA that has this CTA's key of the
+// round between, which is sent after every warp here has read the slot.
+template <int C>
+__device__ __forceinline__ void cluster_max_send(ClusterMax<C> *m, int n, int rank, int lane,
+                                                 unsigned long long key) {
+    uint32_t dst, bar;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(cl_smem(&m->slot[n & 1][rank])), "r"(lane));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(cl_smem(&m->bar[n & 1])), "r"(lane));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+                 "l"(key), "r"(bar)
+                 : "memory");
+}
+
+// Called by every thread: round n's keys of all CTAs, reduced; ok is cleared when the warp's
+// wait gave up.
+template <int C>
+__device__ __forceinline__ unsigned long long cluster_max_wait(ClusterMax<C> *m, int n, bool &ok) {
+    const uint32_t bar = cl_smem(&m->bar[n & 1]);
+    const uint32_t parity = (uint32_t)(n >> 1) & 1u;
+    uint32_t done = 0;
+    for (int spin = 0; spin < CM_SPIN && !done; spin++)
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;"
+            " selp.u32 %0, 1, 0, p; }"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    const int lane = threadIdx.x & 31;
+    ok = __all_sync(0xffffffffu, done);
+    return warp_key_max(ok && lane < C ? *(volatile unsigned long long *)&m->slot[n & 1][lane] : 0ull);
+}
+
+// One thread, after its CTA has passed round n's wait: the barrier's next phase expects C keys.
+template <int C>
+__device__ __forceinline__ void cluster_max_rearm(ClusterMax<C> *m, int n) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(&m->bar[n & 1])),
+                 "r"((uint32_t)(8 * C))
+                 : "memory");
+}

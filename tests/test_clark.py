@@ -128,3 +128,32 @@ def test_gpu_zero_image_reports_reference_error(gpu_ctx, gold):
     with pytest.raises(RuntimeError):
         _gpu(gpu_ctx, np.zeros((128, 128), np.float32), gold["beam"], niter=10)
     assert "Zero range in values" in _abi.last_error()
+
+
+# lists with 1, 2, 3 and 8 entries a minor-cycle thread (8 CTAs x 512 threads) and of a few
+# entries; beam patches in shared memory, too large for it, and of two pixels
+@pytest.mark.gpu
+@pytest.mark.parametrize("numcl,bp,niter", [(4096, 2, 60), (500, 64, 100), (4200, 127, 200), (9000, 300, 150),
+                                            (32768, 128, 400)])
+def test_gpu_long_lists_bit_exact(gpu_ctx, orc, numcl, bp, niter):
+    """A 256x256 window of blobs over noise: one major cycle, so everything equals the oracle."""
+    n = 512
+    rng = np.random.default_rng(numcl + bp)
+    y, x = np.mgrid[0:n, 0:n]
+    c = (n + 1) // 2 - 1
+    r2 = (x - c) ** 2 + (y - c) ** 2
+    psf = (np.exp(-r2 / 18.0) + 1e-3 * np.cos(0.3 * (x - c)) * np.cos(0.2 * (y - c)) / (1 + r2 / 900.0))
+    psf = (psf / psf[c, c]).astype(np.float32)
+    dirty = (0.01 * rng.standard_normal((n, n))).astype(np.float32)
+    for f, px, py in zip(rng.uniform(0.5, 2.0, 40), rng.integers(140, 370, 40), rng.integers(140, 370, 40)):
+        dirty += np.float32(f) * np.roll(psf, (py - c, px - c), (0, 1))
+    kw = dict(niter=niter, gain=0.2, flux=0.0, numcl=numcl, bpatch=bp)
+    o = orc.clark(dirty, psf, **kw)
+    g = _gpu(gpu_ctx, dirty, psf, **kw)
+    a = o["trace"][0][1]
+    assert a >= 1 and g["trace"][0][:2] == o["trace"][0][:2]
+    assert np.array_equal(g["cl"][:a], o["cl"][:a])
+    assert np.array_equal(g["cx"][:a], o["cx"][:a]) and np.array_equal(g["cy"][:a], o["cy"][:a])
+    if g["ncycles"] == o["ncycles"] == 1:
+        assert np.array_equal(g["comp"], o["comp"])
+        assert g["maxres"] == o["maxres"] and g["tflux"] == o["tflux"]
