@@ -9,7 +9,8 @@
 // operations (no FMA), finds its slice's first maximum, and that maximum joins a global one
 // (a packed key, one atomicMax per CTA) inside a grid barrier (bounded spin); every CTA then
 // reads the same global (max, first index), so component positions are identical to the
-// reference's.  Windows that fit one thread-block cluster run in k_hogbom_cluster.
+// reference's.  Windows that fit one thread-block cluster run in k_hogbom_cluster,
+// those that fit the registers of the chip in k_hogbom_regs.
 #include <cooperative_groups.h>
 #include <math.h>
 #include <string.h>
@@ -443,12 +444,265 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// ---------------------------------------------------------------------------------------
+// Windows above one cluster's: the residual stays in the registers of one CTA per SM for all
+// iterations (HR_T threads x HR_PER pixels), and an iteration reads only the PSF (and the box).
+// The pixels of a thread are HR_T apart in the CTA's contiguous slice; a bit per pixel says
+// whether the step to it starts a new row, so the PSF offset is carried by two integer adds.
+// The next group's PSF loads are in flight while one is subtracted.
+// The maximum of a pass: a maximum per group, then only the warp that holds the CTA's searches
+// its group for the first pixel, and the key goes to a slot of every mailbox, which one warp of
+// each of its HR_SHARE CTAs polls.  A 64-bit store carries key and round together (bit 63, the
+// spare sign of |value|), so there is no counter, no atomic and no fence in the chain.  Slots
+// alternate: one written in round n is written again in round n + 2, whose writer has seen every
+// key of round n + 1, each sent after its CTA had read round n.
+// Bound by the L2's rate for the PSF at large windows (2047^2: 4600 cycles of an iteration's
+// 10500, 18 or 27 loads ahead alike) and by the exchange (3000) at small ones: with one mailbox
+// polled by all CTAs it took 8000, with 1, 2, 4, 8, 16 CTAs a mailbox 723^2 takes 2.75, 2.66,
+// 2.73, 2.80, 2.97 us an iteration.  k_hogbom -> here, us an iteration without and with a box:
+// 723^2 4.85 -> 2.66 and 5.34 -> 3.06, 1023^2 5.6 -> 3.0 and 6.5 -> 3.5, 1447^2 7.2 -> 3.75 and
+// 8.8 -> 4.7, 2047^2 9.7 -> 5.4 and 12.8 -> 7.9.
+constexpr int HR_T = 256, HR_PER = 108;
+static_assert(HR_PER % 27 == 0, "whole words of row bits");
+constexpr int HR_MAXCTAS = 160;  // a mailbox: 5 slots a polling lane, all in flight
+constexpr int HR_SHARE = 2;      // CTAs that poll one mailbox
+constexpr int HR_SPIN = 1 << 22;
+constexpr size_t HR_SLOTS = (size_t)HR_MAXCTAS / HR_SHARE * 2 * HR_MAXCTAS;  // [mailbox][round & 1][writer]
+constexpr unsigned long long HR_TAG = 1ull << 63;
+
+template <bool BOX>
+__global__ void __launch_bounds__(HR_T, 1) k_hogbom_regs(CleanArgs A, unsigned long long *slots) {
+    constexpr int HR_G = BOX ? 9 : 18, HR_NG = HR_PER / HR_G;  // (a box value is loaded with each PSF value)
+    __shared__ unsigned s_max[HR_T / 32];
+    __shared__ unsigned s_low;
+    __shared__ unsigned long long s_key;
+    __shared__ int s_ok;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nb = gridDim.x;
+    const int npix = A.nx * A.ny;
+    const int slice = (npix + nb - 1) / nb;
+    const int64_t lo64 = (int64_t)slice * blockIdx.x;
+    const int lo = (int)(lo64 < npix ? lo64 : npix);
+    const int mine = min(slice, npix - lo);                         // the CTA's pixels
+    const int nj = mine > t ? (mine - t + HR_T - 1) / HR_T : 0;     // the thread's
+    const int ncta = (mine + HR_T - 1) / HR_T;                      // the CTA's largest nj
+    const int nbox = (nb + HR_SHARE - 1) / HR_SHARE;
+    const int wrap = A.pnx - A.nx;
+    const uint32_t rnx = row_recip(A.nx);
+    float r[HR_PER];
+    unsigned cross[HR_PER / 27];  // bit j % 27 of word j / 27: pixel j starts a new row
+    int rel0;                     // PSF offset of the first pixel: -ix - iy * pnx
+    {
+        const int k0 = min(lo + t, npix - 1);
+        const int iy = k0 / A.nx;
+        int ix = k0 - iy * A.nx;
+        rel0 = -ix - iy * A.pnx;
+#pragma unroll
+        for (int j = 0; j < HR_PER; j++) {
+            if (j % 27 == 0) cross[j / 27] = 0u;
+            if (j > 0) {
+                ix += HR_T;
+                if (ix >= A.nx) {
+                    ix -= A.nx;
+                    cross[j / 27] |= 1u << (j % 27);
+                }
+            }
+            r[j] = __int_as_float(0x7FC00000);  // no pixel: a NaN, which no maximum takes
+            if (j < nj) {
+                const int k = lo + j * HR_T + t;
+                r[j] = __fmul_rn(A.drt[k], BOX ? A.box[k] : 1.0f);
+            }
+        }
+    }
+    float gmax[HR_NG];  // largest |residual| of a group; NaN pixels never win
+    auto group_max = [&](int g) {
+        float m = -1.0f;
+#pragma unroll
+        for (int i = 0; i < HR_G; i++) m = fmaxf(m, fabsf(r[g * HR_G + i]));
+        gmax[g] = m;
+    };
+#pragma unroll
+    for (int g = 0; g < HR_NG; g++) group_max(g);
+    float tflux = A.tflux_in, maxres = 0.f;
+    const int nabs = A.nsub < 0 ? -A.nsub : A.nsub;
+    int isub = A.bsub, stopped = 0;
+    for (int n = 0;; n++) {
+        // the CTA's maximum: 0 for none, else the bits of |value| plus one
+        float m = gmax[0];
+#pragma unroll
+        for (int g = 1; g < HR_NG; g++) m = fmaxf(m, gmax[g]);
+        const unsigned code = m >= 0.0f ? __float_as_uint(m) + 1u : 0u;
+        const unsigned wcode = __reduce_max_sync(0xffffffffu, code);
+        if (lane == 0) s_max[warp] = wcode;
+        if (t == 0) s_low = 0u;
+        __syncthreads();
+        const unsigned ccode = __reduce_max_sync(0xffffffffu, s_max[lane & (HR_T / 32 - 1)]);
+        if (wcode == ccode && code == ccode && code) {
+            int first = INT32_MAX;
+            float v = 0.f;
+#pragma unroll
+            for (int g = HR_NG - 1; g >= 0; g--)
+                if (gmax[g] == m) {
+#pragma unroll
+                    for (int i = HR_G - 1; i >= 0; i--)
+                        if (fabsf(r[g * HR_G + i]) == m) {
+                            first = g * HR_G + i;
+                            v = r[g * HR_G + i];
+                        }
+                }
+            atomicMax(&s_low, (unsigned)cand_key(Cand{m, lo + first * HR_T + t, v}));
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned long long tag = (n >> 1) & 1 ? 0ull : HR_TAG;
+            const unsigned long long out = (ccode ? (unsigned long long)(ccode - 1u) << 32 : 0ull) | s_low | tag;
+#pragma unroll
+            for (int b = 0; b < (HR_MAXCTAS / HR_SHARE + 31) / 32; b++)
+                if (b * 32 + lane < nbox)
+                    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(
+                                     slots + ((size_t)(b * 32 + lane) * 2 + (n & 1)) * HR_MAXCTAS + blockIdx.x),
+                                 "l"(out)
+                                 : "memory");
+            const unsigned long long *row = slots + ((size_t)(blockIdx.x % nbox) * 2 + (n & 1)) * HR_MAXCTAS;
+            unsigned long long best = 0ull;
+            bool done = false;
+            for (int spin = 0; spin < HR_SPIN && !done; spin++) {
+                unsigned long long k[HR_MAXCTAS / 32];
+#pragma unroll
+                for (int b = 0; b < HR_MAXCTAS / 32; b++) {
+                    k[b] = tag;
+                    if (b * 32 + lane < nb)
+                        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(k[b]) : "l"(row + b * 32 + lane) : "memory");
+                }
+                bool all = true;
+                best = 0ull;
+#pragma unroll
+                for (int b = 0; b < HR_MAXCTAS / 32; b++) {
+                    all = all && (k[b] & HR_TAG) == tag;
+                    k[b] &= ~HR_TAG;
+                    best = k[b] > best ? k[b] : best;
+                }
+                done = __all_sync(0xffffffffu, all);
+            }
+            best = warp_key_max(best);
+            if (lane == 0) {
+                s_key = best;
+                s_ok = done;
+            }
+        }
+        __syncthreads();
+        if (!s_ok) {
+            if (t == 0) atomicExch(&A.status[STATUS_TIMEOUT], 1);
+            return;
+        }
+        const Cand g = key_cand(s_key);
+        maxres = g.v;
+        if (isub > nabs) break;
+        // (a key of 0: no pixel is a number, so there is nothing to subtract)
+        if ((A.nsub < 0 && maxres < 0.0f) || fabsf(maxres) <= A.flux || s_key == 0ull) {
+            stopped = 1;
+            break;
+        }
+        const float pntsub = __fmul_rn(A.gain, maxres);
+        tflux = __fadd_rn(tflux, pntsub);
+        const int gy = row_of(g.idx, A.nx, rnx), gx = g.idx - gy * A.nx;
+        // the component's pixel, in its thread (the add waits until the PSF loads are issued)
+        const int own = g.idx - lo - t;
+        const bool owner = own >= 0 && own < mine - t && own % HR_T == 0;
+        float cln = 0.f;
+        if (owner) cln = A.cln[g.idx];
+        if (blockIdx.x == 0 && t == 0) {
+            A.cflux[isub - 1] = pntsub;
+            A.cx[isub - 1] = gx + 1;
+            A.cy[isub - 1] = gy + 1;
+        }
+        // PSF(OFFX-IX, OFFY-IY), flat: (pmpx-1 + gx - ix) + (pmpy-1 + gy - iy) * pnx
+        const float *p0 = A.psf + (A.pmpx - 1 + gx) + (int64_t)(A.pmpy - 1 + gy) * A.pnx;
+        float p[2][HR_G], bx[2][BOX ? HR_G : 1];
+        int o = rel0;
+        auto load = [&](int q) {
+#pragma unroll
+            for (int i = 0; i < HR_G; i++) {
+                const int j = q * HR_G + i;
+                if (j > 0) {
+                    o -= HR_T;
+                    if (cross[j / 27] >> (j % 27) & 1u) o -= wrap;
+                }
+                p[q & 1][i] = j < nj ? __ldg(p0 + o) : 0.f;
+                if (BOX) bx[q & 1][i] = j < nj ? __ldg(A.box + lo + j * HR_T + t) : 0.f;
+            }
+        };
+        load(0);
+#pragma unroll
+        for (int q = 0; q < HR_NG; q++) {
+            if (q * HR_G < ncta) {
+                if (q + 1 < HR_NG) {
+                    if ((q + 1) * HR_G < ncta) load(q + 1);
+                }
+#pragma unroll
+                for (int i = 0; i < HR_G; i++) {
+                    const int j = q * HR_G + i;
+                    float sub = __fmul_rn(pntsub, p[q & 1][i]);
+                    if (BOX) sub = __fmul_rn(sub, bx[q & 1][i]);
+                    r[j] = __fsub_rn(r[j], sub);
+                }
+                group_max(q);
+            }
+        }
+        if (owner) A.cln[g.idx] = __fadd_rn(cln, pntsub);
+        isub++;
+    }
+#pragma unroll
+    for (int j = 0; j < HR_PER; j++)
+        if (j < nj) A.res[lo + j * HR_T + t] = r[j];
+    if (blockIdx.x == 0 && t == 0) {
+        A.out[0] = maxres;
+        A.out[1] = tflux;
+        A.out[2] = __int_as_float(stopped ? isub - 1 : A.nsub);
+        A.out[3] = __int_as_float(stopped);
+    }
+}
+
 // first strictly-largest |a| (PIXISAMA), two-level
+// (16-byte loads, four in flight a thread, from the first aligned element on; 4096^2: 51 -> 14 us)
 __global__ void __launch_bounds__(CL_THREADS) k_isamax_part(const float *a, int64_t n, Cand *part) {
-    Cand c{-1.0f, INT32_MAX, 0.0f};
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-        c = better(c, Cand{fabsf(a[k]), (int32_t)k, a[k]});
-    c = block_best(c);
+    // a thread's indices rise, so a strictly larger |a| is its first maximum (NaN never is)
+    float la = -1.0f, lv = 0.0f;
+    int li = INT32_MAX;
+    auto take = [&](float v, int64_t k) {
+        if (fabsf(v) > la) {
+            la = fabsf(v);
+            li = (int)k;
+            lv = v;
+        }
+    };
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    const int64_t head = min(n, (int64_t)((16 - ((uintptr_t)a & 15)) & 15) / 4), n4 = (n - head) / 4;
+    const float4 *a4 = reinterpret_cast<const float4 *>(a + head);
+    if (g < head) take(a[g], g);
+    int64_t k = g;
+    for (; k + 3 * step < n4; k += 4 * step) {
+        float4 x[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) x[i] = __ldg(a4 + k + i * step);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t e = head + 4 * (k + i * step);
+            take(x[i].x, e);
+            take(x[i].y, e + 1);
+            take(x[i].z, e + 2);
+            take(x[i].w, e + 3);
+        }
+    }
+    for (; k < n4; k += step) {
+        const float4 x = __ldg(a4 + k);
+        const int64_t e = head + 4 * k;
+        take(x.x, e);
+        take(x.y, e + 1);
+        take(x.z, e + 2);
+        take(x.w, e + 3);
+    }
+    if (head + 4 * n4 + g < n) take(a[head + 4 * n4 + g], head + 4 * n4 + g);
+    const Cand c = block_best(Cand{la, li, lv});
     if (threadIdx.x == 0) part[blockIdx.x] = c;
 }
 
@@ -553,6 +807,8 @@ int clean_preload(sde_ctx *ctx) {
     SDE_CUDA_TRY(cudaFuncGetAttributes(&a, k_max_part));
     SDE_CUDA_TRY(cudaFuncGetAttributes(&a, k_max_final));
     SDE_CUDA_TRY(cudaFuncGetAttributes(&a, k_scale_inv));
+    SDE_CUDA_TRY(cudaFuncGetAttributes(&a, k_hogbom_regs<false>));
+    SDE_CUDA_TRY(cudaFuncGetAttributes(&a, k_hogbom_regs<true>));
     int per_sm = 0;
     SDE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hogbom<false>, CL_THREADS, 0));
     ctx->hogbom_per_sm = per_sm;
@@ -672,6 +928,22 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
     int64_t ip1;
     SDE_TRY(ctx_read_small(ctx, ctx->stream, &ip1, psf_ip, sizeof ip1));
     psf_peak(ip1, pnx, pny, &A.pmpx, &A.pmpy);
+    // a window that the registers hold, rows no shorter than a thread's step, the PSF covering it
+    if (!cancel_flag && nx >= HR_T && ctx->num_sms <= HR_MAXCTAS &&
+        (int64_t)nx * ny <= (int64_t)ctx->num_sms * HR_T * HR_PER && psf_covers(A.pmpx, A.pmpy, nx, ny, pnx, pny)) {
+        unsigned long long *slots;
+        SDE_TRY(ctx_scratch(ctx, "cl_slots", HR_SLOTS * sizeof(*slots), (void **)&slots));
+        SDE_CUDA_TRY(cudaMemsetAsync(slots, 0, HR_SLOTS * sizeof(*slots), ctx->stream));
+        void *args[] = {&A, &slots};
+        {
+            KTimer kt(ctx, "hogbom");
+            SDE_CUDA_TRY(cudaLaunchCooperativeKernel(
+                box ? (const void *)k_hogbom_regs<true> : (const void *)k_hogbom_regs<false>,
+                dim3(ctx->num_sms), dim3(HR_T), args, 0, ctx->stream));
+        }
+        int stopped;
+        return clean_result(ctx, dout, out, &stopped);
+    }
     int per_sm = ctx->hogbom_per_sm;
     if (per_sm < 1) SDE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hogbom<false>, CL_THREADS, 0));
     if (per_sm < 1) {

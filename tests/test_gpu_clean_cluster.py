@@ -56,3 +56,26 @@ def test_box_and_uncovered_psf(gpu_ctx, orc):
 def test_zero_residual(gpu_ctx, orc):
     drt, psf = _case(40, 30, 81, 61, 7)
     _compare(gpu_ctx, orc, np.zeros_like(drt), psf, 10)
+
+
+# windows above the cluster's, in the registers of one CTA per SM: few and many pixels a thread,
+# rows of exactly a thread's step and one less (the general kernel), a narrow and a wide window,
+# the last CTA short or empty, the largest window that fits (152 x 256 x 108 pixels) and one over
+@pytest.mark.parametrize("nx,ny,box", [(513, 513, False), (256, 1030, True), (255, 1040, False), (700, 391, True),
+                                       (5000, 53, False), (1023, 1023, True), (2047, 2047, False), (1152, 3648, False),
+                                       (1153, 3648, True)])
+def test_windows_in_registers(gpu_ctx, orc, nx, ny, box):
+    drt, psf = _case(nx, ny, 2 * nx + 3, 2 * ny, nx + ny)
+    b = None
+    if box:
+        b = (np.random.default_rng(ny).random((ny, nx)) > 0.3).astype(np.float32)
+    _compare(gpu_ctx, orc, drt, psf, 9, gain=0.4, box=b, bsub=2)
+
+
+def test_register_window_stop_rules(gpu_ctx, orc):
+    drt, psf = _case(600, 500, 1201, 1001, 11)
+    drt[3, 5] = -9.0
+    _compare(gpu_ctx, orc, drt, psf, -40)         # a negative maximum stops at once
+    _compare(gpu_ctx, orc, drt, psf, 40, flux=4.0)
+    _compare(gpu_ctx, orc, drt, psf, 0)
+    _compare(gpu_ctx, orc, np.zeros_like(drt), psf, 5)
