@@ -272,6 +272,10 @@ int sde_image_from_grid(sde_ctx *ctx, float *grid, int pitch, int nx, int ny, in
                         int correct, const float *scale_dev, float *image);
 int sde_grid_from_image(sde_ctx *ctx, const float *image, int nx, int ny, int fnu, int nv,
                         int correct, float *grid, int pitch);
+/* The same for an nx x ny image that lies at (lsx, lsy), 0-based, of a px x py one which is zero
+ * elsewhere (IMGDOUBL's padding, img/imgdoubl.f:56-86), without making the padded image. */
+int sde_grid_from_padded(sde_ctx *ctx, const float *image, int nx, int ny, int lsx, int lsy, int px,
+                         int py, int fnu, int nv, int correct, float *grid, int pitch);
 
 /* max over an image (ARRSTAT ARRMAX) into a device float, and OUT = scale*IN + offset
  * with scale = 1/(*max_dev) (task/uvmap.f:434-440, 480-482 with pix/pixrscal.f). */

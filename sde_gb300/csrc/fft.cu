@@ -337,15 +337,16 @@ __global__ void __launch_bounds__(FFT_THREADS) k_row_c2r(const float2 *__restric
 }
 
 // Row pass image -> grid (r2c), one CTA per image row; grid correction on the way in.
+// Image column 0 is FFT input ioff.
 __global__ void __launch_bounds__(FFT_THREADS) k_row_r2c(const float *__restrict__ image, int nx,
-                                                          int ny, int fnu, int rows, int ibegy,
+                                                          int ny, int fnu, int rows, int ioff, int ibegy,
                                                           const float2 *__restrict__ tw,
                                                           CorrParams cp, float2 *grid, int pitch,
                                                           int nu) {
     extern __shared__ float2 s[];
     const int H = fnu >> 1;
     const int logh = __ffs(H) - 1;
-    const int cu = (fnu + 1) / 2 - 1, ioff = (fnu - nx) / 2;
+    const int cu = (fnu + 1) / 2 - 1;
     const int iy0 = blockIdx.x * rows;
     for (int t = threadIdx.x; t < H * rows; t += blockDim.x) {
         const int rr = t >> logh, m = t & (H - 1);
@@ -706,7 +707,7 @@ __global__ void __launch_bounds__(RowShape<LOGH, FEW>::T, RowShape<LOGH, FEW>::M
 // Row pass image -> grid (as k_row_r2c), ROWS rows per CTA, half-length 2^LOGH.
 template <int LOGH, bool FEW>
 __global__ void __launch_bounds__(RowShape<LOGH, FEW>::T, RowShape<LOGH, FEW>::MINB)
-    k_row_r2c_t(const __grid_constant__ FftBatch bt, int nx, int ny, int ibegy,
+    k_row_r2c_t(const __grid_constant__ FftBatch bt, int nx, int ny, int ioff, int ibegy,
                 const float2 *__restrict__ tw, CorrParams cp, int pitch, int *status) {
     const float *__restrict__ image = bt.image[blockIdx.y];
     float2 *grid = bt.grid[blockIdx.y];
@@ -715,7 +716,7 @@ __global__ void __launch_bounds__(RowShape<LOGH, FEW>::T, RowShape<LOGH, FEW>::M
     constexpr int TOTAL = ROWS * H;
     constexpr int PER = (TOTAL + T - 1) / T;
     extern __shared__ __align__(16) float2 s[];
-    const int cu = (FNU + 1) / 2 - 1, ioff = (FNU - nx) / 2;
+    const int cu = (FNU + 1) / 2 - 1;
     const int iy0 = blockIdx.x * ROWS;
     if (!FEW && ROWS == 2 && status) {
         // the CTA's image rows come in by bulk copy (row rr at floats [rr*FNU, rr*FNU+nx) of
@@ -1017,9 +1018,11 @@ __global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // boxes without a row of [r0, r1) are not loaded: the first pass reads those rows as zero
+        const int b0 = r0 / BOX, b1 = (r1 + BOX - 1) / BOX;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bb),
-                     "r"((uint32_t)(sizeof(float4) * N)));
-        for (int b = 0; b < N / BOX; b++)
+                     "r"((uint32_t)(sizeof(float4) * BOX * (b1 - b0))));
+        for (int b = b0; b < b1; b++)
             asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                 " [%0], [%1, {%2, %3}], [%4];" ::"r"(sb + (uint32_t)(b * BOX * sizeof(float4))),
@@ -1332,24 +1335,24 @@ cudaError_t launch_c2r_t(const FftBatch &bt, int nbatch, int pitch, int nx, int 
 }
 
 template <int LOGH, bool FEW>
-cudaError_t launch_r2c_shape(const FftBatch &bt, int nbatch, int nx, int ny, int ibegy, const float2 *tw,
+cudaError_t launch_r2c_shape(const FftBatch &bt, int nbatch, int nx, int ny, int ioff, int ibegy, const float2 *tw,
                              CorrParams cp, int pitch, int *status, cudaStream_t st) {
     using S = RowShape<LOGH, FEW>;
     cudaError_t e = cudaFuncSetAttribute(k_row_r2c_t<LOGH, FEW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
     if (e != cudaSuccess) return e;
     k_row_r2c_t<LOGH, FEW><<<dim3((unsigned)((ny + S::ROWS - 1) / S::ROWS), (unsigned)nbatch), S::T,
-                             S::SMEM, st>>>(bt, nx, ny, ibegy, tw, cp, pitch, status);
+                             S::SMEM, st>>>(bt, nx, ny, ioff, ibegy, tw, cp, pitch, status);
     return cudaGetLastError();
 }
 template <int LOGH>
-cudaError_t launch_r2c_t(const FftBatch &bt, int nbatch, int nx, int ny, int ibegy, const float2 *tw,
+cudaError_t launch_r2c_t(const FftBatch &bt, int nbatch, int nx, int ny, int ioff, int ibegy, const float2 *tw,
                          CorrParams cp, int pitch, int *status, cudaStream_t st) {
     const int rows = RowShape<LOGH, false>::ROWS;
     if constexpr (LOGH < 11)  // two-row CTAs from H = 2048 on stage their rows by bulk copy
         if (few_ctas((ny + rows - 1) / rows, nbatch))
-            return launch_r2c_shape<LOGH, true>(bt, nbatch, nx, ny, ibegy, tw, cp, pitch, status, st);
-    return launch_r2c_shape<LOGH, false>(bt, nbatch, nx, ny, ibegy, tw, cp, pitch, status, st);
+            return launch_r2c_shape<LOGH, true>(bt, nbatch, nx, ny, ioff, ibegy, tw, cp, pitch, status, st);
+    return launch_r2c_shape<LOGH, false>(bt, nbatch, nx, ny, ioff, ibegy, tw, cp, pitch, status, st);
 }
 
 #define SDE_LOG_CASES(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13)
@@ -1381,7 +1384,7 @@ bool c2r_t(int logh, const FftBatch &bt, int nbatch, int pitch, int nx, int ny, 
         default: return false;
     }
 }
-bool r2c_t(int logh, const FftBatch &bt, int nbatch, int nx, int ny, int ibegy, const float2 *tw,
+bool r2c_t(int logh, const FftBatch &bt, int nbatch, int nx, int ny, int ioff, int ibegy, const float2 *tw,
            CorrParams cp, int pitch, cudaStream_t st, cudaError_t *err, int *status) {
     // image rows staged by bulk copy when they start on 16-byte boundaries
     bool staged = status && (nx & 3) == 0;
@@ -1389,7 +1392,7 @@ bool r2c_t(int logh, const FftBatch &bt, int nbatch, int nx, int ny, int ibegy, 
     int *st_status = staged ? status : nullptr;
     switch (logh) {
 #define CASE(L) \
-    case L: *err = launch_r2c_t<L>(bt, nbatch, nx, ny, ibegy, tw, cp, pitch, st_status, st); return true;
+    case L: *err = launch_r2c_t<L>(bt, nbatch, nx, ny, ioff, ibegy, tw, cp, pitch, st_status, st); return true;
         SDE_LOG_CASES(CASE)
 #undef CASE
         default: return false;
@@ -1606,30 +1609,36 @@ int image_from_raw(sde_ctx *ctx, const float2 *raw, const float2 *raw_lo, int nu
     return c2r_pass(ctx, grid, pitch, nx, ny, fnu, nv, correct, scale_dev, image, twu);
 }
 
-int sde_grid_from_image(sde_ctx *ctx, const float *image, int nx, int ny, int fnu, int nv,
-                        int correct, float *grid, int pitch) {
+// The grid of an nx x ny image lying at (lsx, lsy) of a px x py one that is zero elsewhere.  Only
+// the image's rows are read and transformed; the column pass takes the others as zero.
+static int grid_from_image_at(sde_ctx *ctx, const float *image, int nx, int ny, int lsx, int lsy, int px, int py,
+                              int fnu, int nv, int correct, float *grid, int pitch) {
     if (!ctx || !grid || !image) return SDE_EINVAL;
-    SDE_TRY(check_fft_args(nx, ny, fnu, nv, pitch));
+    SDE_TRY(check_fft_args(px, py, fnu, nv, pitch));
     SDE_CUDA_TRY(cudaSetDevice(ctx->device));
     const int nu = fnu / 2 + 1;
     const float2 *twv, *twu;
     SDE_TRY(ctx_twiddles(ctx, nv, &twv));
     SDE_TRY(ctx_twiddles(ctx, fnu, &twu));
     CorrParams cp = {nullptr, nullptr, nullptr};
-    if (correct) SDE_TRY(corr_params(ctx, nx, ny, &cp));
-    const int ibegy = (nv + 1) / 2 - (ny + 1) / 2;
+    if (correct) {
+        SDE_TRY(corr_params(ctx, px, py, &cp));
+        cp.corrx += lsx;
+        cp.corry += lsy;
+    }
+    const int ibegy = (nv + 1) / 2 - (py + 1) / 2 + lsy, ioff = (fnu - px) / 2 + lsx;
     {
         KTimer kt(ctx, "row_r2c");
         cudaError_t e = cudaSuccess;
         FftBatch bt{};
         bt.grid[0] = (float2 *)grid;
         bt.image[0] = const_cast<float *>(image);
-        if (!r2c_t(ilog2(fnu / 2), bt, 1, nx, ny, ibegy, twu, cp, pitch, ctx->stream, &e, ctx->d_status)) {
+        if (!r2c_t(ilog2(fnu / 2), bt, 1, nx, ny, ioff, ibegy, twu, cp, pitch, ctx->stream, &e, ctx->d_status)) {
             int rows, thr;
             row_shape(fnu, &rows, &thr);
             const size_t smr = sizeof(float2) * (size_t)(fnu / 2) * rows;
             SDE_CUDA_TRY(cudaFuncSetAttribute(k_row_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
-            k_row_r2c<<<ceil_div(ny, rows), thr, smr, ctx->stream>>>(image, nx, ny, fnu, rows, ibegy, twu,
+            k_row_r2c<<<ceil_div(ny, rows), thr, smr, ctx->stream>>>(image, nx, ny, fnu, rows, ioff, ibegy, twu,
                                                                     cp, (float2 *)grid, pitch, nu);
             e = cudaGetLastError();
         }
@@ -1654,4 +1663,18 @@ int sde_grid_from_image(sde_ctx *ctx, const float *image, int nx, int ny, int fn
     }
     SDE_CUDA_TRY(e);
     return SDE_OK;
+}
+
+int sde_grid_from_image(sde_ctx *ctx, const float *image, int nx, int ny, int fnu, int nv,
+                        int correct, float *grid, int pitch) {
+    return grid_from_image_at(ctx, image, nx, ny, 0, 0, nx, ny, fnu, nv, correct, grid, pitch);
+}
+
+int sde_grid_from_padded(sde_ctx *ctx, const float *image, int nx, int ny, int lsx, int lsy, int px, int py,
+                         int fnu, int nv, int correct, float *grid, int pitch) {
+    if (nx < 1 || ny < 1 || lsx < 0 || lsy < 0 || px < 1 || py < 1 || nx > px - lsx || ny > py - lsy) {
+        sde_set_error("sde_grid_from_padded: a %dx%d image at (%d, %d) does not lie in %dx%d", nx, ny, lsx, lsy, px, py);
+        return SDE_EINVAL;
+    }
+    return grid_from_image_at(ctx, image, nx, ny, lsx, lsy, px, py, fnu, nv, correct, grid, pitch);
 }

@@ -374,12 +374,27 @@ def imgtovis(ctx, geom, plan_padded, image, vis_out, wt_out):
     then IMGGRIDC CORRECT, IMGFFT and VISDEGRI on the padded image's grid.  plan_padded is a
     Plan built on padded_geom(geom) (once per job, like the degrid plan of a major cycle)."""
     pg = plan_padded.geom
-    pad, rx, ry = image_double(ctx, image, geom.cenx, geom.ceny)
+    ny, nx = int(image.shape[0]), int(image.shape[1])
+    if nx > 1 and ny > 1 and (fftpwr2(2 * nx), fftpwr2(2 * ny)) == (pg.nx, pg.ny):
+        # IMGDOUBL's margins NINT(P/2 - RPIX), whole numbers here; the padded image is not made:
+        # its rows of zeros need no transform
+        ls = [p // 2 - int(c) for p, c in ((pg.nx, geom.cenx), (pg.ny, geom.ceny))]
+        rx, ry = geom.cenx + ls[0], geom.ceny + ls[1]
+    else:
+        ls = None
+        pad, rx, ry = image_double(ctx, image, geom.cenx, geom.ceny)
     if (rx, ry) != (pg.cenx, pg.ceny):
         raise ValueError("imgtovis: the padded reference pixel (%g, %g) is not the padded grid's "
                          "centre (%g, %g)" % (rx, ry, pg.cenx, pg.ceny))
-    grid = ctx.grid_buffer(pg)
-    ctx.grid_from_image(pg, pad, grid)
+    if ls is None:
+        grid = ctx.grid_buffer(pg)
+        ctx.grid_from_image(pg, pad, grid)
+    else:
+        # the transform writes every cell but the pitch's padding
+        grid = ctx.empty((pg.nv, pg.pitch), ctx.torch.complex64)
+        grid[:, pg.nu:].zero_()
+        check(lib().sde_grid_from_padded(ctx.h, _ptr(image), nx, ny, ls[0], ls[1], pg.nx, pg.ny, pg.fnu, pg.nv, 1,
+                                         _ptr(grid), pg.pitch), "sde_grid_from_padded")
     return plan_padded.degrid(grid, vis_out, wt_out)
 
 

@@ -42,3 +42,39 @@ def test_narrow_shapes(gpu_ctx, orc, nx, ny, fnu, nv):
     back = ctx.zeros((nv, pitch), ctx.torch.complex64)
     ctx.grid_from_image(g, ctx.tensor(im), back, correct=False)
     assert rel_err(back.cpu().numpy()[:, :nu], refX) < 2e-6
+
+
+# IMGDOUBL's padding folded into the transform: the grid of the padded image, at margins that
+# are even and odd, with images of one row or column, and where whole 256-row boxes of the
+# column pass's input hold no image row (2048 and 4096 rows)
+@pytest.mark.parametrize("nx,ny,lsx,lsy,px,py", [(33, 30, 15, 17, 64, 64), (1, 7, 5, 0, 16, 16), (100, 1, 14, 127, 128, 128),
+                                                 (501, 499, 262, 263, 1024, 1024), (300, 900, 0, 1148, 2048, 2048),
+                                                 (750, 700, 649, 675, 2048, 2048), (1499, 1499, 1298, 1298, 4096, 4096),
+                                                 (2048, 100, 1024, 2000, 4096, 4096)])
+@pytest.mark.parametrize("correct", [False, True])
+def test_grid_of_padded_image(gpu_ctx, nx, ny, lsx, lsy, px, py, correct):
+    """Equal to padding first: the same operations on the same numbers (zeros of either sign)."""
+    from sde_gb300._abi import check, lib
+    from sde_gb300.imaging import _ptr
+    ctx, torch = gpu_ctx, gpu_ctx.torch
+    rng = np.random.default_rng(nx + ny)
+    im = ctx.tensor(rng.standard_normal((ny, nx)).astype(np.float32))
+    pad = ctx.zeros((py, px), torch.float32)
+    pad[lsy:lsy + ny, lsx:lsx + nx] = im
+    pitch = (px // 2 + 1 + 3) & ~3
+    want = ctx.zeros((py, pitch), torch.complex64)
+    got = torch.full_like(want, float("nan"))
+    check(lib().sde_grid_from_image(ctx.h, _ptr(pad), px, py, px, py, int(correct), _ptr(want), pitch), "image")
+    check(lib().sde_grid_from_padded(ctx.h, _ptr(im), nx, ny, lsx, lsy, px, py, px, py, int(correct), _ptr(got), pitch),
+          "padded")
+    nu = px // 2 + 1
+    assert torch.equal(torch.view_as_real(got[:, :nu]), torch.view_as_real(want[:, :nu]))
+
+
+def test_padded_image_must_lie_inside(gpu_ctx):
+    from sde_gb300._abi import lib
+    from sde_gb300.imaging import _ptr
+    ctx, torch = gpu_ctx, gpu_ctx.torch
+    im, g = ctx.zeros((8, 8), torch.float32), ctx.zeros((32, 20), torch.complex64)
+    for nx, ny, lsx, lsy in ((8, 8, -1, 0), (8, 8, 25, 0), (8, 8, 0, 25), (0, 8, 0, 0)):
+        assert lib().sde_grid_from_padded(ctx.h, _ptr(im), nx, ny, lsx, lsy, 32, 32, 32, 32, 0, _ptr(g), 20) == 1
