@@ -661,11 +661,26 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
         // Every lane of a warp runs the same number of group iterations (the loop bounds are
         // per item), so the shuffles below always see all 32 lanes.
         const int ngroups_iter = (it.cend - it.cbeg + DG_GROUPS - 1) / DG_GROUPS;
-        for (int gi = it.r0; gi < ngroups_iter; gi += it.rstep) {
+        // The next round's chunk word and the first words of its visibilities are loaded a round
+        // ahead, so that short chunks (a few visibilities) do not wait for three loads in turn:
+        // 1.3 M visibilities on 4096^2, residuals 67 -> 59 us, in the caller's frame 94 -> 81.
+        auto chunk_of = [&](int gi) {
             const int c = it.cbeg + gi * DG_GROUPS + grp;
-            const bool live = c < it.cend;
-            const uint2 ch = live ? chunks[c] : make_uint2(0u, 0u);
-            const int start = (int)ch.x, len = live ? (int)(ch.y >> 16) : 0;
+            return gi < ngroups_iter && c < it.cend ? chunks[c] : make_uint2(0u, 0u);
+        };
+        uint2 ch1 = chunk_of(it.r0), ch2 = chunk_of(it.r0 + it.rstep);
+        uint32_t gq1 = q < (int)(ch1.y >> 16) ? gdd[(int)ch1.x + q] : GDD_PAD;
+        float2 ob1 = make_float2(0.f, 0.f);
+        if (MODE == 0 && q < (int)(ch1.y >> 16)) ob1 = fobs[(int)ch1.x + q];
+        for (int gi = it.r0; gi < ngroups_iter; gi += it.rstep) {
+            const uint2 ch = ch1;
+            const int start = (int)ch.x, len = (int)(ch.y >> 16);
+            uint32_t gqn = gq1;
+            float2 obn = ob1;
+            ch1 = ch2;
+            gq1 = q < (int)(ch1.y >> 16) ? gdd[(int)ch1.x + q] : GDD_PAD;
+            if (MODE == 0 && q < (int)(ch1.y >> 16)) ob1 = fobs[(int)ch1.x + q];
+            ch2 = chunk_of(gi + 2 * it.rstep);
             const int cell = (int)(ch.y & 4095u), lu = cell & 63, lv = cell >> 6;
             float2 G0[NTAP], G1[NTAP];
 #pragma unroll
@@ -680,9 +695,6 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
             for (int d = 4; d < 32; d <<= 1) wlen = max(wlen, __shfl_xor_sync(FULL, wlen, d));
             // lane q loads the offset word and observed value of visibility q of the next
             // batch (one coalesced load per group); the group shares the words by shuffle
-            uint32_t gqn = q < len ? gdd[start + q] : GDD_PAD;
-            float2 obn = make_float2(0.f, 0.f);
-            if (MODE == 0 && q < len) obn = fobs[start + q];
             for (int k = 0; k < wlen; k += 4) {
                 const int pq = start + k + q;
                 const bool mine = k + q < len;
@@ -691,6 +703,15 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
                 if (k + 4 + q < len) {
                     gqn = gdd[pq + 4];
                     if (MODE == 0) obn = fobs[pq + 4];
+                }
+                // the frame of the caller's visibility, on its way while the four are summed
+                uint8_t cj = 0;
+                float2 rt = make_float2(1.f, 0.f);
+                float w = 0.f;
+                if (MODE == 1 && mine) {
+                    cj = gconj[pq];
+                    if (rot) rt = rot[pq];
+                    w = wt[pq];
                 }
                 float pr[4], pim[4];
 #pragma unroll
@@ -734,13 +755,10 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
                 } else {
                     // caller's frame, staged in plan order (k_gather_user puts it in the
                     // caller's order with coalesced writes)
-                    if (gconj[pq]) mi = -mi;
+                    if (cj) mi = -mi;
                     float2 vv = make_float2(mr, mi);
-                    if (rot) {
-                        const float2 rt = rot[pq];
-                        vv = make_float2(mr * rt.x - mi * rt.y, mr * rt.y + mi * rt.x);
-                    }
-                    stage[pq] = make_float4(vv.x, vv.y, wt[pq], 0.f);
+                    if (rot) vv = make_float2(mr * rt.x - mi * rt.y, mr * rt.y + mi * rt.x);
+                    stage[pq] = make_float4(vv.x, vv.y, w, 0.f);
                 }
             }
         }
