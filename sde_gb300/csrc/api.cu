@@ -322,7 +322,11 @@ static int ensure_sums(sde_plan *pl) {
 static int plan_raw_pass(sde_plan *pl, int what, float2 **raw, float2 **raw_lo) {
     sde_ctx *ctx = pl->ctx;
     const size_t cells = (size_t)pl->spec.nv * pl->pitch;
-    SDE_TRY(ctx_scratch(ctx, "raw_grid", sizeof(float2) * cells * (ctx->compensated ? 2 : 1), (void **)raw));
+    // the launch list's counter lies before the grid: one memset clears both
+    float2 *base;
+    SDE_TRY(ctx_scratch(ctx, "raw_grid", RAW_HEAD + sizeof(float2) * cells * (ctx->compensated ? 2 : 1),
+                        (void **)&base));
+    *raw = base + RAW_HEAD / sizeof(float2);
     *raw_lo = ctx->compensated ? *raw + cells : nullptr;
     // the compensation plane stays zero between passes (the fold re-zeroes what a pass
     // wrote); it is cleared only when the scratch is new
@@ -627,6 +631,15 @@ static int fstr_eq(const char *s, size_t len, const char *lit) {
 
 // upload the caller's 'SF'-style table into the plan (1+2*(SUPP+1)*OSAMP values)
 static int plan_use_table(sde_plan *pl, const float *cf) {
+    // its own table in place of the context's
+    if (!pl->table) {
+        const size_t cfs = (CFLEN + 63) / 64 * 64, bytes = sizeof(float) * (cfs + 129 * 8);
+        SDE_TRY(ctx_alloc(pl->ctx, (void **)&pl->table, bytes));
+        pl->bytes += (int64_t)bytes;
+        pl->ctx->bytes += (int64_t)bytes;
+        pl->cf = pl->table;
+        pl->cft = pl->table + cfs;
+    }
     SDE_CUDA_TRY(shim_memcpy(pl->cf, cf, sizeof(float) * (2 * (SUPP + 1) * OSAMP + 1),
                                  cudaMemcpyHostToDevice, pl->ctx->stream));
     return plan_build_cft(pl);

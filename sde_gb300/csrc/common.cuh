@@ -220,6 +220,10 @@ struct sde_plan {
     int64_t nitems = 0, nchunks = 0, nexc = 0;
     int item_max = ITEM_MAX, chunk_max = CHUNK_MAX;  // sort-bucket sizes of this plan
     // sorted, gridding-valid visibilities
+    // the arrays below lie in two allocations: what the first counts size, and what the number
+    // of chunks sizes (one malloc costs the host about a microsecond while the device waits)
+    void *slab[2] = {nullptr, nullptr};
+    float *table = nullptr;
     float2 *fobs = nullptr;   // observed, in the gridding frame (rotated, conjugated)
     float4 *rec = nullptr;    // {WT, gdg bits, residual re, residual im} (gridding frame):
                               // the gridder reads one 16-byte record per visibility
@@ -232,7 +236,7 @@ struct sde_plan {
     WorkItem *items = nullptr;
     WorkItem *parts = nullptr;  // launch list of the gridder and degridder (item_parts)
     int64_t parts_max = 0;      // entries it has room for; their count is at nparts
-    unsigned long long *nparts = nullptr;  // after the entries, in the same allocation
+    unsigned long long *nparts = nullptr;  // device count of the launch list's entries
     DegridExc *exc = nullptr; // exception list (includes degrid-only visibilities)
     float *wt_all = nullptr;  // caller-order weights (for user-frame degridding)
     uint8_t *core_lo = nullptr;  // (ntu+1) x (ntv+1) raw-grid cores where the compensation
@@ -240,7 +244,9 @@ struct sde_plan {
     int32_t *inv = nullptr;   // caller index -> position of the tiled visibilities (-1 else),
                               // built on the first caller-order degrid
     int64_t nuntouched = 0;   // caller visibilities with WT <= 0 (GRDDEH2D leaves them as they are)
-    float *cf = nullptr;      // gridding function used by this plan (device, CFLEN)
+    // gridding function used by this plan (device, CFLEN): the context's, or the plan's own
+    // (table) after plan_use_table
+    float *cf = nullptr;
     float *cft = nullptr;     // transposed table
     double *d_sums = nullptr; // [0] sum of UVWT (LSUMWT), [1] SUMWT
     double h_lsumwt = 0.0, h_sumwt = 0.0;
@@ -249,6 +255,12 @@ struct sde_plan {
 };
 
 // grid.cu internals used by api.cu
+int weights_queue(sde_ctx *ctx, int rmode, const float robust[3], float ds, const float *wt, const float *u,
+                  const float *v, const float *w, int64_t nvis, float uscale, float uoffset, float vscale,
+                  float voffset, int uorigin, int vorigin, int nu, int nv, const double shift[9], float *newwt,
+                  float *gwt, sde_wstats *stats);
+// bytes before a raw grid (plan_raw_pass) that hold the gridder's counter
+constexpr size_t RAW_HEAD = 256;
 int plan_build_cft(sde_plan *pl);
 int ctx_build_cft(sde_ctx *ctx);
 int plan_sums(sde_plan *pl, double *lsumwt, double *sumwt);

@@ -1051,7 +1051,8 @@ int launch_fold_lo_batch(sde_ctx *ctx, const BatchPlan *d_plans, const int2 *cor
 int plan_grid_raw(sde_plan *pl, int what, float2 *raw, float2 *raw_lo, bool lo_clean) {
     sde_ctx *ctx = pl->ctx;
     const int nu = pl->spec.nu, nv = pl->spec.nv;
-    SDE_CUDA_TRY(cudaMemsetAsync(raw, 0, sizeof(float2) * (size_t)nv * pl->pitch, ctx->stream));
+    unsigned long long *counter = reinterpret_cast<unsigned long long *>(raw - RAW_HEAD / sizeof(float2));
+    SDE_CUDA_TRY(cudaMemsetAsync(counter, 0, RAW_HEAD + sizeof(float2) * (size_t)nv * pl->pitch, ctx->stream));
     if (raw_lo && !lo_clean)
         SDE_CUDA_TRY(cudaMemsetAsync(raw_lo, 0, sizeof(float2) * (size_t)nv * pl->pitch, ctx->stream));
     if (pl->nitems == 0) return SDE_OK;
@@ -1067,9 +1068,6 @@ int plan_grid_raw(sde_plan *pl, int what, float2 *raw, float2 *raw_lo, bool lo_c
                                           (int)grid_smem()));
         attr = true;
     }
-    unsigned long long *counter;
-    SDE_TRY(ctx_scratch(ctx, "grid_counter", sizeof(unsigned long long), (void **)&counter));
-    SDE_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), ctx->stream));
     KTimer kt(ctx, what == SDE_GRID_PSF ? "grid_psf" : "grid");
     const int64_t want = (int64_t)ctx->num_sms;
     const dim3 g((unsigned)(pl->parts_max < want ? pl->parts_max : want)), b(GRID_THREADS);

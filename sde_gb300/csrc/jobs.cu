@@ -42,13 +42,15 @@ extern "C" int sde_uvmap(sde_ctx *ctx, const sde_uvmap_args *a, int64_t nvis, co
     sde_uvmap_result r{};
     if (a->rmode >= 0) {
         sde_wstats ws{};
-        SDE_TRY(sde_weights(ctx, a->rmode, a->robust, a->ds, dwt, du, dv, dw, nvis, a->wuscale, 0.0f,
-                            a->wvscale, 0.0f, sp.uorigin, sp.vorigin, sp.nu, sp.nv, sp.shift, dwt,
-                            nullptr, &ws));
+        SDE_TRY(weights_queue(ctx, a->rmode, a->robust, a->ds, dwt, du, dv, dw, nvis, a->wuscale, 0.0f, a->wvscale,
+                              0.0f, sp.uorigin, sp.vorigin, sp.nu, sp.nv, sp.shift, dwt, nullptr, &ws));
         r.ndrop = ws.ndrop;
     }
     sde_plan *pl = nullptr;
-    SDE_TRY(sde_plan_create(ctx, &sp, nvis, du, dv, dw, dvis, dwt, SDE_DEVICE, &pl));
+    if (const int e = sde_plan_create(ctx, &sp, nvis, du, dv, dw, dvis, dwt, SDE_DEVICE, &pl)) {
+        cudaStreamSynchronize(st);  // the weighting may still read the caller's arrays
+        return e;
+    }
     r.ngrid = pl->nvis;
     const int pitch = sde_grid_pitch(sp.nu);
     const int64_t npix = (int64_t)a->nx * a->ny;

@@ -557,20 +557,39 @@ int sde_plan_stats(const sde_plan *plan, int64_t *nitems, int64_t *nchunks, int6
     return SDE_OK;
 }
 
-static int plan_alloc(sde_plan *pl, void **p, size_t bytes) {
-    if (bytes == 0) bytes = 16;
-    int rc = ctx_alloc(pl->ctx, p, bytes);
-    if (rc == SDE_OK) pl->bytes += (int64_t)bytes;
-    return rc;
-}
+// Several arrays in one allocation, each on a 256-byte boundary.
+struct Slab {
+    size_t bytes = 0;
+    struct Part {
+        void **p;
+        size_t off;
+    };
+    std::vector<Part> parts;
+    template <class T>
+    void add(T **p, size_t n) {
+        parts.push_back({reinterpret_cast<void **>(p), bytes});
+        bytes += (n + 255) & ~(size_t)255;
+    }
+    // The size is rounded up by at most 1/16, so that plans of about the same number of
+    // visibilities take each other's blocks from the pool: mapping new ones costs milliseconds
+    // at 65 M visibilities.
+    int alloc(sde_plan *pl, void **base) {
+        size_t step = 256;
+        while (step * 32 <= bytes) step *= 2;
+        bytes = (bytes + step - 1) / step * step;
+        SDE_TRY(ctx_alloc(pl->ctx, base, bytes));
+        pl->bytes += (int64_t)bytes;
+        for (const Part &q : parts) *q.p = static_cast<char *>(*base) + q.off;
+        return SDE_OK;
+    }
+};
 
 int sde_plan_destroy(sde_plan *pl) {
     if (!pl) return SDE_OK;
     sde_ctx *ctx = pl->ctx;
     cudaSetDevice(ctx->device);
     // stream-ordered frees: after the plan's last use on the context's stream
-    void *ptrs[] = {pl->fobs, pl->rec, pl->wt, pl->gdd, pl->orig, pl->rot, pl->gconj, pl->chunks,
-                    pl->items, pl->parts, pl->exc, pl->wt_all, pl->cf, pl->cft, pl->d_sums, pl->inv, pl->core_lo};
+    void *ptrs[] = {pl->slab[0], pl->slab[1], pl->table, pl->wt_all, pl->inv};
     for (void *p : ptrs) ctx_free(ctx, p, 0);
     ctx->bytes -= pl->bytes;
     delete pl;
@@ -724,18 +743,26 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
         pl->nvis = nvalid;
         pl->nexc = nexc;
         const size_t nv1 = (size_t)(nvalid > 0 ? nvalid : 1);
-        PL_TRY(plan_alloc(pl, (void **)&pl->fobs, 8 * nv1));
-        PL_TRY(plan_alloc(pl, (void **)&pl->rec, 16 * nv1));
-        PL_TRY(plan_alloc(pl, (void **)&pl->wt, 4 * nv1));
-        PL_TRY(plan_alloc(pl, (void **)&pl->gdd, 4 * nv1));
-        PL_TRY(plan_alloc(pl, (void **)&pl->orig, 4 * nv1));
-        PL_TRY(plan_alloc(pl, (void **)&pl->gconj, nv1));
-        if (pl->doshift) PL_TRY(plan_alloc(pl, (void **)&pl->rot, 8 * nv1));
-        PL_TRY(plan_alloc(pl, (void **)&pl->d_sums, 4 * sizeof(double)));
+        // at most one item per tile that has a run and one more per item_max visibilities; a
+        // chunk per run, per item inside a run, and per chunk_max visibilities
+        const int64_t nruns = nvalid > 0 ? (int64_t)hc.runs.total : 0;
+        const int64_t max_items = std::min(ntiles, nruns) + nvalid / pl->item_max;
+        const int64_t max_chunks = nruns + max_items + nvalid / pl->chunk_max;
+        const size_t ne1 = (size_t)(nexc > 0 ? nexc : 1);
+        Slab a;
+        a.add(&pl->fobs, 8 * nv1);
+        a.add(&pl->rec, 16 * nv1);
+        a.add(&pl->wt, 4 * nv1);
+        a.add(&pl->gdd, 4 * nv1);
+        a.add(&pl->orig, 4 * nv1);
+        a.add(&pl->gconj, nv1);
+        if (pl->doshift) a.add(&pl->rot, 8 * nv1);
+        a.add(&pl->d_sums, 4 * sizeof(double));
+        a.add(&pl->exc, exc_bytes(ne1));
+        if (nvalid > 0) a.add(&pl->items, sizeof(WorkItem) * (size_t)max_items);
+        PL_TRY(a.alloc(pl, &pl->slab[0]));
         // exception list (also carries the GRDDEH2D geometry of non-gridding visibilities);
         // the gather below fills in the sorted positions
-        size_t ne1 = (size_t)(nexc > 0 ? nexc : 1);
-        PL_TRY(plan_alloc(pl, (void **)&pl->exc, exc_bytes(ne1)));
         if (nexc > 0) {
             float *exc_wt = (float *)((char *)pl->exc + exc_wt_off(ne1));
             float2 *exc_rot = (float2 *)((char *)pl->exc + exc_rot_off(ne1));
@@ -745,18 +772,12 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
         }
         // runs, chunks, work items
         if (nvalid > 0) {
-            // at most one item per tile that has a run and one more per item_max visibilities; a
-            // chunk per run, per item inside a run, and per chunk_max visibilities
-            const int64_t nruns = (int64_t)hc.runs.total;
-            const int64_t max_items = std::min(ntiles, nruns) + nvalid / pl->item_max;
-            const int64_t max_chunks = nruns + max_items + nvalid / pl->chunk_max;
             uint64_t *ckey;
             uint2 *craw;
             uint32_t *csrc;
             PL_TRY(ctx_scratch(ctx, "pl_ckey", 8 * (size_t)max_chunks, (void **)&ckey));
             PL_TRY(ctx_scratch(ctx, "pl_craw", 8 * (size_t)max_chunks, (void **)&craw));
             PL_TRY(ctx_scratch(ctx, "pl_csrc", 4 * (size_t)max_chunks, (void **)&csrc));
-            PL_TRY(plan_alloc(pl, (void **)&pl->items, sizeof(WorkItem) * (size_t)max_items));
             const int jbits = bits_for(pl->item_max / pl->chunk_max);
             const int lbits = bits_for(pl->chunk_max - 1);
             k_run_emit<<<ceil_div(nruns, SC_T * SC_R), SC_T, 0, st>>>(
@@ -767,16 +788,19 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
             const int64_t nitems = (int64_t)(hc.emit.total >> 31), nchunks = (int64_t)(hc.emit.total & 0x7FFFFFFFull);
             pl->nitems = nitems;
             pl->nchunks = nchunks;
-            PL_TRY(plan_alloc(pl, (void **)&pl->chunks, sizeof(uint2) * (size_t)nchunks));
             // an item has at most ceil(visibilities / part) entries
             const int part = part_size(nvis);
             pl->parts_max = nitems + nvalid / part;
-            PL_TRY(plan_alloc(pl, (void **)&pl->parts, sizeof(WorkItem) * (size_t)(pl->parts_max + 1)));
-            pl->nparts = reinterpret_cast<unsigned long long *>(pl->parts + pl->parts_max);
-            PL_CUDA(cudaMemsetAsync(pl->nparts, 0, sizeof(unsigned long long), st));
             const size_t ncore = (size_t)(pl->ntu + 1) * (pl->ntv + 1);
-            PL_TRY(plan_alloc(pl, (void **)&pl->core_lo, ncore));
-            PL_CUDA(cudaMemsetAsync(pl->core_lo, 0, ncore, st));
+            uint8_t *zero;  // the entries' count, then the cores
+            Slab b;
+            b.add(&pl->chunks, sizeof(uint2) * (size_t)nchunks);
+            b.add(&pl->parts, sizeof(WorkItem) * (size_t)pl->parts_max);
+            b.add(&zero, sizeof(unsigned long long) + ncore);
+            PL_TRY(b.alloc(pl, &pl->slab[1]));
+            pl->nparts = reinterpret_cast<unsigned long long *>(zero);
+            pl->core_lo = zero + sizeof(unsigned long long);
+            PL_CUDA(cudaMemsetAsync(zero, 0, sizeof(unsigned long long) + ncore, st));
             k_item_finish<<<ceil_div(nitems, T), T, 0, st>>>(pl->items, nitems, nchunks, nvalid, pl->ntu, pl->core_lo,
                                                            pl->item_max, part, pl->parts, pl->nparts);
             PL_CUDA(cudaGetLastError());
@@ -789,10 +813,8 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
             PL_CUDA(cudaGetLastError());
         }
         // gridding function: the context's 'SF' table
-        PL_TRY(plan_alloc(pl, (void **)&pl->cf, sizeof(float) * CFLEN));
-        PL_TRY(plan_alloc(pl, (void **)&pl->cft, sizeof(float) * 129 * 8));
-        PL_CUDA(cudaMemcpyAsync(pl->cf, ctx->d_cf, sizeof(float) * CFLEN, cudaMemcpyDeviceToDevice, st));
-        PL_CUDA(cudaMemcpyAsync(pl->cft, ctx->d_cft, sizeof(float) * 129 * 8, cudaMemcpyDeviceToDevice, st));
+        pl->cf = ctx->d_cf;
+        pl->cft = ctx->d_cft;
     }
     ctx->bytes += pl->bytes;
     *out = pl;

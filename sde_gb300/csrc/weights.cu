@@ -458,10 +458,11 @@ int key_bits(int64_t maxkey) {
 
 }  // namespace
 
-int sde_weights(sde_ctx *ctx, int rmode, const float robust[3], float ds, const float *wt,
-                const float *u, const float *v, const float *w, int64_t nvis, float uscale,
-                float uoffset, float vscale, float voffset, int uorigin, int vorigin, int nu,
-                int nv, const double shift[9], float *newwt, float *gwt, sde_wstats *stats) {
+// sde_weights up to its last wait: the new weights may still be on their way on the stream.
+int weights_queue(sde_ctx *ctx, int rmode, const float robust[3], float ds, const float *wt, const float *u,
+                  const float *v, const float *w, int64_t nvis, float uscale, float uoffset, float vscale,
+                  float voffset, int uorigin, int vorigin, int nu, int nv, const double shift[9], float *newwt,
+                  float *gwt, sde_wstats *stats) {
     if (!ctx || nvis < 0 || nu <= 0 || nv <= 0 || !shift) {
         sde_set_error("sde_weights: bad arguments");
         return SDE_EINVAL;
@@ -494,8 +495,9 @@ int sde_weights(sde_ctx *ctx, int rmode, const float robust[3], float ds, const 
     SDE_TRY(ctx_scratch(ctx, "w_vals", nb4, (void **)&vals));
     SDE_TRY(ctx_scratch(ctx, "w_ktmp", nb4, (void **)&ktmp));
     SDE_TRY(ctx_scratch(ctx, "w_vtmp", nb4, (void **)&vtmp));
-    SDE_TRY(ctx_scratch(ctx, "w_counts", 64, (void **)&counts));
-    SDE_CUDA_TRY(cudaMemsetAsync(counts, 0, 64, st));
+    SDE_TRY(ctx_scratch(ctx, "w_counts", 64 + 2 * sizeof(double), (void **)&counts));
+    double *sums = reinterpret_cast<double *>(counts + 8);  // [0] sumwt [1] sumlocwt
+    SDE_CUDA_TRY(cudaMemsetAsync(counts, 0, 64 + 2 * sizeof(double), st));
     if (nvis > 0) {
         (rot ? k_wkey<true> : k_wkey<false>)<<<ceil_div(nvis, W_T * W_PER), W_T, 0, st>>>(p, wt, u, v, w, nvis, keys, counts);
         SDE_CHECK_LAUNCH();
@@ -512,9 +514,6 @@ int sde_weights(sde_ctx *ctx, int rmode, const float robust[3], float ds, const 
     float f2 = 1.0f, d2 = 0.0f;
     AzParams az;
     memset(&az, 0, sizeof az);
-    double *sums;  // [0] sumwt [1] sumlocwt
-    SDE_TRY(ctx_scratch(ctx, "w_sums", 2 * sizeof(double), (void **)&sums));
-    SDE_CUDA_TRY(cudaMemsetAsync(sums, 0, 2 * sizeof(double), st));
     unsigned long long hcounts[8] = {0};
     double hs[2] = {0.0, 0.0};
     const int robust_mode = rmode >= 1;
@@ -536,12 +535,11 @@ int sde_weights(sde_ctx *ctx, int rmode, const float robust[3], float ds, const 
             k_sum_partials<<<1, RED_THREADS, 0, st>>>(part, nbc, sums + 1);
             SDE_CHECK_LAUNCH();
         }
-        // both through the context's pinned bytes (one wait)
-        SDE_CUDA_TRY(cudaMemcpyAsync(ctx->h_small, sums, sizeof hs, cudaMemcpyDeviceToHost, st));
-        SDE_CUDA_TRY(cudaMemcpyAsync(ctx->h_small + sizeof hs, counts, sizeof hcounts, cudaMemcpyDeviceToHost, st));
-        SDE_CUDA_TRY(cudaStreamSynchronize(st));
-        memcpy(hs, ctx->h_small, sizeof hs);
-        memcpy(hcounts, ctx->h_small + sizeof hs, sizeof hcounts);
+        // counts and sums lie together: one copy
+        unsigned char both[sizeof hcounts + sizeof hs];
+        SDE_TRY(ctx_read_small(ctx, st, both, counts, sizeof both));
+        memcpy(hcounts, both, sizeof hcounts);
+        memcpy(hs, both + sizeof hcounts, sizeof hs);
         if (hcounts[7]) {
             sde_set_error("sde_weights: a device wait timed out");
             return SDE_ETIMEDOUT;
@@ -585,7 +583,16 @@ int sde_weights(sde_ctx *ctx, int rmode, const float robust[3], float ds, const 
         stats->sumlocwt = hs[1];
         stats->f2 = f2;
         stats->d2 = d2;
-        SDE_CUDA_TRY(cudaStreamSynchronize(st));
     }
+    return SDE_OK;
+}
+
+int sde_weights(sde_ctx *ctx, int rmode, const float robust[3], float ds, const float *wt,
+                const float *u, const float *v, const float *w, int64_t nvis, float uscale,
+                float uoffset, float vscale, float voffset, int uorigin, int vorigin, int nu,
+                int nv, const double shift[9], float *newwt, float *gwt, sde_wstats *stats) {
+    SDE_TRY(weights_queue(ctx, rmode, robust, ds, wt, u, v, w, nvis, uscale, uoffset, vscale, voffset, uorigin, vorigin,
+                          nu, nv, shift, newwt, gwt, stats));
+    if (stats) SDE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return SDE_OK;
 }
