@@ -440,6 +440,7 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
         std::vector<BatchItem> list;
         std::vector<WorkItem> items;
         const int part = part_size(set_vis);
+        std::vector<char> in_parts((size_t)n, 0);  // plans with items in parts (of the set)
         for (int i = 0; i < n && e == cudaSuccess; i++) {
             const sde_plan *pl = b->plans[i];
             items.resize((size_t)pl->nitems);
@@ -449,6 +450,10 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
             if (e != cudaSuccess) break;
             for (WorkItem it : items) {
                 it.rstep = item_parts(it, part);
+                if (it.rstep > 1) {
+                    it.dense = 1;
+                    in_parts[(size_t)i] = 1;
+                }
                 for (it.r0 = 0; it.r0 < it.rstep; it.r0++) list.push_back(BatchItem{it, i});
             }
         }
@@ -474,7 +479,7 @@ extern "C" int sde_batch_create(sde_ctx *ctx, int n, sde_plan *const *plans, con
                 if (e == cudaSuccess) e = cudaStreamSynchronize(st);
                 for (int cv = 0; cv < ncv && e == cudaSuccess; cv++)
                     for (int cu = 0; cu < ncu; cu++)
-                        if (core[(size_t)cv * ncu + cu]) fold.push_back(make_int2(i, cu | (cv << 16)));
+                        if (core[(size_t)cv * ncu + cu] & (in_parts[(size_t)i] ? ~0u : CORE_DENSE)) fold.push_back(make_int2(i, cu | (cv << 16)));
             }
         }
         if (e == cudaSuccess && !fold.empty()) {

@@ -136,6 +136,7 @@ __host__ __device__ inline int item_parts(const WorkItem &it, int part) {
 // A tile this full has many work items, so its cells receive long sums across items: those
 // sums are the ones compensated (sde_ctx_set_compensated).
 constexpr int DENSE_TILE_VIS = 65536;
+constexpr unsigned CORE_DENSE = 1, CORE_PARTS = 2;
 
 // ---------------------------------------------------------------------------------------
 // Context: one device, one stream, grow-only scratch buffers, cached tables.
@@ -239,8 +240,9 @@ struct sde_plan {
     unsigned long long *nparts = nullptr;  // device count of the launch list's entries
     DegridExc *exc = nullptr; // exception list (includes degrid-only visibilities)
     float *wt_all = nullptr;  // caller-order weights (for user-frame degridding)
-    uint8_t *core_lo = nullptr;  // (ntu+1) x (ntv+1) raw-grid cores where the compensation
-                                 // plane can be non-zero (dense tiles' footprints)
+    // (ntu+1) x (ntv+1) raw-grid cores where the compensation plane can be non-zero: the
+    // footprints of dense tiles (CORE_DENSE) and of items in parts (CORE_PARTS)
+    uint8_t *core_lo = nullptr;
     int32_t *inv = nullptr;   // caller index -> position of the tiled visibilities (-1 else),
                               // built on the first caller-order degrid
     int64_t nuntouched = 0;   // caller visibilities with WT <= 0 (GRDDEH2D leaves them as they are)

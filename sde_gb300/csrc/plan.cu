@@ -421,12 +421,13 @@ __global__ void __launch_bounds__(SC_T) k_run_emit(const uint32_t *__restrict__ 
 // cells and 3-cell halo, raw rows [64 tv - 3, 64 tv + 67), raw indices [64 tu - 2,
 // 64 tu + 68)) lies in cores (tu, tv), (tu+1, tv), (tu, tv+1), (tu+1, tv+1), where core
 // (cu, cv) is raw rows [64 cv - 3, 64 cv + 61) x raw indices [64 cu - 2, 64 cu + 62).
-__device__ __forceinline__ void mark_cores(int tile, int ntu, uint8_t *core) {
+// (core starts on a 4-byte boundary, and its last word is the plan's)
+__device__ __forceinline__ void mark_cores(int tile, int ntu, uint8_t *core, unsigned mark) {
     const int tu = tile % ntu, tv = tile / ntu, ncu = ntu + 1;
-    core[tv * ncu + tu] = 1;
-    core[tv * ncu + tu + 1] = 1;
-    core[(tv + 1) * ncu + tu] = 1;
-    core[(tv + 1) * ncu + tu + 1] = 1;
+    uint32_t *words = reinterpret_cast<uint32_t *>(core);
+    const int at[4] = {tv * ncu + tu, tv * ncu + tu + 1, (tv + 1) * ncu + tu, (tv + 1) * ncu + tu + 1};
+#pragma unroll
+    for (int k = 0; k < 4; k++) atomicOr(&words[at[k] >> 2], mark << (8 * (at[k] & 3)));
 }
 
 // Each item's ends, its dense flag (its tile's items, contiguous, hold >= DENSE_TILE_VIS
@@ -461,8 +462,12 @@ __global__ void k_item_finish(WorkItem *items, int64_t nitems, int64_t nchunks, 
     items[t].cend = it.cend;
     items[t].vend = it.vend;
     items[t].dense = it.dense;
-    if (it.dense) mark_cores(tile, ntu, core);
+    // parts add to the same cells as items of a dense tile do: their sums are compensated too
+    // (84 240 visibilities on 512^2, two runs' PSFs apart: 2.4e-4 without, 8e-5 with, 1.6e-4 with
+    // whole items; gridding 27.6 -> 28.1 us)
     const int np = item_max <= part ? 1 : item_parts(it, part);
+    if (it.dense || np > 1) mark_cores(tile, ntu, core, it.dense ? CORE_DENSE : CORE_PARTS);
+    if (np > 1) it.dense = 1;
     const unsigned long long at =
         item_max <= part ? (unsigned long long)t : atomicAdd(nparts, (unsigned long long)np);
     if (item_max <= part && t == 0) *nparts = (unsigned long long)nitems;
