@@ -15,11 +15,12 @@ __device__ __forceinline__ void lb_publish(unsigned long long *w, unsigned long 
 }
 
 // Sum of the tiles before `tile` (one thread; the words of consecutive tiles are `stride`
-// apart).  Four words are read at a time, in flight together.  *fail is set and 0 returned
-// when a word does not arrive.
+// apart).  Eight words are read at a time, in flight together (four: 2 % slower in a sort pass of
+// 64.7 million pairs, 12 % at 1.3 million).  *fail is set and 0 returned when a word does not
+// arrive.
 __device__ __forceinline__ unsigned long long lb_sum_before(const unsigned long long *words, int64_t tile,
                                                             int64_t stride, unsigned long long *fail) {
-    constexpr int A = 4;
+    constexpr int A = 8;
     unsigned long long sum = 0;
     int64_t p = tile - 1;
     for (int spin = 0; spin < LB_SPIN; spin++) {

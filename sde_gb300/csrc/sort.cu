@@ -9,7 +9,7 @@
 // sums the counts of the tiles before it by look-back (lookback.cuh) and writes each digit's
 // run of the tile to consecutive addresses.  Separate count, scan and scatter kernels read
 // the keys twice a pass and took five launches: 64.7 million pairs, three passes 1.75 ms, here
-// 1.46 ms; 84 240 pairs 0.11 ms, here 0.04 ms.
+// 1.27 ms; 84 240 pairs 0.11 ms, here 0.04 ms.
 #include <algorithm>
 
 #include "common.cuh"
@@ -84,7 +84,11 @@ __global__ void __launch_bounds__(RS_HT) k_rs_hist(const uint32_t *__restrict__ 
 // item order is (warp, round, lane)).  vin == NULL: the values are the items' indices.  The
 // lanes of a round with the same digit find each other through a word per digit in shared
 // memory, whose bits they set by atomics (64.7 million pairs a pass: match.any 670 us, eight
-// ballots 660 us, this 390 us, at 6144 items a tile).
+// ballots 660 us, this 390 us, at 6144 items a tile of 256 threads).  Bound by the latency of
+// ranking and of the loads, so by the warps resident: three passes of 64.7 million pairs take
+// 1.52 ms with tiles of 256 x 24, 1.39 of 384 x 12, 1.37 of 320 x 16 and of 256 x 16 (four an
+// SM), 1.58 of 512 x 12 (two an SM), 1.27 of 384 x 16; one buffer for keys and values in turn,
+// for a fourth CTA, spills (1.54).
 template <int T, int R>
 struct SweepSmem {
     uint32_t wcnt[T / 32][256];  // per-warp digit counts, then the warp's offsets
@@ -237,7 +241,7 @@ int launch_radix_sort_u32(sde_ctx *ctx, uint32_t **keys, const uint32_t *first_v
         const uint32_t *vin = p == 0 ? first_vals : sv;
         unsigned long long *st = state + per_pass / sizeof(unsigned long long) * p;
         SDE_TRY(small ? (sweep<256, 8>(ctx, sk, vin, dk, dv, n, p, ctl, st, fail))
-                      : (sweep<256, 24>(ctx, sk, vin, dk, dv, n, p, ctl, st, fail)));
+                      : (sweep<384, 16>(ctx, sk, vin, dk, dv, n, p, ctl, st, fail)));
         std::swap(sk, dk);
         std::swap(sv, dv);
     }
