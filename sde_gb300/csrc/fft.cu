@@ -1182,7 +1182,9 @@ struct RowPair {
     static constexpr int H = 1 << LOGH;
     static constexpr int T = H / 16;
     static constexpr size_t SMEM = sizeof(float4) * (size_t)H + 16;
-    static constexpr int MINB = T <= 128 ? 4 : 2;
+    // resident CTAs the registers are kept to.  us, cold: 2048^2 with 4 CTAs 41, 8 (128
+    // registers) 25, 10 (96) 26; 4096^2 with 4 82, 5 (96) 74
+    static constexpr int MINB = T <= 64 ? 512 / T : T == 128 ? 5 : 2;
 };
 
 // c2r first-pass input: FFTR's pre-step of element k for both staged grid rows
@@ -1248,23 +1250,29 @@ __global__ void __launch_bounds__(RowPair<LOGH>::T, RowPair<LOGH>::MINB)
     const int cu = (FNU + 1) / 2 - 1, ioff = (FNU - nx) / 2;
     const float sc = scale_dev ? 1.0f / *scale_dev : 1.0f;
     const float cy0 = cp.ccf ? cp.corry[iy0] : 1.0f, cy1 = cp.ccf && two ? cp.corry[iy0 + 1] : 1.0f;
+    // four pixels a thread of both rows (nx is a multiple of 4, the rows start on 16 bytes):
+    // ix is even and (FNU - nx) / 2 too, so the first one is an element's second half
     float *im0 = image + (int64_t)iy0 * nx;
-    for (int ix = threadIdx.x; ix < nx; ix += T) {
-        int n = ix + ioff - cu;
-        if (n < 0) n += FNU;
-        const float4 z = s[swz4(n >> 1)];
-        float v0 = ((n & 1) ? z.y : z.x) * inv, v1 = ((n & 1) ? z.w : z.z) * inv;
-        if (cp.ccf) {
-            const float cx = cp.corrx[ix];
-            v0 = __fdiv_rn(v0, __fmul_rn(cx, cy0));
-            v1 = __fdiv_rn(v1, __fmul_rn(cx, cy1));
+    for (int ix = 4 * threadIdx.x; ix < nx; ix += 4 * T) {
+        const int m = (ix + ioff - cu + FNU) >> 1;
+        const float4 z0 = s[swz4(m & (H - 1))], z1 = s[swz4((m + 1) & (H - 1))], z2 = s[swz4((m + 2) & (H - 1))];
+        float v[2][4] = {{z0.y, z1.x, z1.y, z2.x}, {z0.w, z1.z, z1.w, z2.z}};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            v[0][q] *= inv;
+            v[1][q] *= inv;
+            if (cp.ccf) {
+                const float cx = cp.corrx[ix + q];
+                v[0][q] = __fdiv_rn(v[0][q], __fmul_rn(cx, cy0));
+                v[1][q] = __fdiv_rn(v[1][q], __fmul_rn(cx, cy1));
+            }
+            if (scale_dev) {
+                v[0][q] = __fadd_rn(__fmul_rn(sc, v[0][q]), 0.0f);
+                v[1][q] = __fadd_rn(__fmul_rn(sc, v[1][q]), 0.0f);
+            }
         }
-        if (scale_dev) {
-            v0 = __fadd_rn(__fmul_rn(sc, v0), 0.0f);
-            v1 = __fadd_rn(__fmul_rn(sc, v1), 0.0f);
-        }
-        im0[ix] = v0;
-        if (two) im0[nx + ix] = v1;
+        *reinterpret_cast<float4 *>(im0 + ix) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+        if (two) *reinterpret_cast<float4 *>(im0 + nx + ix) = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
     }
 }
 
@@ -1279,10 +1287,13 @@ cudaError_t launch_c2r_pair(const FftBatch &bt, int nbatch, int pitch, int nx, i
         bt, pitch, nx, ny, ibegy, tw, cp, status);
     return cudaGetLastError();
 }
-// Whether the row-pair c2r kernel applies: half-lengths 1024..4096, grid rows that start
+// Whether the row-pair c2r kernel applies: half-lengths 512..4096, grid rows that start
 // on 16-byte boundaries (pitch even, 16-byte aligned grids), image rows of whole float4s.
-static bool row_pair_ok(int logh, const FftBatch &bt, int nbatch, int pitch, int nx) {
-    if (logh < 10 || logh > 12) return false;
+// Half-length 512 only in launches that fill the chip: 16 grids of 1024^2 71 -> 54 us against
+// the row kernel, but a single one 14 -> 23 (CTAs of one warp).
+static bool row_pair_ok(int logh, const FftBatch &bt, int nbatch, int pitch, int nx, int ny) {
+    if (logh < 9 || logh > 12) return false;
+    if (logh == 9 && few_ctas((ny + 7) / 8, nbatch)) return false;
     if ((pitch & 1) || (nx & 3)) return false;
     for (int b = 0; b < nbatch; b++)
         if (((uintptr_t)bt.grid[b] & 15u) || ((uintptr_t)bt.image[b] & 15u)) return false;
@@ -1370,8 +1381,9 @@ bool col_fft_t(int logn, const FftBatch &bt, int nbatch, int pitch, int nu, cons
 }
 bool c2r_t(int logh, const FftBatch &bt, int nbatch, int pitch, int nx, int ny, int ibegy,
            const float2 *tw, CorrParams cp, cudaStream_t st, cudaError_t *err, int *status) {
-    if (status && row_pair_ok(logh, bt, nbatch, pitch, nx)) {
-        *err = logh == 10   ? launch_c2r_pair<10>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, status, st)
+    if (status && row_pair_ok(logh, bt, nbatch, pitch, nx, ny)) {
+        *err = logh == 9    ? launch_c2r_pair<9>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, status, st)
+               : logh == 10   ? launch_c2r_pair<10>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, status, st)
                : logh == 11 ? launch_c2r_pair<11>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, status, st)
                             : launch_c2r_pair<12>(bt, nbatch, pitch, nx, ny, ibegy, tw, cp, status, st);
         return true;

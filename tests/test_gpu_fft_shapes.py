@@ -78,3 +78,27 @@ def test_padded_image_must_lie_inside(gpu_ctx):
     im, g = ctx.zeros((8, 8), torch.float32), ctx.zeros((32, 20), torch.complex64)
     for nx, ny, lsx, lsy in ((8, 8, -1, 0), (8, 8, 25, 0), (8, 8, 0, 25), (0, 8, 0, 0)):
         assert lib().sde_grid_from_padded(ctx.h, _ptr(im), nx, ny, lsx, lsy, 32, 32, 32, 32, 0, _ptr(g), 20) == 1
+
+
+# the row-pair kernel: four pixels a thread, image widths that are any multiple of 4 (the first
+# pixel's place in the transform wraps or not), odd row counts, and 512-long half-rows in a batch
+@pytest.mark.parametrize("nx,ny,n", [(4, 3, 2048), (2044, 2047, 2048), (1028, 9, 2048), (4096, 5, 4096), (2052, 33, 4096),
+                                     (8188, 7, 8192), (1020, 1024, 1024)])
+def test_row_pairs(gpu_ctx, orc, nx, ny, n):
+    ctx = gpu_ctx
+    rng = np.random.default_rng(nx + ny)
+    nv, nu = 64 if ny <= 64 else n, n // 2 + 1
+    pitch = (nu + 3) & ~3
+
+    class G:
+        pass
+    g = G()
+    g.pitch, g.nx, g.ny, g.fnu, g.nv = pitch, nx, ny, n, nv
+    X = (rng.standard_normal((nv, nu)) + 1j * rng.standard_normal((nv, nu))).astype(np.complex64)
+    ref, _ = orc.fftr2d(nx, ny, n, nv, -1, xarray=X)
+    Xp = np.zeros((nv, pitch), np.complex64)
+    Xp[:, :nu] = X
+    img = ctx.empty((ny, nx), ctx.torch.float32)
+    scale = ctx.tensor(np.array([4.0], np.float32))
+    ctx.image_from_grid(g, ctx.tensor(Xp), img, correct=False, scale_dev=scale)
+    assert rel_err(img.cpu().numpy(), ref * np.float32(0.25)) < 2e-6
