@@ -588,11 +588,51 @@ struct RowShape {
     static constexpr int MINB = 1024 / T;
 };
 
-// Column pass along v (as k_col_fft), CC columns per CTA read as 16-byte column pairs.
-template <int LOGN, bool INV, bool FEW>
+// GRDH2D's finalize (grd/grdh2d.f:202-226) applied while a column pass reads its input from
+// the raw accumulation: out(u, v) = scale * (R(u+SUPP+1, v) + conj(R(UC-k, 2VC-v)) for the
+// k = 0..SUPP columns next to the axis), 0 for u+1 > NU-SUPP; R is stored at raw index U
+// (RAW_SHIFT) and already holds the folded compensation plane.  nullptr raw: no finalize.
+struct FinParams {
+    const float2 *raw;
+    int raw_pitch, nu, nv, uorigin, vorigin, supp;
+    float scale;
+};
+constexpr int FIN_MAXB = 8;  // grids per finalize-fused column launch (load + store maps)
+struct FinBatch {
+    FinParams f[FIN_MAXB];
+};
+// The same for a k_col_fft_t launch: a grid's parameters per blockIdx.y.
+constexpr int FIN_COLB = 32;
+template <bool FIN>
+struct FinArg {};
+template <>
+struct FinArg<true> {
+    FinParams f[FIN_COLB];
+};
+__device__ __forceinline__ float2 fin_cell(const FinParams &f, float2 r, int u, int v) {
+    const int u1 = u + 1, v1 = v + 1;
+    if (u1 > f.nu - f.supp) return make_float2(0.f, 0.f);
+    const int U = u1 + f.supp, UC = f.uorigin + f.supp, k = U - UC;
+    if (k >= 0 && k <= f.supp) {
+        const int dvv = v1 - f.vorigin, vm = 2 * f.vorigin - v1;
+        if (dvv >= -(f.nv / 2) + 1 && dvv <= f.nv / 2 - 1 && vm >= 1 && vm <= f.nv) {
+            const float2 m = f.raw[(int64_t)(vm - 1) * f.raw_pitch + (UC - k)];
+            r.x = r.x + m.x;
+            r.y = r.y - m.y;
+        }
+    }
+    r.x *= f.scale;
+    r.y *= f.scale;
+    return r;
+}
+
+// Column pass along v (as k_col_fft), CC columns per CTA read as 16-byte column pairs.  FIN: the
+// input is a raw accumulation, finalized on the way in (the raw grid's first column of the pass
+// lies RAW_SHIFT cells in).
+template <int LOGN, bool INV, bool FEW, bool FIN>
 __global__ void __launch_bounds__(ColShape<LOGN, FEW>::T, ColShape<LOGN, FEW>::MINB)
     k_col_fft_t(const __grid_constant__ FftBatch bt, int pitch, int nu, const float2 *__restrict__ tw,
-                int r0, int r1) {
+                int r0, int r1, const __grid_constant__ FinArg<FIN> fa) {
     float2 *grid = bt.grid[blockIdx.y];
     using S = ColShape<LOGN, FEW>;
     constexpr int N = S::N, CC = S::CC, T = S::T;
@@ -609,8 +649,13 @@ __global__ void __launch_bounds__(ColShape<LOGN, FEW>::T, ColShape<LOGN, FEW>::M
         const int v = idx >> LP, jp = idx & ((1 << LP) - 1);
         const int u = u0 + 2 * jp;
         x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if ((TOTAL % T == 0 || idx < TOTAL) && u < nu && (INV || (v >= r0 && v < r1)))
+        if constexpr (FIN) {
+            const FinParams &fp = fa.f[blockIdx.y];
+            if ((TOTAL % T == 0 || idx < TOTAL) && u + 1 <= fp.nu - fp.supp)
+                x[i] = *reinterpret_cast<const float4 *>(&fp.raw[(int64_t)v * pitch + u + RAW_SHIFT]);
+        } else if ((TOTAL % T == 0 || idx < TOTAL) && u < nu && (INV || (v >= r0 && v < r1))) {
             x[i] = *reinterpret_cast<const float4 *>(&grid[(int64_t)v * pitch + u]);
+        }
     }
 #pragma unroll
     for (int i = 0; i < PER; i++) {
@@ -619,6 +664,12 @@ __global__ void __launch_bounds__(ColShape<LOGN, FEW>::T, ColShape<LOGN, FEW>::M
         const int v = idx >> LP, jp = idx & ((1 << LP) - 1);
         int k = v - c;
         if (k < 0) k += N;
+        if constexpr (FIN) {
+            const FinParams &fp = fa.f[blockIdx.y];
+            const float2 c0 = fin_cell(fp, make_float2(x[i].x, x[i].y), u0 + 2 * jp, v);
+            const float2 c1 = fin_cell(fp, make_float2(x[i].z, x[i].w), u0 + 2 * jp + 1, v);
+            x[i] = make_float4(c0.x, c0.y, c1.x, c1.y);
+        }
         s[((2 * jp) << LOGN) + swz(k)] = make_float2(x[i].x, x[i].y);
         s[((2 * jp + 1) << LOGN) + swz(k)] = make_float2(x[i].z, x[i].w);
     }
@@ -867,39 +918,17 @@ __device__ __forceinline__ void twiddle_powers2(float2 *a, float2 *b, const floa
     }
 }
 
-// GRDH2D's finalize (grd/grdh2d.f:202-226) applied while a column pass reads its input from
-// the raw accumulation: out(u, v) = scale * (R(u+SUPP+1, v) + conj(R(UC-k, 2VC-v)) for the
-// k = 0..SUPP columns next to the axis), 0 for u+1 > NU-SUPP; R is stored at raw index U
-// (RAW_SHIFT) and already holds the folded compensation plane.  nullptr raw: no finalize.
-struct FinParams {
-    const float2 *raw;
-    int raw_pitch, nu, nv, uorigin, vorigin, supp;
-    float scale;
-};
-constexpr int FIN_MAXB = 8;  // grids per finalize-fused column launch (load + store maps)
-struct FinBatch {
-    FinParams f[FIN_MAXB];
-};
-__device__ __forceinline__ float2 fin_cell(const FinParams &f, float2 r, int u, int v) {
-    const int u1 = u + 1, v1 = v + 1;
-    if (u1 > f.nu - f.supp) return make_float2(0.f, 0.f);
-    const int U = u1 + f.supp, UC = f.uorigin + f.supp, k = U - UC;
-    if (k >= 0 && k <= f.supp) {
-        const int dvv = v1 - f.vorigin, vm = 2 * f.vorigin - v1;
-        if (dvv >= -(f.nv / 2) + 1 && dvv <= f.nv / 2 - 1 && vm >= 1 && vm <= f.nv) {
-            const float2 m = f.raw[(int64_t)(vm - 1) * f.raw_pitch + (UC - k)];
-            r.x = r.x + m.x;
-            r.y = r.y - m.y;
-        }
-    }
-    r.x *= f.scale;
-    r.y *= f.scale;
-    return r;
+// Element x of a CTA's column pair `pair` in shared memory.  One pair: a float4 a row.  Two: the
+// TMA's rows are 32 bytes, in its 32-byte swizzle (address bit 4 ^= bit 7), which makes eight
+// elements of a pair whose places differ modulo 8 free of bank conflicts.
+template <int PAIRS>
+__device__ __forceinline__ int pair_at(int x, int pair) {
+    return PAIRS == 1 ? x : 2 * x + (pair ^ ((x >> 2) & 1));
 }
 
-template <int LOGN, int LOGR, int LOGNS, bool INV, int T, bool FIRST, bool LAST, bool FIN = false>
+template <int LOGN, int LOGR, int LOGNS, bool INV, int T, int PAIRS, bool FIRST, bool LAST, bool FIN = false>
 __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ tw, int r0, int r1,
-                                         const FinParams *fp = nullptr, int u0 = 0) {
+                                         int tid, int pair, const FinParams *fp = nullptr, int u0 = 0) {
     constexpr int N = 1 << LOGN, R = 1 << LOGR, NB = 1 << (LOGN - LOGR), NS = 1 << LOGNS;
     constexpr int PER = (NB + T - 1) / T;
     constexpr int TSHIFT = LOGN - LOGNS - LOGR;
@@ -907,7 +936,7 @@ __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ t
     float2 a[PER][R], b[PER][R];
 #pragma unroll
     for (int i = 0; i < PER; i++) {
-        const int j = threadIdx.x + i * T;
+        const int j = tid + i * T;
         if (NB % T == 0 || j < NB) {
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -915,7 +944,7 @@ __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ t
                 float4 x;
                 if (FIRST) {
                     const int v = (idx + C) & (N - 1);
-                    x = s[v];
+                    x = s[pair_at<PAIRS>(v, pair)];
                     if (!INV && (v < r0 || v >= r1)) x = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (FIN) {
                         const float2 c0 = fin_cell(*fp, make_float2(x.x, x.y), u0, v);
@@ -923,7 +952,7 @@ __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ t
                         x = make_float4(c0.x, c0.y, c1.x, c1.y);
                     }
                 } else {
-                    x = s[swz4(idx)];
+                    x = s[pair_at<PAIRS>(swz4(idx), pair)];
                 }
                 a[i][r] = make_float2(x.x, x.y);
                 b[i][r] = make_float2(x.z, x.w);
@@ -933,7 +962,7 @@ __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ t
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < PER; i++) {
-        const int j = threadIdx.x + i * T;
+        const int j = tid + i * T;
         if (NB % T == 0 || j < NB) {
             const int jm = j & (NS - 1);
             if (LOGNS > 0 && jm)
@@ -950,9 +979,9 @@ __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ t
                     if (INV) {
                         y.x *= sc; y.y *= sc; y.z *= sc; y.w *= sc;
                     }
-                    s[(p + C) & (N - 1)] = y;
+                    s[pair_at<PAIRS>((p + C) & (N - 1), pair)] = y;
                 } else {
-                    s[swz4(p)] = make_float4(a[i][r].x, a[i][r].y, b[i][r].x, b[i][r].y);
+                    s[pair_at<PAIRS>(swz4(p), pair)] = make_float4(a[i][r].x, a[i][r].y, b[i][r].x, b[i][r].y);
                 }
             }
         }
@@ -960,29 +989,36 @@ __device__ __forceinline__ void st_pass2(float4 *s, const float2 *__restrict__ t
     __syncthreads();
 }
 
-template <int LOGN, int LOGNS, bool INV, int T, bool FIN>
+template <int LOGN, int LOGNS, bool INV, int T, int PAIRS, bool FIN>
 struct St2Passes {
     static __device__ __forceinline__ void run(float4 *s, const float2 *__restrict__ tw, int r0, int r1,
-                                               const FinParams *fp, int u0) {
+                                               int tid, int pair, const FinParams *fp, int u0) {
         constexpr int REM = LOGN - LOGNS;
         constexpr int LOGR = REM >= 4 ? 4 : REM;
-        st_pass2<LOGN, LOGR, LOGNS, INV, T, LOGNS == 0, LOGNS + LOGR == LOGN, FIN && LOGNS == 0>(
-            s, tw, r0, r1, fp, u0);
-        St2Passes<LOGN, LOGNS + LOGR, INV, T, FIN>::run(s, tw, r0, r1, fp, u0);
+        st_pass2<LOGN, LOGR, LOGNS, INV, T, PAIRS, LOGNS == 0, LOGNS + LOGR == LOGN, FIN && LOGNS == 0>(
+            s, tw, r0, r1, tid, pair, fp, u0);
+        St2Passes<LOGN, LOGNS + LOGR, INV, T, PAIRS, FIN>::run(s, tw, r0, r1, tid, pair, fp, u0);
     }
 };
-template <int LOGN, bool INV, int T, bool FIN>
-struct St2Passes<LOGN, LOGN, INV, T, FIN> {
-    static __device__ __forceinline__ void run(float4 *, const float2 *__restrict__, int, int,
+template <int LOGN, bool INV, int T, int PAIRS, bool FIN>
+struct St2Passes<LOGN, LOGN, INV, T, PAIRS, FIN> {
+    static __device__ __forceinline__ void run(float4 *, const float2 *__restrict__, int, int, int, int,
                                                const FinParams *, int) {}
 };
 
 template <int LOGN>
 struct ColTma {
     static constexpr int N = 1 << LOGN;
-    static constexpr int T = N / 16 < 128 ? 128 : N / 16;  // one radix-16 butterfly per thread
-    static constexpr int BOX = N < 256 ? N : 256;          // rows per TMA box
-    static constexpr size_t SMEM = sizeof(float4) * (size_t)N + 16;
+    // Column pairs a CTA: a box row of one pair is 16 bytes, half a sector, and the L2's requests
+    // bound the pass; two pairs of 2048 rows keep the bytes in flight (two CTAs of 64 KB for four
+    // of 32).  12 + 4 grids of 2048^2 171 -> 125 us, one 21 -> 19; at 4096 rows only one CTA of
+    // two pairs fits and nothing overlaps it: 54 -> 60.
+    static constexpr int PAIRS = LOGN == 11 ? 2 : 1;
+    static constexpr int TP = N / 16 < 128 ? 128 : N / 16;    // threads a pair: a radix-16 butterfly each
+    static constexpr int T = PAIRS * TP;
+    static constexpr int BOX = N < 256 ? N : 256;             // rows per TMA box
+    static constexpr size_t BYTES = sizeof(float4) * (size_t)N * PAIRS;
+    static constexpr size_t SMEM = BYTES + 16 + 256;          // + an mbarrier, + the base's alignment
     static constexpr int MINB = 2 * SMEM <= 227 * 1024 ? 2 : 1;  // resident CTAs (shared memory)
 };
 
@@ -1002,15 +1038,16 @@ __global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
     const FinParams &fp = fb.f[FIN ? blockIdx.y : 0];
     const CUtensorMap *tmap = &tb.map[blockIdx.y];
     const CUtensorMap *smap = &tb.map[blockIdx.y + store_off];
-    const int xl = 4 * blockIdx.x + (FIN ? 2 * RAW_SHIFT : 0);  // load box: raw index u0+4
     using S = ColTma<LOGN>;
-    constexpr int N = S::N, BOX = S::BOX;
-    extern __shared__ __align__(128) unsigned char smem_ct[];
+    constexpr int N = S::N, BOX = S::BOX, PAIRS = S::PAIRS;
+    const int xl = 4 * PAIRS * blockIdx.x + (FIN ? 2 * RAW_SHIFT : 0);  // load box: raw index u0+4
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    unsigned char *smem_ct = smem_dyn + (256u - ((uint32_t)__cvta_generic_to_shared(smem_dyn) & 255u)) % 256u;
     float4 *s = reinterpret_cast<float4 *>(smem_ct);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_ct + sizeof(float4) * (size_t)N);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_ct + S::BYTES);
     const uint32_t sb = (uint32_t)__cvta_generic_to_shared(s);
     const uint32_t bb = (uint32_t)__cvta_generic_to_shared(bar);
-    const int x = 4 * blockIdx.x;  // first float of this CTA's two complex columns
+    const int x = 4 * PAIRS * blockIdx.x;  // first float of this CTA's columns
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bb));
         asm volatile("fence.mbarrier_init.release.cluster;");
@@ -1021,11 +1058,11 @@ __global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
         // boxes without a row of [r0, r1) are not loaded: the first pass reads those rows as zero
         const int b0 = r0 / BOX, b1 = (r1 + BOX - 1) / BOX;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bb),
-                     "r"((uint32_t)(sizeof(float4) * BOX * (b1 - b0))));
+                     "r"((uint32_t)(sizeof(float4) * PAIRS * BOX * (b1 - b0))));
         for (int b = b0; b < b1; b++)
             asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                " [%0], [%1, {%2, %3}], [%4];" ::"r"(sb + (uint32_t)(b * BOX * sizeof(float4))),
+                " [%0], [%1, {%2, %3}], [%4];" ::"r"(sb + (uint32_t)(b * BOX * PAIRS * sizeof(float4))),
                 "l"(reinterpret_cast<uint64_t>(tmap)), "r"(xl), "r"(b * BOX), "r"(bb)
                 : "memory");
     }
@@ -1044,7 +1081,8 @@ __global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
             return;
         }
     }
-    St2Passes<LOGN, 0, INV, S::T, FIN>::run(s, tw, r0, r1, &fp, 2 * blockIdx.x);
+    const int pair = PAIRS == 1 ? 0 : (int)threadIdx.x / S::TP, tid = PAIRS == 1 ? (int)threadIdx.x : (int)threadIdx.x % S::TP;
+    St2Passes<LOGN, 0, INV, S::TP, PAIRS, FIN>::run(s, tw, r0, r1, tid, pair, &fp, 2 * (PAIRS * blockIdx.x + pair));
     // the last pass's generic stores must be visible to the bulk copies that read them
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -1052,18 +1090,20 @@ __global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
         for (int b = 0; b < N / BOX; b++)
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
                              reinterpret_cast<uint64_t>(smap)),
-                         "r"(x), "r"(b * BOX), "r"(sb + (uint32_t)(b * BOX * sizeof(float4)))
+                         "r"(x), "r"(b * BOX), "r"(sb + (uint32_t)(b * BOX * PAIRS * sizeof(float4)))
                          : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
 }
 
+uint32_t col_tma_pairs(int logn) { return logn == 11 ? ColTma<11>::PAIRS : logn == 12 ? ColTma<12>::PAIRS : ColTma<13>::PAIRS; }
+
 template <int LOGN>
 cudaError_t launch_col_tma(const TmaBatch &map, int nbatch, int nu, const float2 *tw, bool inverse,
                            int r0, int r1, int *status, cudaStream_t st, const FinBatch *fin = nullptr) {
     using S = ColTma<LOGN>;
-    const dim3 nb((unsigned)((nu + 1) / 2), (unsigned)nbatch);
+    const dim3 nb((unsigned)((nu + 2 * S::PAIRS - 1) / (2 * S::PAIRS)), (unsigned)nbatch);
     cudaError_t e;
     if (fin) {
         e = cudaFuncSetAttribute(k_col_fft_tma<LOGN, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1094,9 +1134,10 @@ bool col_fft_tma(sde_ctx *ctx, int logn, float2 *const *grids, int n, int pitch,
     for (int b0 = 0; b0 < n && *rc == SDE_OK && *err == cudaSuccess; b0 += TMA_MAXB) {
         const int nb = n - b0 < TMA_MAXB ? n - b0 : TMA_MAXB;
         TmaBatch tb;
+        const uint32_t pairs = col_tma_pairs(logn);
         for (int i = 0; i < nb && *rc == SDE_OK; i++)
             *rc = encode_tmap_f32_2d(&tb.map[i], grids[b0 + i], (uint64_t)nu * 2, (uint64_t)nv,
-                                     (uint64_t)pitch * 8, 4, (uint32_t)(nv < 256 ? nv : 256));
+                                     (uint64_t)pitch * 8, 4 * pairs, (uint32_t)(nv < 256 ? nv : 256), pairs == 2);
         if (*rc != SDE_OK) break;
         switch (logn) {
             case 11: *err = launch_col_tma<11>(tb, nb, nu, tw, inverse, r0, r1, ctx->d_status, ctx->stream); break;
@@ -1301,27 +1342,47 @@ static bool row_pair_ok(int logh, const FftBatch &bt, int nbatch, int pitch, int
 }
 
 // Launchers for the compile-time shapes: false if the size has no instance.
-template <int LOGN, bool INV, bool FEW>
+template <int LOGN, bool INV, bool FEW, bool FIN>
 cudaError_t launch_col_shape(const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw, int r0,
-                             int r1, cudaStream_t st) {
+                             int r1, cudaStream_t st, const FinArg<FIN> &fa) {
     using S = ColShape<LOGN, FEW>;
-    cudaError_t e = cudaFuncSetAttribute(k_col_fft_t<LOGN, INV, FEW>,
+    cudaError_t e = cudaFuncSetAttribute(k_col_fft_t<LOGN, INV, FEW, FIN>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
     if (e != cudaSuccess) return e;
-    k_col_fft_t<LOGN, INV, FEW><<<dim3((unsigned)((nu + S::CC - 1) / S::CC), (unsigned)nbatch), S::T,
-                                  S::SMEM, st>>>(bt, pitch, nu, tw, r0, r1);
+    k_col_fft_t<LOGN, INV, FEW, FIN><<<dim3((unsigned)((nu + S::CC - 1) / S::CC), (unsigned)nbatch), S::T,
+                                       S::SMEM, st>>>(bt, pitch, nu, tw, r0, r1, fa);
     return cudaGetLastError();
 }
 template <int LOGN>
 cudaError_t launch_col_t(const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw,
                          bool inverse, int r0, int r1, cudaStream_t st) {
     const int cc = ColShape<LOGN, false>::CC;
+    const FinArg<false> no;
     if constexpr (LOGN < 12)
         if (few_ctas((nu + cc - 1) / cc, nbatch))
-            return inverse ? launch_col_shape<LOGN, true, true>(bt, nbatch, pitch, nu, tw, r0, r1, st)
-                           : launch_col_shape<LOGN, false, true>(bt, nbatch, pitch, nu, tw, r0, r1, st);
-    return inverse ? launch_col_shape<LOGN, true, false>(bt, nbatch, pitch, nu, tw, r0, r1, st)
-                   : launch_col_shape<LOGN, false, false>(bt, nbatch, pitch, nu, tw, r0, r1, st);
+            return inverse ? launch_col_shape<LOGN, true, true>(bt, nbatch, pitch, nu, tw, r0, r1, st, no)
+                           : launch_col_shape<LOGN, false, true>(bt, nbatch, pitch, nu, tw, r0, r1, st, no);
+    return inverse ? launch_col_shape<LOGN, true, false>(bt, nbatch, pitch, nu, tw, r0, r1, st, no)
+                   : launch_col_shape<LOGN, false, false>(bt, nbatch, pitch, nu, tw, r0, r1, st, no);
+}
+// inverse, from raw accumulations: at most FIN_COLB grids of 32 to 1024 rows
+template <int LOGN>
+cudaError_t launch_col_fin(const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw, cudaStream_t st,
+                           const FinArg<true> &fa) {
+    const int cc = ColShape<LOGN, false>::CC;
+    if (few_ctas((nu + cc - 1) / cc, nbatch))
+        return launch_col_shape<LOGN, true, true>(bt, nbatch, pitch, nu, tw, 0, 1 << LOGN, st, fa);
+    return launch_col_shape<LOGN, true, false>(bt, nbatch, pitch, nu, tw, 0, 1 << LOGN, st, fa);
+}
+cudaError_t col_fft_fin(int logn, const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw, cudaStream_t st,
+                        const FinArg<true> &fa) {
+    switch (logn) {
+#define CASE(L) \
+    case L: return launch_col_fin<L>(bt, nbatch, pitch, nu, tw, st, fa);
+        CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10)
+#undef CASE
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 template <int LOGH, bool FEW>
@@ -1460,14 +1521,16 @@ int fft_images_from_grids(sde_ctx *ctx, int n, float2 *const *grids, float *cons
 }
 
 bool fin_fused_shape(int nu, int nv) {
-    const int logn = ilog2(nv);
-    return logn >= 11 && logn <= 13 && (1 << logn) == nv && nu >= 2;
+    const int logn = ilog2(nv), logh = nu >= 2 ? ilog2(nu - 1) : 0;
+    return logn >= 5 && logn <= 13 && (1 << logn) == nv && logh >= 5 && logh <= 13 && (1 << logh) == nu - 1;
 }
 
 // Images of n same-shape gridding passes straight from their raw accumulations (compensation
-// planes already folded: every fd[i].raw_lo is NULL): finalize-fused TMA column passes,
-// FIN_MAXB grids per launch (fd[i].out receives the finalized, column-transformed grid), then
-// the batched row c2r pass.  Shapes without a fused column pass: EINVAL.
+// planes already folded: every fd[i].raw_lo is NULL): finalize-fused column passes, FIN_COLB or
+// (TMA) FIN_MAXB grids per launch (fd[i].out receives the finalized, column-transformed grid),
+// then the batched row c2r pass.  Shapes without a fused column pass: EINVAL.  A pass over the
+// grids for the finalize alone took 42 us of a mosaic with 37 grids of 256^2 to 1024^2, whose
+// column passes take 68 us with it and 62 without; 3.4 us of a 512^2 image.
 int fft_images_from_raw(sde_ctx *ctx, int n, const FinalizeDesc *fd, float *const *images,
                         const float *const *scales, int nx, int ny, int correct) {
     if (!ctx || n < 0) return SDE_EINVAL;
@@ -1484,18 +1547,32 @@ int fft_images_from_raw(sde_ctx *ctx, int n, const FinalizeDesc *fd, float *cons
     CorrParams cp = {nullptr, nullptr, nullptr};
     if (correct) SDE_TRY(corr_params(ctx, nx, ny, &cp));
     const int ibegy = (nv + 1) / 2 - (ny + 1) / 2;
-    {
+    if (logn < 11) {
+        KTimer kt(ctx, "col_fft_fin_batch");
+        for (int b0 = 0; b0 < n; b0 += FIN_COLB) {
+            const int nb = n - b0 < FIN_COLB ? n - b0 : FIN_COLB;
+            FftBatch bt{};
+            FinArg<true> fa{};
+            for (int i = 0; i < nb; i++) {
+                const FinalizeDesc &f = fd[b0 + i];
+                bt.grid[i] = f.out;
+                fa.f[i] = FinParams{f.raw, pitch, nu, nv, f.uorigin, f.vorigin, f.supp, f.scale};
+            }
+            SDE_CUDA_TRY(col_fft_fin(logn, bt, nb, pitch, nu, twv, ctx->stream, fa));
+        }
+    } else {
         KTimer kt(ctx, "col_fft_fin_batch");
         for (int b0 = 0; b0 < n; b0 += FIN_MAXB) {
             const int nb = n - b0 < FIN_MAXB ? n - b0 : FIN_MAXB;
             TmaBatch tb;
+            const uint32_t pairs = col_tma_pairs(logn);
             FinBatch fb{};
             for (int i = 0; i < nb; i++) {
                 const FinalizeDesc &f = fd[b0 + i];
                 SDE_TRY(encode_tmap_f32_2d(&tb.map[i], f.raw, (uint64_t)pitch * 2, (uint64_t)nv,
-                                           (uint64_t)pitch * 8, 4, 256));
+                                           (uint64_t)pitch * 8, 4 * pairs, 256, pairs == 2));
                 SDE_TRY(encode_tmap_f32_2d(&tb.map[nb + i], f.out, (uint64_t)nu * 2, (uint64_t)nv,
-                                           (uint64_t)pitch * 8, 4, 256));
+                                           (uint64_t)pitch * 8, 4 * pairs, 256, pairs == 2));
                 fb.f[i] = FinParams{f.raw, pitch, nu, nv, f.uorigin, f.vorigin, f.supp, f.scale};
             }
             cudaError_t e;
@@ -1584,16 +1661,15 @@ int sde_image_from_grid(sde_ctx *ctx, float *grid, int pitch, int nx, int ny, in
     return c2r_pass(ctx, grid, pitch, nx, ny, fnu, nv, correct, scale_dev, image, twu);
 }
 
-// The dirty image (or PSF) of a plan pass straight from the raw accumulation: where the
-// column pass is TMA-fed (2048..8192 rows) it applies GRDH2D's finalize to its input and
-// writes the column-transformed grid to grid; otherwise finalize into grid, then the column
-// pass.  Then the row c2r pass.
+// The dirty image (or PSF) of a plan pass straight from the raw accumulation: the column pass
+// applies GRDH2D's finalize to its input and writes the column-transformed grid to grid (lengths
+// without a compiled pass: finalize into grid, then the column pass).  Then the row c2r pass.
 int image_from_raw(sde_ctx *ctx, const float2 *raw, const float2 *raw_lo, int nu, int nv,
                    int uorigin, int vorigin, int supp, float scale, float *grid, int pitch, int nx,
                    int ny, int fnu, int correct, const float *scale_dev, float *image) {
     SDE_TRY(check_fft_args(nx, ny, fnu, nv, pitch));
     const int logn = ilog2(nv);
-    if (raw_lo || logn < 11 || logn > 13 || nu != fnu / 2 + 1) {
+    if (raw_lo || !fin_fused_shape(nu, nv) || nu != fnu / 2 + 1) {
         SDE_TRY(grid_finalize_scale(ctx, raw, raw_lo, (float2 *)grid, nu, nv, pitch, uorigin, vorigin,
                                     supp, scale));
         return sde_image_from_grid(ctx, grid, pitch, nx, ny, fnu, nv, correct, scale_dev, image);
@@ -1601,13 +1677,21 @@ int image_from_raw(sde_ctx *ctx, const float2 *raw, const float2 *raw_lo, int nu
     const float2 *twv, *twu;
     SDE_TRY(ctx_twiddles(ctx, nv, &twv));
     SDE_TRY(ctx_twiddles(ctx, fnu, &twu));
-    {
+    if (logn < 11) {
+        KTimer kt(ctx, "col_fft_fin");
+        FftBatch bt{};
+        FinArg<true> fa{};
+        bt.grid[0] = reinterpret_cast<float2 *>(grid);
+        fa.f[0] = FinParams{raw, pitch, nu, nv, uorigin, vorigin, supp, scale};
+        SDE_CUDA_TRY(col_fft_fin(logn, bt, 1, pitch, nu, twv, ctx->stream, fa));
+    } else {
         KTimer kt(ctx, "col_fft_fin");
         TmaBatch tb;
-        SDE_TRY(encode_tmap_f32_2d(&tb.map[0], raw, (uint64_t)pitch * 2, (uint64_t)nv, (uint64_t)pitch * 8, 4,
-                                   256));
-        SDE_TRY(encode_tmap_f32_2d(&tb.map[1], grid, (uint64_t)nu * 2, (uint64_t)nv, (uint64_t)pitch * 8, 4,
-                                   256));
+        const uint32_t pairs = col_tma_pairs(logn);
+        SDE_TRY(encode_tmap_f32_2d(&tb.map[0], raw, (uint64_t)pitch * 2, (uint64_t)nv, (uint64_t)pitch * 8,
+                                   4 * pairs, 256, pairs == 2));
+        SDE_TRY(encode_tmap_f32_2d(&tb.map[1], grid, (uint64_t)nu * 2, (uint64_t)nv, (uint64_t)pitch * 8,
+                                   4 * pairs, 256, pairs == 2));
         FinBatch fb{};
         fb.f[0] = FinParams{raw, pitch, nu, nv, uorigin, vorigin, supp, scale};
         cudaError_t e;

@@ -919,7 +919,7 @@ size_t degrid_smem() { return DG_BAR_OFF + 8 * TEAMS; }
 // A 2-D FP32 tensor map (width floats x rows, row pitch in bytes, box box_w x box_h) for
 // cp.async.bulk.tensor; out-of-range elements read as zero and are not written.
 int encode_tmap_f32_2d(CUtensorMap *map, const void *base, uint64_t width, uint64_t rows,
-                       uint64_t row_bytes, uint32_t box_w, uint32_t box_h) {
+                       uint64_t row_bytes, uint32_t box_w, uint32_t box_h, bool swizzle32) {
     typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                       const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                       const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -945,7 +945,8 @@ int encode_tmap_f32_2d(CUtensorMap *map, const void *base, uint64_t width, uint6
     cuuint32_t box[2] = {box_w, box_h};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims, strides,
-                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         sde_set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
