@@ -469,49 +469,53 @@ __device__ __forceinline__ float2 finalize_cell(const float2 *__restrict__ raw,
 // The compensation plane folded into the raw grid over one marked core (see k_core_lo):
 // raw = raw + lo where lo != 0 (the add finalize would do), lo = 0.  A core row is 32 pairs
 // of cells starting at an even raw index (16-byte aligned: the pitch is a multiple of 4);
-// each thread loads 8 pairs before touching any.
-__device__ __forceinline__ void fold_core(float2 *raw, float2 *raw_lo, int cu, int cv, int nv, int pitch) {
-    const int r0 = cv * TILE - SUPP, i0 = cu * TILE - (SUPP - 1);
+// A block folds a quarter of a core, and reads raw and lo together: in small grids, where a core
+// or two is all there is, the pass is the latency of its loads (512^2: 3.6 us, 7.7 with whole
+// cores and raw read after lo).
+constexpr int FOLD_Q = 4;
+__device__ __forceinline__ void fold_core(float2 *raw, float2 *raw_lo, int cu, int cv, int quarter, int nv, int pitch) {
+    const int r0 = cv * TILE - SUPP + quarter * (TILE / FOLD_Q), i0 = cu * TILE - (SUPP - 1);
     float4 *raw4 = reinterpret_cast<float4 *>(raw);
     float4 *lo4 = reinterpret_cast<float4 *>(raw_lo);
-    constexpr int PAIRS = TILE * TILE / 2 / 256;  // 8
-    float4 e[PAIRS];
+    constexpr int PAIRS = TILE * TILE / 2 / 256 / FOLD_Q;  // 2
+    float4 e[PAIRS], h[PAIRS];
     int64_t q[PAIRS];
 #pragma unroll
     for (int j = 0; j < PAIRS; j++) {
         const int k = threadIdx.x + j * 256;
         const int r = r0 + (k >> 5), i = i0 + 2 * (k & 31);
         q[j] = -1;
-        e[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        e[j] = h[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < 0 || r >= nv || i < 0 || i >= pitch) continue;
         q[j] = ((int64_t)r * pitch + i) >> 1;
         e[j] = lo4[q[j]];
+        h[j] = raw4[q[j]];
     }
 #pragma unroll
     for (int j = 0; j < PAIRS; j++) {
         if (q[j] < 0 || (e[j].x == 0.f && e[j].y == 0.f && e[j].z == 0.f && e[j].w == 0.f)) continue;
-        float4 h = raw4[q[j]];
-        h.x = h.x + e[j].x;
-        h.y = h.y + e[j].y;
-        h.z = h.z + e[j].z;
-        h.w = h.w + e[j].w;
-        raw4[q[j]] = h;
+        h[j].x = h[j].x + e[j].x;
+        h[j].y = h[j].y + e[j].y;
+        h[j].z = h[j].z + e[j].z;
+        h[j].w = h[j].w + e[j].w;
+        raw4[q[j]] = h[j];
         lo4[q[j]] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
 __global__ void __launch_bounds__(256) k_fold_lo(float2 *raw, float2 *raw_lo, const uint8_t *__restrict__ core,
                                                  int ncu, int nv, int pitch) {
-    if (!core[blockIdx.x]) return;
-    fold_core(raw, raw_lo, blockIdx.x % ncu, blockIdx.x / ncu, nv, pitch);
+    const int c = blockIdx.x / FOLD_Q;
+    if (!core[c]) return;
+    fold_core(raw, raw_lo, c % ncu, c / ncu, blockIdx.x % FOLD_Q, nv, pitch);
 }
 
 // the marked cores of many grids, one block per (grid, core) pair of the list
 __global__ void __launch_bounds__(256) k_fold_lo_batch(const BatchPlan *__restrict__ d,
                                                        const int2 *__restrict__ cores) {
-    const int2 c = cores[blockIdx.x];
+    const int2 c = cores[blockIdx.x / FOLD_Q];
     const BatchPlan &p = d[c.x];
-    fold_core(p.raw, p.raw_lo, c.y & 0xFFFF, c.y >> 16, p.nv, p.pitch);
+    fold_core(p.raw, p.raw_lo, c.y & 0xFFFF, c.y >> 16, blockIdx.x % FOLD_Q, p.nv, p.pitch);
 }
 
 __global__ void k_finalize(const float2 *__restrict__ raw, const float2 *__restrict__ raw_lo,
@@ -1058,7 +1062,7 @@ int launch_finalize_batch(sde_ctx *ctx, const FinalizeDesc *d_desc, const uint16
 int launch_fold_lo_batch(sde_ctx *ctx, const BatchPlan *d_plans, const int2 *cores, int64_t ncores) {
     if (ncores <= 0) return SDE_OK;
     KTimer kt(ctx, "fold_lo_batch");
-    k_fold_lo_batch<<<(unsigned)ncores, 256, 0, ctx->stream>>>(d_plans, cores);
+    k_fold_lo_batch<<<(unsigned)(ncores * FOLD_Q), 256, 0, ctx->stream>>>(d_plans, cores);
     SDE_CHECK_LAUNCH();
     return SDE_OK;
 }
@@ -1123,7 +1127,7 @@ int plan_fold_lo(sde_plan *pl, float2 *raw, float2 *raw_lo) {
     sde_ctx *ctx = pl->ctx;
     KTimer kt(ctx, "fold_lo");
     const int ncu = pl->ntu + 1, ncv = pl->ntv + 1;
-    k_fold_lo<<<ncu * ncv, 256, 0, ctx->stream>>>(raw, raw_lo, pl->core_lo, ncu, pl->spec.nv, pl->pitch);
+    k_fold_lo<<<ncu * ncv * FOLD_Q, 256, 0, ctx->stream>>>(raw, raw_lo, pl->core_lo, ncu, pl->spec.nv, pl->pitch);
     SDE_CHECK_LAUNCH();
     return SDE_OK;
 }
