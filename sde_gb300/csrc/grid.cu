@@ -61,7 +61,12 @@ constexpr int UT_ROW = 32;                         // floats per u-table row (4 
 static_assert(UT_ROW * 4 == TAPROW_BYTES, "the plan record's u-table offsets");
 constexpr int UT_FLOATS = 2 * 129 * UT_ROW;
 constexpr int GTAB_FLOATS = VT_FLOATS + UT_FLOATS;
-constexpr int GTILE_FLOATS = 2 * STILE * STILE;    // a team's tile: re and im planes
+// Row stride of the tiles in shared memory.  The windows of one colour are 8 n columns and 7 m
+// rows apart; 7 * 76 = 4 mod 8, so windows that differ in n mod 4 or in m mod 2 lie in different
+// banks, and the chunk order puts such windows next to each other (plan.cu).
+constexpr int TROW = 76;
+constexpr int GPLANE = STILE * TROW;
+constexpr int GTILE_FLOATS = 2 * GPLANE;           // a team's tile: re and im planes
 constexpr int NPAIR = (NTAP + 1) / 2;              // window rows taken in pairs
 
 // cft_g[d * 8 + a] = tap a (0..6) of offset row d; cft_g[d * 8 + 7] = 0
@@ -186,8 +191,8 @@ __device__ __forceinline__ void grid_item(const WorkItem &it, const uint2 *__res
         if (!live) continue;
 #pragma unroll
         for (int b = 0; b < NTAP; b++) {
-            float *rr_ = &tre[(lv + b) * STILE + lu + q];
-            float *ri = &tim[(lv + b) * STILE + lu + q];
+            float *rr_ = &tre[(lv + b) * TROW + lu + q];
+            float *ri = &tim[(lv + b) * TROW + lu + q];
             const int p = b >> 1;
             atomicAdd(rr_, (b & 1) ? A0r[p].y : A0r[p].x);
             if (!PSF) atomicAdd(ri, (b & 1) ? A0i[p].y : A0i[p].x);
@@ -209,11 +214,11 @@ __device__ __forceinline__ void grid_item(const WorkItem &it, const uint2 *__res
             gi[j] = -1;
             val[j] = make_float2(0.f, 0.f);
             if (k >= STILE * STILE) continue;
-            val[j] = make_float2(tre[k], tim[k]);
+            const int r = k / STILE, cc = k - r * STILE, at = r * TROW + cc;
+            val[j] = make_float2(tre[at], tim[at]);
             if (val[j].x == 0.f && val[j].y == 0.f) continue;
-            tre[k] = 0.f;
-            tim[k] = 0.f;
-            const int r = k / STILE, cc = k - r * STILE;
+            tre[at] = 0.f;
+            tim[at] = 0.f;
             // GRDH2D's 0-based raw cell; stored at raw index gu0 + 1 (RAW_SHIFT = SUPP + 1)
             const int gv0 = tv * TILE + r - SUPP, gu0 = tu * TILE + cc - SUPP;
             if (gv0 < 0 || gv0 >= nv || gu0 < 0 || gu0 >= nu) continue;
@@ -253,10 +258,10 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
     float *ut = vt + VT_FLOATS;
     const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x % TEAM_THREADS;
     float *tre = ut + UT_FLOATS + team * GTILE_FLOATS;
-    float *tim = tre + STILE * STILE;
+    float *tim = tre + GPLANE;
     // the team's item, read from here where it is used: the accumulators leave no registers
     __shared__ WorkItem s_item[TEAMS];
-    for (int k = tid; k < STILE * STILE; k += TEAM_THREADS) {
+    for (int k = tid; k < GPLANE; k += TEAM_THREADS) {
         tre[k] = 0.f;
         tim[k] = 0.f;
     }
@@ -296,10 +301,10 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
     float *ut = vt + VT_FLOATS;
     const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x % TEAM_THREADS;
     float *tre = ut + UT_FLOATS + team * GTILE_FLOATS;
-    float *tim = tre + STILE * STILE;
+    float *tim = tre + GPLANE;
     __shared__ WorkItem s_item[TEAMS];  // the team's item and its plan, as in k_grid
     __shared__ BatchPlan s_plan[TEAMS];
-    for (int k = tid; k < STILE * STILE; k += TEAM_THREADS) {
+    for (int k = tid; k < GPLANE; k += TEAM_THREADS) {
         tre[k] = 0.f;
         tim[k] = 0.f;
     }

@@ -5,7 +5,7 @@
 // grd/grddeh2d.f:92-118), with the reference's results: its exact operations, or FP32
 // arithmetic whose error bound decides the same roundings (geom.cuh).  Visibilities are
 // then sorted by (uv tile, cell), split into same-cell chunks of <= CHUNK_MAX, and the
-// chunks of each work item are ordered by (7x7 colour class, chunk index, cell) so that
+// chunks of each work item are ordered by (length, 7x7 colour class, chunk index, place) so that
 // the 32 chunks a warp flushes at once never overlap; the plan stores the visibilities in
 // that chunk order, so a team's concurrent chunks read one contiguous range.  The observed
 // visibilities are stored already rotated/conjugated into the gridding frame (FVIS of
@@ -338,8 +338,8 @@ __device__ __forceinline__ void run_pieces(int64_t rs, int64_t re, int64_t ts, i
 // The runs' chunks and the items that start in them, numbered by a scan of both counts (31
 // bits each).  A chunk's entry: where its visibilities are in the sort's order, its even cell
 // and length, and its sort key within the item, in bits from the top: a coarse length bin
-// (LENBIN_BITS, longest first), the colour class, the length class, the chunk index and (16
-// bits) its number in the item.  The 8 chunks that a warp of the gridder or degridder takes
+// (LENBIN_BITS, longest first), the colour class, the length class, the chunk index, the window's
+// place among its colour's and (16 bits) its number in the item.  The 8 chunks that a warp of the gridder or degridder takes
 // together then have similar lengths (the warp runs to its longest) and mostly one colour.  On
 // the large single field the lanes do useful work in 94% of the warps' visibility slots with 8
 // bins, 81% with the colour class alone above the length (a simulation of both orders on its
@@ -365,12 +365,17 @@ __global__ void __launch_bounds__(SC_T) k_run_emit(const uint32_t *__restrict__ 
     auto piece_chunks = [&](uint32_t cell, int64_t c, int64_t a, int64_t b, int first, int step) {
         const uint32_t lu = cell & 63u, lv = cell >> 6;
         const uint64_t color = ((lu >> 1) & 3u) * 7u + (lv % 7u);
+        // the windows of a colour, so that neighbours differ in banks (TROW, grid.cu): four in a
+        // row cover n mod 2 and m mod 2, eight n mod 4 as well (64.7 million visibilities, gridding:
+        // 704 -> 689 us with the row stride; 10 million on 2048^2 197 -> 191)
+        const uint32_t n = lu >> 3, m = lv / 7u;
+        const uint64_t place = (m >> 1) << 4 | (n >> 2) << 3 | (n >> 1 & 1u) << 2 | (m & 1u) << 1 | (n & 1u);
         const int nc = (int)((b - a + chunk_max - 1) / chunk_max);
         for (int j = first; j < nc; j += step) {
             const int64_t q = a + (int64_t)j * chunk_max;
             const int len = (int)min((int64_t)chunk_max, b - q), cls = chunk_max - len;
             const int bin = min(cls * (1 << LENBIN_BITS) / chunk_max, (1 << LENBIN_BITS) - 1);
-            ckey[c + j] = ((((((uint64_t)bin << 6) | color) << lbits) | (uint64_t)cls) << jbits) | (uint64_t)j;
+            ckey[c + j] = (((((((uint64_t)bin << 6) | color) << lbits) | (uint64_t)cls) << jbits) | (uint64_t)j) << 7 | place;
             craw[c + j] = make_uint2((uint32_t)q, cell | ((uint32_t)len << 16));
         }
         return nc;
