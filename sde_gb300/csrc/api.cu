@@ -200,7 +200,7 @@ extern "C" int sde_ctx_create(sde_ctx **out, int device) {
         sde_ctx_destroy(c);
         return SDE_ENOMEM;
     }
-    if ((rc = clean_preload(c)) != SDE_OK) {
+    if ((rc = clean_preload(c)) != SDE_OK || (rc = fft_preload()) != SDE_OK) {
         sde_ctx_destroy(c);
         return rc;
     }

@@ -314,6 +314,7 @@ struct FftBatch {
     float *image[FFT_MAXB];
     const float *scale[FFT_MAXB];
 };
+int fft_preload();
 int clean_preload(sde_ctx *ctx);  // loads the CLEAN kernels, caches their occupancy
 size_t grid_smem_bytes();
 int grid_ctas_per_sm();  // resident persistent gridding CTAs per SM

@@ -1358,10 +1358,9 @@ cudaError_t launch_col_t(const FftBatch &bt, int nbatch, int pitch, int nu, cons
                          bool inverse, int r0, int r1, cudaStream_t st) {
     const int cc = ColShape<LOGN, false>::CC;
     const FinArg<false> no;
-    if constexpr (LOGN < 12)
-        if (few_ctas((nu + cc - 1) / cc, nbatch))
-            return inverse ? launch_col_shape<LOGN, true, true>(bt, nbatch, pitch, nu, tw, r0, r1, st, no)
-                           : launch_col_shape<LOGN, false, true>(bt, nbatch, pitch, nu, tw, r0, r1, st, no);
+    if (few_ctas((nu + cc - 1) / cc, nbatch))
+        return inverse ? launch_col_shape<LOGN, true, true>(bt, nbatch, pitch, nu, tw, r0, r1, st, no)
+                       : launch_col_shape<LOGN, false, true>(bt, nbatch, pitch, nu, tw, r0, r1, st, no);
     return inverse ? launch_col_shape<LOGN, true, false>(bt, nbatch, pitch, nu, tw, r0, r1, st, no)
                    : launch_col_shape<LOGN, false, false>(bt, nbatch, pitch, nu, tw, r0, r1, st, no);
 }
@@ -1429,13 +1428,14 @@ cudaError_t launch_r2c_t(const FftBatch &bt, int nbatch, int nx, int ny, int iof
 
 #define SDE_LOG_CASES(X) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13)
 
-// Column pass through the compile-time kernels when 2^logn has an instance.
+// Column pass through the compile-time kernels when 2^logn has an instance (32..1024 rows; longer
+// columns are the TMA-fed kernel's).
 bool col_fft_t(int logn, const FftBatch &bt, int nbatch, int pitch, int nu, const float2 *tw,
                bool inverse, int r0, int r1, cudaStream_t st, cudaError_t *err) {
     switch (logn) {
 #define CASE(L) \
     case L: *err = launch_col_t<L>(bt, nbatch, pitch, nu, tw, inverse, r0, r1, st); return true;
-        SDE_LOG_CASES(CASE)
+        CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10)
 #undef CASE
         default: return false;
     }
@@ -1517,6 +1517,14 @@ int fft_images_from_grids(sde_ctx *ctx, int n, float2 *const *grids, float *cons
         }
         SDE_CUDA_TRY(e);
     }
+    return SDE_OK;
+}
+
+// Loads this file's kernels when the context is created: with lazy loading the module would come
+// with the first transform of a process (12 ms measured).
+int fft_preload() {
+    cudaFuncAttributes a;
+    SDE_CUDA_TRY(cudaFuncGetAttributes(&a, k_row_c2r));
     return SDE_OK;
 }
 
