@@ -483,13 +483,18 @@ int fail(const char *m) {
 int clark_resid(sde_ctx *ctx, const float *comp, const float *drt, const float2 *xfr, float2 *mvis, int pitch,
                 float *res, int w, int n) {
     const int nu = n / 2 + 1;
-    SDE_TRY(sde_grid_from_image(ctx, comp, w, w, n, n, 0, (float *)mvis, pitch));
-    {
-        KTimer kt(ctx, "clark_cmul");
-        k_clark_cmul<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(mvis, xfr, nu, n, pitch);
-        SDE_CHECK_LAUNCH();
+    int rc = SDE_OK;
+    if (convolve_images(ctx, comp, xfr, mvis, pitch, w, n, res, &rc)) {
+        SDE_TRY(rc);
+    } else {
+        SDE_TRY(sde_grid_from_image(ctx, comp, w, w, n, n, 0, (float *)mvis, pitch));
+        {
+            KTimer kt(ctx, "clark_cmul");
+            k_clark_cmul<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(mvis, xfr, nu, n, pitch);
+            SDE_CHECK_LAUNCH();
+        }
+        SDE_TRY(sde_image_from_grid(ctx, (float *)mvis, pitch, w, w, n, n, 0, nullptr, res));
     }
-    SDE_TRY(sde_image_from_grid(ctx, (float *)mvis, pitch, w, w, n, n, 0, nullptr, res));
     KTimer kt(ctx, "clark_sub");
     k_clark_sub<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(drt, res, (int64_t)w * w);
     SDE_CHECK_LAUNCH();

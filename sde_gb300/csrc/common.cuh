@@ -314,6 +314,9 @@ struct FftBatch {
     float *image[FFT_MAXB];
     const float *scale[FFT_MAXB];
 };
+// FFTR2D, the product with a transfer function and FFTR2D back (fft.cu; false: n has no such pass)
+bool convolve_images(sde_ctx *ctx, const float *image, const float2 *xfr, float2 *mvis, int pitch, int w, int n,
+                     float *image_out, int *rc);
 int fft_preload();
 int clean_preload(sde_ctx *ctx);  // loads the CLEAN kernels, caches their occupancy
 size_t grid_smem_bytes();

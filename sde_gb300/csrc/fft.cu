@@ -1097,6 +1097,96 @@ __global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
     }
 }
 
+// A column's forward transform, its product with the transfer function's column (PIXXMULT,
+// pix/pixxmult.f: the complex product in REAL) and the inverse transform, in shared memory: the
+// three passes wrote and read the grid twice more between them (2048^2: 16 + 10 + 16 us, here 21).
+template <int LOGN>
+__global__ void __launch_bounds__(ColTma<LOGN>::T, ColTma<LOGN>::MINB)
+    k_col_mul_tma(const __grid_constant__ TmaBatch tb, const float2 *__restrict__ tw, int r0, int r1, int *status,
+                  const float2 *__restrict__ xfr, int pitch) {
+    const CUtensorMap *tmap = &tb.map[0], *smap = &tb.map[0];
+    using S = ColTma<LOGN>;
+    constexpr int N = S::N, BOX = S::BOX, PAIRS = S::PAIRS;
+    const int xl = 4 * PAIRS * blockIdx.x;
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    unsigned char *smem_ct = smem_dyn + (256u - ((uint32_t)__cvta_generic_to_shared(smem_dyn) & 255u)) % 256u;
+    float4 *s = reinterpret_cast<float4 *>(smem_ct);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_ct + S::BYTES);
+    const uint32_t sb = (uint32_t)__cvta_generic_to_shared(s);
+    const uint32_t bb = (uint32_t)__cvta_generic_to_shared(bar);
+    const int x = xl;
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bb));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+        asm volatile("fence.proxy.async.shared::cta;");
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // boxes without a row of [r0, r1) are not loaded: the first pass reads those rows as zero
+        const int b0 = r0 / BOX, b1 = (r1 + BOX - 1) / BOX;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bb),
+                     "r"((uint32_t)(sizeof(float4) * PAIRS * BOX * (b1 - b0))));
+        for (int b = b0; b < b1; b++)
+            asm volatile(
+                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                " [%0], [%1, {%2, %3}], [%4];" ::"r"(sb + (uint32_t)(b * BOX * PAIRS * sizeof(float4))),
+                "l"(reinterpret_cast<uint64_t>(tmap)), "r"(xl), "r"(b * BOX), "r"(bb)
+                : "memory");
+    }
+    {
+        uint32_t done = 0;
+        for (int spin = 0; spin < (1 << 24) && !done; spin++) {
+            asm volatile(
+                "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;"
+                " selp.u32 %0, 1, 0, p; }"
+                : "=r"(done)
+                : "r"(bb)
+                : "memory");
+        }
+        if (!done) {
+            atomicExch(&status[STATUS_TIMEOUT], 1);
+            return;
+        }
+    }
+    const int pair = PAIRS == 1 ? 0 : (int)threadIdx.x / S::TP, tid = PAIRS == 1 ? (int)threadIdx.x : (int)threadIdx.x % S::TP;
+    St2Passes<LOGN, 0, false, S::TP, PAIRS, false>::run(s, tw, r0, r1, tid, pair, nullptr, 0);
+    // (columns beyond NU lie in the pitch; the store leaves them out)
+    const float2 *xc = xfr + 2 * (PAIRS * blockIdx.x + pair);
+#pragma unroll 8
+    for (int v = tid; v < N; v += S::TP) {
+        const float4 b = __ldg(reinterpret_cast<const float4 *>(xc + (int64_t)v * pitch));
+        const float4 a = s[pair_at<PAIRS>(v, pair)];
+        s[pair_at<PAIRS>(v, pair)] =
+            make_float4(__fsub_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)), __fadd_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x)),
+                        __fsub_rn(__fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w)), __fadd_rn(__fmul_rn(a.z, b.w), __fmul_rn(a.w, b.z)));
+    }
+    __syncthreads();
+    St2Passes<LOGN, 0, true, S::TP, PAIRS, false>::run(s, tw, 0, N, tid, pair, nullptr, 0);
+    // the last pass's generic stores must be visible to the bulk copies that read them
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < N / BOX; b++)
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                             reinterpret_cast<uint64_t>(smap)),
+                         "r"(x), "r"(b * BOX), "r"(sb + (uint32_t)(b * BOX * PAIRS * sizeof(float4)))
+                         : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+}
+
+template <int LOGN>
+cudaError_t launch_col_mul(const TmaBatch &map, int nu, const float2 *tw, int r0, int r1, const float2 *xfr, int pitch,
+                           int *status, cudaStream_t st) {
+    using S = ColTma<LOGN>;
+    cudaError_t e = cudaFuncSetAttribute(k_col_mul_tma<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e != cudaSuccess) return e;
+    k_col_mul_tma<LOGN><<<(unsigned)((nu + 2 * S::PAIRS - 1) / (2 * S::PAIRS)), S::T, S::SMEM, st>>>(map, tw, r0, r1, status,
+                                                                                                  xfr, pitch);
+    return cudaGetLastError();
+}
+
 uint32_t col_tma_pairs(int logn) { return logn == 11 ? ColTma<11>::PAIRS : logn == 12 ? ColTma<12>::PAIRS : ColTma<13>::PAIRS; }
 
 template <int LOGN>
@@ -1781,4 +1871,43 @@ int sde_grid_from_padded(sde_ctx *ctx, const float *image, int nx, int ny, int l
         return SDE_EINVAL;
     }
     return grid_from_image_at(ctx, image, nx, ny, lsx, lsy, px, py, fnu, nv, correct, grid, pitch);
+}
+
+// image_out = FFTR2D^-1(FFTR2D(image) * xfr), images w x w, transforms n x n, through mvis.  One
+// column kernel for 2048 to 8192 rows; shorter columns by the separate passes (false: not done).
+bool convolve_images(sde_ctx *ctx, const float *image, const float2 *xfr, float2 *mvis, int pitch, int w, int n,
+                     float *image_out, int *rc) {
+    const int logn = ilog2(n), nu = n / 2 + 1, ibeg = (n + 1) / 2 - (w + 1) / 2;
+    if (logn < 11 || logn > 13 || (1 << logn) != n || pitch < (nu + 3) / 4 * 4) return false;
+    auto run = [&]() -> int {
+        SDE_TRY(check_fft_args(w, w, n, n, pitch));
+        const float2 *tw;
+        SDE_TRY(ctx_twiddles(ctx, n, &tw));
+        const CorrParams cp = {nullptr, nullptr, nullptr};
+        FftBatch bt{};
+        bt.grid[0] = mvis;
+        bt.image[0] = const_cast<float *>(image);
+        cudaError_t e = cudaSuccess;
+        {
+            KTimer kt(ctx, "row_r2c");
+            r2c_t(logn - 1, bt, 1, w, w, (n - w) / 2, ibeg, tw, cp, pitch, ctx->stream, &e, ctx->d_status);
+        }
+        SDE_CUDA_TRY(e);
+        {
+            KTimer kt(ctx, "col_mul");
+            TmaBatch tb;
+            const uint32_t pairs = col_tma_pairs(logn);
+            SDE_TRY(encode_tmap_f32_2d(&tb.map[0], mvis, (uint64_t)nu * 2, (uint64_t)n, (uint64_t)pitch * 8, 4 * pairs, 256,
+                                       pairs == 2));
+            switch (logn) {
+                case 11: e = launch_col_mul<11>(tb, nu, tw, ibeg, ibeg + w, xfr, pitch, ctx->d_status, ctx->stream); break;
+                case 12: e = launch_col_mul<12>(tb, nu, tw, ibeg, ibeg + w, xfr, pitch, ctx->d_status, ctx->stream); break;
+                default: e = launch_col_mul<13>(tb, nu, tw, ibeg, ibeg + w, xfr, pitch, ctx->d_status, ctx->stream); break;
+            }
+        }
+        SDE_CUDA_TRY(e);
+        return c2r_pass(ctx, reinterpret_cast<float *>(mvis), pitch, w, w, n, n, 0, nullptr, image_out, tw);
+    };
+    *rc = run();
+    return true;
 }

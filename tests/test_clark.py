@@ -157,3 +157,27 @@ def test_gpu_long_lists_bit_exact(gpu_ctx, orc, numcl, bp, niter):
     if g["ncycles"] == o["ncycles"] == 1:
         assert np.array_equal(g["comp"], o["comp"])
         assert g["maxres"] == o["maxres"] and g["tflux"] == o["tflux"]
+
+
+# the residual's column kernel (forward, transfer function, inverse in one) at its three lengths
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2048, 4096, 8192])
+def test_gpu_residual_of_large_images(gpu_ctx, n):
+    """Residual = dirty - sum of the components' shifted PSFs, summed in 64 bits.  Three FP32
+    transforms, each within 2e-6 of its largest value (the bar of the transforms' own tests), the
+    PSF's peak being 1: 1e-5 of the components' total flux."""
+    rng = np.random.default_rng(n)
+    psf = (0.02 * rng.standard_normal((n, n), dtype=np.float32))
+    c, w = (n + 1) // 2 - 1, n // 2
+    psf[c, c] = 1.0
+    dirty = 0.05 * rng.standard_normal((n, n), dtype=np.float32)
+    lo = n // 4
+    for f, y, x in ((3.0, 5, 9), (-2.0, w - 1, 0), (2.5, w // 2, w // 3)):
+        dirty[lo + y, lo + x] += f
+    r = _gpu(gpu_ctx, dirty, psf, niter=6, gain=0.5, bpatch=64, numcl=2000)
+    a = r["aniter"] if "aniter" in r else r["trace"][-1][1]
+    assert a >= 2
+    want = dirty[lo:lo + w, lo:lo + w].astype(np.float64)
+    for f, x, y in zip(r["cl"][:a], r["cx"][:a], r["cy"][:a]):
+        want -= float(f) * psf[c - (y - 1):c - (y - 1) + w, c - (x - 1):c - (x - 1) + w]
+    assert np.abs(r["resid"] - want).max() <= 1e-5 * np.abs(r["cl"][:a]).sum()

@@ -102,3 +102,28 @@ def test_row_pairs(gpu_ctx, orc, nx, ny, n):
     scale = ctx.tensor(np.array([4.0], np.float32))
     ctx.image_from_grid(g, ctx.tensor(Xp), img, correct=False, scale_dev=scale)
     assert rel_err(img.cpu().numpy(), ref * np.float32(0.25)) < 2e-6
+
+
+# the finalize inside the register column passes: every length, images narrower than the grid
+@pytest.mark.parametrize("imsize,cell", [(64, 8.0), (100, 5.0), (500, 1.0), (1024, 0.5)])
+def test_finalize_in_short_columns(gpu_ctx, obs_small, imsize, cell):
+    """sde_plan_image against sde_plan_grid + sde_image_from_grid: the image bars of the two
+    gridding passes' FP32 rounding (1e-5 of the peak in the CLEAN window, 5e-3 at the corners)."""
+    from sde_gb300.imaging import Geom, Plan
+    ctx, torch, o = gpu_ctx, gpu_ctx.torch, obs_small
+    g = Geom(imsize, cell, vdec=o["vdec"])
+    t = {k: ctx.tensor(o[k], None) for k in ("u", "v", "w", "wt", "vis")}
+    plan = Plan(ctx, g, t["u"], t["v"], t["w"], t["vis"], t["wt"])
+    for psf in (True, False):
+        ga, gb, ia, ib = ctx.grid_buffer(g), ctx.grid_buffer(g), ctx.image_buffer(g), ctx.image_buffer(g)
+        plan.grid(ga, psf=psf)
+        ctx.image_from_grid(g, ga, ia)
+        plan.image(ib, gb, psf=psf)
+        ctx.sync()
+        a, b = ia.cpu().numpy(), ib.cpu().numpy()
+        w = slice(imsize // 4, imsize // 4 + imsize // 2 - 1)
+        pk = np.abs(a).max()
+        assert np.abs(a - b)[w, w].max() / pk < 1e-5
+        assert np.abs(a - b).max() / pk < 5e-3
+        assert float((ga - gb)[:, :g.nu].abs().max()) / float(ga.abs().max()) < 1e-5
+    plan.close()
