@@ -1894,7 +1894,7 @@ bool convolve_images(sde_ctx *ctx, const float *image, const float2 *xfr, float2
         }
         SDE_CUDA_TRY(e);
         {
-            KTimer kt(ctx, "col_mul");
+            KTimer kt(ctx, "col_fft");
             TmaBatch tb;
             const uint32_t pairs = col_tma_pairs(logn);
             SDE_TRY(encode_tmap_f32_2d(&tb.map[0], mvis, (uint64_t)nu * 2, (uint64_t)n, (uint64_t)pitch * 8, 4 * pairs, 256,
