@@ -303,8 +303,8 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
  *                  may be NULL.
  *   sde_dft_vis    IMGDFT2D (img/imgdft2d.f; task/vismodel.f:75): V_k = sum I(ix,iy) conj(E)
  *                  for WT_k > 0; other points keep their VIS.
- * images [ny][nx] float32, vis complex64 pairs, refx/refy the 1-based reference pixel (a
- * multiple of 1/2), deltx/delty degrees per pixel; nx, ny, |refx|, |refy| <= 8192.  Phases
+ * images [ny][nx] float32, vis complex64 pairs, refx/refy the 1-based reference pixel (anywhere,
+ * not only on a pixel), deltx/delty degrees per pixel; nx, ny, |refx|, |refy| <= 8192.  Phases
  * are exact to FP32 rounding (no rotation recurrence) and sums over visibilities are
  * compensated, so both are accurate to ~1e-7 of the peak. */
 int sde_dft_image(sde_ctx *ctx, int64_t nvis, const float *u, const float *v, const float *vis,

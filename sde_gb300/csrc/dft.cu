@@ -9,7 +9,9 @@
 // and output, packed FP32x2).  Phases are exact to FP32 rounding: the turns per pixel, g, are
 // split into two 8-bit heads and a tail (a head times a pixel offset of at most 16 bits is
 // exact in FP32, so is its fractional part; the tail's product is 2^-15 of the phase); the
-// reference's rotation recurrence, whose error grows along each row, is not used.  Sums over
+// reference's rotation recurrence, whose error grows along each row, is not used.  Offsets are
+// taken from the half pixel nearest the reference pixel; what is left of it, on both axes, is
+// one phase per visibility, computed in 64 bits and added to the row factor's.  Sums over
 // chunks are compensated (TwoSum).
 #include <algorithm>
 
@@ -25,7 +27,7 @@ constexpr int DTHR = 128;
 // the weights
 struct DftVis {
     float4 gx;  // h1, h2, tail, 0
-    float4 gy;
+    float4 gy;  // h1, h2, tail, turns of the reference pixel's rest on both axes (k_dft_prep)
     float4 w;   // (RNORM WT V) re, im; RNORM WT; 0     (zero for WT <= 0)
 };
 
@@ -38,25 +40,26 @@ __device__ __forceinline__ double head8(double x) {
 }
 
 // whole turns per half pixel (offsets are multiples of 1/2) change no phase
-__device__ __forceinline__ float4 split3(double g) {
+__device__ __forceinline__ float4 split3(double g, float rest) {
     g -= 2.0 * rint(0.5 * g);
     const double h1 = head8(g), r = g - h1, h2 = head8(r);
-    return make_float4((float)h1, (float)h2, (float)(r - h2), 0.f);
+    return make_float4((float)h1, (float)h2, (float)(r - h2), rest);
 }
 
-// exp(2 pi i s t), t = (h1 + h2 + l) n for a pixel offset n (|n| < 2^15, a multiple of 1/2):
+// exp(2 pi i s t), t = (h1 + h2 + l) n + t0 for a pixel offset n (|n| < 2^15, a multiple of 1/2):
 // h n is exact for both heads, so are their fractional parts (rounding to an integer by adding
-// 1.5 * 2^23; |h n| < 2^16 since split3's turns lie in [-1, 1]).  |t| <= 1 + 2^-3 or so: the
+// 1.5 * 2^23; |h n| < 2^16 since split3's turns lie in [-1, 1]).  |t| <= 1.6 or so: the
 // quarter turn nearest t is taken off exactly, and sine and cosine of the rest, |r| <= 1/8
 // turn, are polynomials in r^2 (least maximum error, fitted to the functions by iteratively
 // reweighted least squares; 3.3e-9 relative and 5e-11).  Against the functions in 64 bits the
 // result's rms error is 1.5e-8 (correctly rounded values: 1.4e-8), its largest 5.9e-8.  A
 // third of the instructions of sincospif with its own reduction of t.
-__device__ __forceinline__ float2 cis_turns(float4 g, float n, float s) {
+// (t0 = -0 adds nothing, and the compiler leaves it out.)
+__device__ __forceinline__ float2 cis_turns(float4 g, float n, float s, float t0 = -0.f) {
     constexpr float M = 12582912.f;  // 1.5 * 2^23
     const float a1 = __fsub_rn(__fmaf_rn(g.x, n, M), M), a2 = __fsub_rn(__fmaf_rn(g.y, n, M), M);
     const float f = __fadd_rn(__fmaf_rn(g.x, n, -a1), __fmaf_rn(g.y, n, -a2));
-    const float t = __fmaf_rn(g.z, n, f);
+    const float t = __fmaf_rn(g.z, n, f) + t0;
     const float qm = __fmaf_rn(t, 4.f, M);
     const int q = __float_as_int(qm);  // its low bits: the quarter turns
     const float r = __fmaf_rn(__fsub_rn(qm, M), -0.25f, t), r2 = __fmul_rn(r, r);
@@ -90,16 +93,18 @@ __global__ void k_dft_sumwt(const float *__restrict__ wt, int64_t n, double *sum
     if ((threadIdx.x & 31) == 0) atomicAdd(sum, s);
 }
 
-// CF u DX / (2 pi) = u DX pi/180 turns per pixel
+// CF u DX / (2 pi) = u DX pi/180 turns per pixel; (fx, fy): the reference pixel beyond the half
+// pixel that the offsets count from (ref_half)
 __global__ void k_dft_prep(const float *__restrict__ u, const float *__restrict__ v, const float2 *__restrict__ vis,
-                           const float *__restrict__ wt, int64_t n, double dx, double dy, const double *sumwt,
-                           DftVis *out) {
+                           const float *__restrict__ wt, int64_t n, double dx, double dy, double fx, double fy,
+                           const double *sumwt, DftVis *out) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const double d2r = 3.14159265358979323846 / 180.0;
     DftVis r;
-    r.gx = split3((double)u[k] * dx * d2r);
-    r.gy = split3((double)v[k] * dy * d2r);
+    const double gx = (double)u[k] * dx * d2r, gy = (double)v[k] * dy * d2r, rest = -(gx * fx + gy * fy);
+    r.gx = split3(gx, 0.f);
+    r.gy = split3(gy, (float)(rest - rint(rest)));
     const float w = wt ? wt[k] : 1.f;
     if (w > 0.f) {
         const float c = sumwt ? (float)((double)w / *sumwt) : 1.f;
@@ -121,7 +126,7 @@ __device__ __forceinline__ void two_sum2(float2 &hi, float2 &lo, float2 x) {
     lo = __fadd2_rn(lo, __fadd2_rn(e1, e2));
 }
 
-// VISDFT3D tile, dirty image and PSF together: the factors of a visibility (two sincospif per
+// VISDFT3D tile, dirty image and PSF together: the factors of a visibility (two cis_turns per
 // row or column) cost as much as the FMAs of 30 pixels, so one pass makes both images from
 // them.  Thread (tx, ty) of 8 x 16 owns columns 4 tx + {0..3} and 32 + 4 tx + {0..3} (a
 // quarter-warp's 16-byte reads are contiguous) of rows 4 ty + {0..3}, as column pairs.  The
@@ -168,7 +173,7 @@ __global__ void __launch_bounds__(DTHR, 2) k_dft_image(const DftVis *__restrict_
             const int k = e / DT, i = e % DT;
             const float4 gx = S.pv[buf][3 * k], gy = S.pv[buf][3 * k + 1], w = S.pv[buf][3 * k + 2];
             const float2 fx = cis_turns(gx, (float)(x0 + i + 1) - rx, -1.f);
-            const float2 c = cis_turns(gy, (float)(y0 + i + 1) - ry, -1.f);
+            const float2 c = cis_turns(gy, (float)(y0 + i + 1) - ry, -1.f, gy.w);
             const float2 fp = make_float2(w.z * c.x, w.z * c.y);
             const float2 fd = make_float2(__fsub_rn(__fmul_rn(w.x, c.x), __fmul_rn(w.y, c.y)),
                                           __fadd_rn(__fmul_rn(w.x, c.y), __fmul_rn(w.y, c.x)));
@@ -319,7 +324,7 @@ __global__ void __launch_bounds__(DTHR, R == 8 ? 2 : 3) k_dft_vis(const float *_
         for (int b = 0; b < R; b++) {
             const int row = y0 + R * tr + b;
             if (row >= ny) continue;
-            const float2 f = cis_turns(gy, (float)(row + 1) - ry, 1.f);
+            const float2 f = cis_turns(gy, (float)(row + 1) - ry, 1.f, gy.w);
             s.x = fmaf(f.x, acc[a][b].x, fmaf(-f.y, acc[a][b].y, s.x));
             s.y = fmaf(f.x, acc[a][b].y, fmaf(f.y, acc[a][b].x, s.y));
         }
@@ -361,6 +366,9 @@ int dft_rows(int ny) {
     return best;
 }
 
+// the half pixel nearest a reference pixel
+double ref_half(double ref) { return 0.5 * rint(2.0 * ref); }
+
 int fail(const char *m) {
     sde_set_error("%s", m);
     return SDE_EINVAL;
@@ -378,6 +386,7 @@ extern "C" int sde_dft_image(sde_ctx *ctx, int64_t nvis, const float *u, const f
         return fail("sde_dft_image: image over 8192 pixels or reference pixel outside +-8192");
     SDE_CUDA_TRY(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
+    const double hx = ref_half(refx), hy = ref_half(refy);
     double *sw;
     DftVis *pv;
     SDE_TRY(ctx_scratch(ctx, "dft_sumwt", sizeof(double), (void **)&sw));
@@ -385,7 +394,7 @@ extern "C" int sde_dft_image(sde_ctx *ctx, int64_t nvis, const float *u, const f
     SDE_CUDA_TRY(cudaMemsetAsync(sw, 0, sizeof(double), st));
     k_dft_sumwt<<<ctx->num_sms * 4, 256, 0, st>>>(wt, nvis, sw);
     k_dft_prep<<<(unsigned)ceil_div(nvis, (int64_t)256), 256, 0, st>>>(
-        u, v, reinterpret_cast<const float2 *>(vis), wt, nvis, deltx, delty, sw, pv);
+        u, v, reinterpret_cast<const float2 *>(vis), wt, nvis, deltx, delty, refx - hx, refy - hy, sw, pv);
     SDE_CHECK_LAUNCH();
     double h = 0.0;
     SDE_CUDA_TRY(cudaMemcpyAsync(&h, sw, sizeof h, cudaMemcpyDeviceToHost, st));
@@ -407,7 +416,7 @@ extern "C" int sde_dft_image(sde_ctx *ctx, int64_t nvis, const float *u, const f
     KTimer kt(ctx, "dft_image");
     auto kern = dirty && psf ? k_dft_image<true, true> : dirty ? k_dft_image<true, false> : k_dft_image<false, true>;
     SDE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DftTile)));
-    kern<<<grid, DTHR, sizeof(DftTile), st>>>(pv, nvis, nx, ny, (float)refx, (float)refy, kper, part, part_p);
+    kern<<<grid, DTHR, sizeof(DftTile), st>>>(pv, nvis, nx, ny, (float)hx, (float)hy, kper, part, part_p);
     SDE_CHECK_LAUNCH();
     if (dirty) k_dft_reduce<<<ctx->num_sms * 4, 256, 0, st>>>(part, nsplit, npix, dirty);
     if (psf) k_dft_reduce<<<ctx->num_sms * 4, 256, 0, st>>>(part_p, nsplit, npix, psf);
@@ -424,18 +433,19 @@ extern "C" int sde_dft_vis(sde_ctx *ctx, const float *image, int nx, int ny, dou
         return fail("sde_dft_vis: image over 8192 pixels or reference pixel outside +-8192");
     SDE_CUDA_TRY(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
+    const double hx = ref_half(refx), hy = ref_half(refy);
     DftVis *pv;
     SDE_TRY(ctx_scratch(ctx, "dft_vis", sizeof(DftVis) * (size_t)nvis, (void **)&pv));
     k_dft_prep<<<(unsigned)ceil_div(nvis, (int64_t)256), 256, 0, st>>>(u, v, nullptr, wt, nvis, deltx, delty,
-                                                                      nullptr, pv);
+                                                                      refx - hx, refy - hy, nullptr, pv);
     SDE_CHECK_LAUNCH();
     const int r = dft_rows(ny), nband = ceil_div(ny, 16 * r);
     float2 *part;
     SDE_TRY(ctx_scratch(ctx, "dft_part", sizeof(float2) * (size_t)nband * (size_t)nvis, (void **)&part));
     KTimer kt(ctx, "dft_vis");
     auto kern = r == 4 ? k_dft_vis<4> : r == 6 ? k_dft_vis<6> : k_dft_vis<8>;
-    kern<<<dim3((unsigned)ceil_div(nvis, (int64_t)DT), (unsigned)nband), DTHR, 0, st>>>(image, nx, ny, (float)refx,
-                                                                                       (float)refy, pv, nvis, part);
+    kern<<<dim3((unsigned)ceil_div(nvis, (int64_t)DT), (unsigned)nband), DTHR, 0, st>>>(image, nx, ny, (float)hx,
+                                                                                       (float)hy, pv, nvis, part);
     SDE_CHECK_LAUNCH();
     k_dft_vis_sum<<<(unsigned)ceil_div(nvis, (int64_t)256), 256, 0, st>>>(part, nband, pv, nvis,
                                                                          reinterpret_cast<float2 *>(vis));
