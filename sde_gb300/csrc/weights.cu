@@ -340,8 +340,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_sumwt_part(const uint32_t *vals
         for (int k = 0; k < per_thread; k++)
             if (base + k < nvalid) sum3(hi, mid, lo, __uint_as_float(vals[base + k]));
     }
-    // (an infinite sum leaves NaN in the error terms)
-    const double s = isinf(hi) ? (double)hi : __dadd_rn((double)hi, __dadd_rn((double)mid, (double)lo));
+    double s;
+    if (isfinite(hi)) {
+        s = __dadd_rn((double)hi, __dadd_rn((double)mid, (double)lo));
+    } else {  // weights whose sum leaves the REALs: SUMWT is DOUBLE (grd/grdruw2d.f:132-159)
+        s = 0.0;
+        for (int k = 0; k < per_thread; k++)
+            if (base + k < nvalid) s = __dadd_rn(s, (double)__uint_as_float(vals[base + k]));
+    }
     double r = block_sum_d(s);
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
