@@ -362,16 +362,16 @@ constexpr float TWOPI_R = 6.2831855f;  // TWOPI = 8 * ATAN(1.0), REAL (grd/grdh2
 // that quotient rounded to nearest (its ties to even, as W is an even number of units).  Where
 // W is a power of two and k < 0, S*W lies in the binade below, of half the spacing, and k/2
 // is exact.  The difference times TWOPI, a REAL, fits a DOUBLE, so the phase is the REAL
-// product TWOPI * (difference in units), scaled.  False for other S, and for W so small or
-// large that the scaling leaves the REALs or the phase is not below 2^-27 (where COS is 1 and
-// SIN the phase itself).
+// product TWOPI * (difference in units), scaled.  False for other S, for an infinite W or a NaN
+// (W - W is a NaN even where S is 1), and for W so small or large that the scaling leaves the
+// REALs or the phase is not below 2^-27 (where COS is 1 and SIN the phase itself).
 GEOM_HD bool tiny_phase(double s, float w, float &sn) {
     const long long ulps = d_bits(s) - 0x3FF0000000000000ll;  // 2^-52 above 1, 2^-53 below
     const long long kl = ulps > 0 ? 2 * ulps : ulps;
     sn = 0.0f;
-    if (kl == 0 || w == 0.0f) return true;
     if (kl < -8 || kl > 8) return false;
     const float aw = fabsf(w);
+    if (aw == 0.0f || (kl == 0 && aw <= 3.402823466e38f)) return true;
     if (!(aw >= 0x1p-60f && aw < 0x1p21f)) return false;
     const int k = (int)kl, b = f_bits(aw);
     const int m = (b & 0x007FFFFF) | 0x00800000;
