@@ -111,13 +111,14 @@ __device__ __forceinline__ void mos_load(const MosCol &c, float *val) {
     for (int j = 0; j < MOS_PER; j++)
         val[j] = (unsigned)(c.iy + 4 * j) < (unsigned)c.ny ? c.image[(int64_t)j * c.step] : 0.f;
 }
-// acc += wt PB I; a pixel outside the image adds a zero
+// acc += wt PB I, inside the image (a weight may be infinite or a NaN)
 __device__ __forceinline__ void mos_add(const MosCol &c, const float *val, float *acc) {
 #pragma unroll
     for (int j = 0; j < MOS_PER; j++) {
         const float dy = c.dy + (float)(4 * j);
         const float pb = expf(c.npbk * (c.dx2 + dy * dy));
-        acc[j] += c.wt * pb * val[j];
+        const float a = acc[j] + c.wt * pb * val[j];
+        acc[j] = (unsigned)(c.iy + 4 * j) < (unsigned)c.ny ? a : acc[j];
     }
 }
 
