@@ -307,6 +307,12 @@ extern "C" int sde_ctx_set_compensated(sde_ctx *c, int on) {
     return SDE_OK;
 }
 
+extern "C" int sde_ctx_set_wait_limit(sde_ctx *c, int polls) {
+    if (!c) return SDE_EINVAL;
+    c->wait_limit = polls;
+    return SDE_OK;
+}
+
 // ---------------------------------------------------------------------------------------
 // plan-level operations
 static int ensure_sums(sde_plan *pl) {

@@ -166,6 +166,7 @@ struct sde_ctx {
     int64_t nlaunch = 0;
     // gridding sums across work items with TwoSum compensation (sde_ctx_set_compensated)
     bool compensated = true;
+    int wait_limit = -1;  // polls of the device waits (sde_ctx_set_wait_limit); < 0: each one's default
     bool hogbom_cluster = false;      // k_hogbom_cluster can be resident
     int hogbom_per_sm = 0;            // resident k_hogbom CTAs per SM (queried at creation)
     const void *lo_clean = nullptr;  // compensation plane of the raw-grid scratch known to be zero

@@ -9,6 +9,7 @@
 
 constexpr unsigned long long LB_AGG = 1ull << 62, LB_PREFIX = 2ull << 62, LB_FLAGS = 3ull << 62;
 constexpr int LB_SPIN = 1 << 22;  // polls of one word before giving up (about a second)
+inline int lb_spin(const sde_ctx *ctx) { return ctx->wait_limit < 0 ? LB_SPIN : ctx->wait_limit; }
 
 __device__ __forceinline__ void lb_publish(unsigned long long *w, unsigned long long flag, unsigned long long v) {
     *reinterpret_cast<volatile unsigned long long *>(w) = flag | v;
@@ -17,13 +18,14 @@ __device__ __forceinline__ void lb_publish(unsigned long long *w, unsigned long 
 // Sum of the tiles before `tile` (one thread; the words of consecutive tiles are `stride`
 // apart).  Eight words are read at a time, in flight together (four: 2 % slower in a sort pass of
 // 64.7 million pairs, 12 % at 1.3 million).  *fail is set and 0 returned when a word does not
-// arrive.
+// arrive in `limit` polls; what was made from the sum is then wrong, and whatever reads it has to
+// look at *fail first.
 __device__ __forceinline__ unsigned long long lb_sum_before(const unsigned long long *words, int64_t tile,
-                                                            int64_t stride, unsigned long long *fail) {
+                                                            int64_t stride, unsigned long long *fail, int limit) {
     constexpr int A = 8;
     unsigned long long sum = 0;
     int64_t p = tile - 1;
-    for (int spin = 0; spin < LB_SPIN; spin++) {
+    for (int spin = 0; spin < limit; spin++) {
         unsigned long long w[A];
 #pragma unroll
         for (int a = 0; a < A; a++)
@@ -46,7 +48,8 @@ __device__ __forceinline__ unsigned long long lb_sum_before(const unsigned long 
 // tile).  Values are below 2^62 in sum (two counts of 31 bits, say).
 template <int T, int R, class In, class Out>
 __device__ __forceinline__ void lb_scan_tile(int64_t n, unsigned long long *words, uint32_t *next,
-                                             unsigned long long *total, unsigned long long *fail, In in, Out out) {
+                                             unsigned long long *total, unsigned long long *fail, int limit, In in,
+                                             Out out) {
     __shared__ unsigned long long sv[T * R * 17 / 16];  // padded: a thread reads its R consecutive items
     __shared__ unsigned long long wsum[T / 32], sbefore;
     __shared__ uint32_t stile;
@@ -85,7 +88,7 @@ __device__ __forceinline__ void lb_scan_tile(int64_t n, unsigned long long *word
         unsigned long long b = 0;
         if (tile > 0) {
             lb_publish(&words[tile], LB_AGG, all);
-            b = lb_sum_before(words, tile, 1, fail);
+            b = lb_sum_before(words, tile, 1, fail, limit);
         }
         lb_publish(&words[tile], LB_PREFIX, b + all);
         sbefore = b;

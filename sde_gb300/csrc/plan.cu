@@ -266,14 +266,22 @@ __global__ void k_exc_write(GParams p, const float *__restrict__ u, const float 
 // registers.
 constexpr int RU_T = 512, RU_R = 16;  // 8192 keys a scan tile
 __global__ void __launch_bounds__(RU_T) k_runs(const uint32_t *__restrict__ keys, PlanCounts *counts, int64_t n,
-                                               unsigned long long *words, uint32_t *rstart, uint32_t *tstart) {
+                                               unsigned long long *words, uint32_t *rstart, uint32_t *tstart,
+                                               int limit) {
     __shared__ uint32_t wsum[RU_T / 32];
     __shared__ unsigned long long before;
     __shared__ uint32_t stile;
+    __shared__ bool failed;
     const int64_t nv = (int64_t)counts->ngrid;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (t == 0) stile = atomicAdd(&counts->runs.next, 1u);
+    if (t == 0) {
+        stile = atomicAdd(&counts->runs.next, 1u);
+        failed = *(volatile unsigned long long *)&counts->fail != 0;
+    }
     __syncthreads();
+    // the sort gave up: its keys index nothing (one thread reads the word for the block, as
+    // another block's look-back may set it at any moment)
+    if (failed) return;
     const int64_t tile = stile, base = tile * (RU_T * RU_R), w0 = base + (int64_t)warp * 32 * RU_R;
     uint32_t key[RU_R], mask[RU_R];
 #pragma unroll
@@ -304,7 +312,7 @@ __global__ void __launch_bounds__(RU_T) k_runs(const uint32_t *__restrict__ keys
         unsigned long long b = 0;
         if (tile > 0) {
             lb_publish(&words[tile], LB_AGG, all);
-            b = lb_sum_before(words, tile, 1, &counts->fail);
+            b = lb_sum_before(words, tile, 1, &counts->fail, limit);
         }
         lb_publish(&words[tile], LB_PREFIX, b + all);
         before = b;
@@ -348,7 +356,8 @@ __global__ void __launch_bounds__(SC_T) k_run_emit(const uint32_t *__restrict__ 
                                                    const uint32_t *__restrict__ rstart,
                                                    const uint32_t *__restrict__ tstart, int64_t nruns,
                                                    int item_max, int chunk_max, int lbits, int jbits,
-                                                   int64_t max_items, int64_t max_chunks, unsigned long long *words,
+                                                   int64_t max_items, int64_t max_chunks, int limit,
+                                                   unsigned long long *words,
                                                    uint64_t *ckey, uint2 *craw, WorkItem *items) {
     const int64_t nvalid = (int64_t)counts->ngrid;
     auto run_end = [&](int64_t r) { return r + 1 < nruns ? (int64_t)rstart[r + 1] : nvalid; };
@@ -412,7 +421,8 @@ __global__ void __launch_bounds__(SC_T) k_run_emit(const uint32_t *__restrict__ 
             c += is_long ? (b - a + chunk_max - 1) / chunk_max : piece_chunks(k & 4094u, c, a, b, 0, 1);
         });
     };
-    lb_scan_tile<SC_T, SC_R>(nruns, words, &counts->emit.next, &counts->emit.total, &counts->fail, in, out);
+    lb_scan_tile<SC_T, SC_R>(nruns, words, &counts->emit.next, &counts->emit.total, &counts->fail, limit, in,
+                             out);
     __syncthreads();
     for (int e = threadIdx.x >> 5; e < nlong; e += SC_T / 32) {
         const LongRun r = lrun[e];
@@ -742,7 +752,8 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
         }
         if (nvis > 0) {
             PL_TRY(launch_radix_sort_u32(ctx, &keys, nullptr, &vals, nvis, kbits, ktmp, vtmp, &counts->fail));
-            k_runs<<<ceil_div(nvis, RU_T * RU_R), RU_T, 0, st>>>(keys, counts, nvis, words, rstart, tstart);
+            k_runs<<<ceil_div(nvis, RU_T * RU_R), RU_T, 0, st>>>(keys, counts, nvis, words, rstart, tstart,
+                                                                 lb_spin(ctx));
             PL_CUDA(cudaGetLastError());
         }
         // the counts and the number of runs: one wait for both
@@ -792,7 +803,7 @@ int sde_plan_create_opts(sde_ctx *ctx, const sde_gridspec *spec, int64_t nvis, c
             const int lbits = bits_for(pl->chunk_max - 1);
             k_run_emit<<<ceil_div(nruns, SC_T * SC_R), SC_T, 0, st>>>(
                 keys, counts, rstart, tstart, nruns, pl->item_max, pl->chunk_max, lbits, jbits, max_items, max_chunks,
-                words + nscan, ckey, craw, pl->items);
+                lb_spin(ctx), words + nscan, ckey, craw, pl->items);
             PL_CUDA(cudaGetLastError());
             PL_TRY(read_counts(ctx, counts, &hc));
             const int64_t nitems = (int64_t)(hc.emit.total >> 31), nchunks = (int64_t)(hc.emit.total & 0x7FFFFFFFull);

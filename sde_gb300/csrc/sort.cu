@@ -104,7 +104,7 @@ template <int T, int R>
 __global__ void __launch_bounds__(T, 3) k_rs_sweep(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                                                 uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int64_t n,
                                                 int pass, SortCtl *ctl, unsigned long long *state,
-                                                unsigned long long *fail) {
+                                                unsigned long long *fail, int limit) {
     extern __shared__ __align__(16) unsigned char rs_smem[];
     SweepSmem<T, R> &S = *reinterpret_cast<SweepSmem<T, R> *>(rs_smem);
     constexpr int TILE = T * R;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(T, 3) k_rs_sweep(const uint32_t *__restrict__ 
     if (t < 256) {
         unsigned long long before = 0;
         if (tile > 0) {
-            before = lb_sum_before(state + t, tile, 256, fail);
+            before = lb_sum_before(state + t, tile, 256, fail, limit);
             lb_publish(&state[tile * 256 + t], LB_PREFIX, before + total);
         }
         S.gbase[t] = ctl->hist[pass][t] + (uint32_t)before;
@@ -190,7 +190,8 @@ __global__ void __launch_bounds__(T, 3) k_rs_sweep(const uint32_t *__restrict__ 
         if (p < ntile) {
             const uint32_t k = S.kbuf[p];
             const uint32_t digit = (k >> shift) & 255u;
-            // (a look-back that gave up leaves a wrong position: kept inside the arrays)
+            // (a look-back that gave up leaves a wrong position, kept inside the arrays, and places
+            // that nothing is written to: the sorted arrays then hold what the scratch held)
             const uint32_t d = S.gbase[digit] + (uint32_t)p - S.dstart[digit];
             if (d < (uint64_t)n) {
                 kout[d] = k;
@@ -205,7 +206,8 @@ int sweep(sde_ctx *ctx, const uint32_t *kin, const uint32_t *vin, uint32_t *kout
           SortCtl *ctl, unsigned long long *state, unsigned long long *fail) {
     const int sm = (int)sizeof(SweepSmem<T, R>);
     SDE_CUDA_TRY(cudaFuncSetAttribute(k_rs_sweep<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    k_rs_sweep<T, R><<<ceil_div(n, T * R), T, sm, ctx->stream>>>(kin, vin, kout, vout, n, pass, ctl, state, fail);
+    k_rs_sweep<T, R><<<ceil_div(n, T * R), T, sm, ctx->stream>>>(kin, vin, kout, vout, n, pass, ctl, state, fail,
+                                                               lb_spin(ctx));
     SDE_CHECK_LAUNCH();
     return SDE_OK;
 }
@@ -215,7 +217,8 @@ int sweep(sde_ctx *ctx, const uint32_t *kin, const uint32_t *vin, uint32_t *kout
 // Sorts pairs by the low `bits` bits of the keys, stably.  *keys: the keys; first_vals: their
 // values, NULL for the items' indices; keys_tmp, *vals and vals_tmp: scratch.  On return *keys
 // and *vals are whichever of the arrays hold the result.  *fail (device, zeroed by the caller)
-// is set when a bounded wait gave up.
+// is set when a bounded wait gave up: the result then holds any keys and values at all, and a
+// kernel that uses them as indexes looks at *fail first.
 int launch_radix_sort_u32(sde_ctx *ctx, uint32_t **keys, const uint32_t *first_vals, uint32_t **vals, int64_t n,
                           int bits, uint32_t *keys_tmp, uint32_t *vals_tmp, unsigned long long *fail) {
     if (n < 1) return SDE_OK;

@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(SEG_T) k_segsum(const uint32_t *__restrict__ k
     __shared__ float sv[SEG_TILE + SEG_SHORT + SEG_U];          // vals[base ...]
     __shared__ uint16_t head[SEG_TILE];
     __shared__ int nhead;
+    if (counts[7]) return;  // the sort gave up: its keys index nothing
     const int64_t nvalid = (int64_t)counts[0];
     const int64_t base = (int64_t)blockIdx.x * SEG_TILE;
     if (base >= nvalid) return;
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(SEG_WARPS * 32) k_segsum_long(
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int PER = SEG_BLK / 32;
     __shared__ __align__(16) float buf[SEG_WARPS][SEG_RING][SEG_BLK];
+    if (counts[7]) return;  // the sort gave up
     const int64_t nvalid = (int64_t)counts[0];
     const int64_t nlong = (int64_t)counts[2];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -427,13 +429,15 @@ __device__ __forceinline__ float new_weight(const WParams &p, int robust, float 
 }
 
 // W_PER visibilities a thread: their loads, then their density reads, in flight together (64.7
-// million: one a thread 428 us, here 314).
+// million: one a thread 428 us, here 314).  When the sort gave up (*fail) there are no densities:
+// NEWWT is left alone and the context's time-out word set, for callers that read no counts.
 template <bool ROT>
 __global__ void __launch_bounds__(W_T) k_newwt(WParams p, int robust, float f2, float d2, AzParams az,
                         const float *wt, const float *__restrict__ u, const float *__restrict__ v,
                         const float *__restrict__ w, const float *__restrict__ gwt, int64_t n,
-                        float *newwt) {
+                        float *newwt, const unsigned long long *__restrict__ fail, int *status) {
     const int64_t i0 = (int64_t)blockIdx.x * (W_T * W_PER) + threadIdx.x;
+    const bool failed = *fail != 0;
     float wi[W_PER], ui[W_PER], vi[W_PER], g[W_PER], ul[W_PER], vl[W_PER];
     int uc[W_PER], vc[W_PER];
     bool on[W_PER];
@@ -451,9 +455,10 @@ __global__ void __launch_bounds__(W_T) k_newwt(WParams p, int robust, float f2, 
     }
 #pragma unroll
     for (int j = 0; j < W_PER; j++)
-        if (!(wi[j] <= 0.0f) && i0 + j * W_T < n)
+        if (!(wi[j] <= 0.0f) && i0 + j * W_T < n && !failed)
             newwt[i0 + j * W_T] = on[j] ? new_weight(p, robust, f2, d2, az, wi[j], g[j], uc[j], vc[j], ul[j], vl[j])
                                         : -1.0f;
+    if (failed && i0 == 0) atomicExch(&status[STATUS_TIMEOUT], 1);
 }
 
 int key_bits(int64_t maxkey) {
@@ -580,7 +585,7 @@ int weights_queue(sde_ctx *ctx, int rmode, const float robust[3], float ds, cons
     }
     if (nvis > 0) {
         (rot ? k_newwt<true> : k_newwt<false>)<<<ceil_div(nvis, W_T * W_PER), W_T, 0, st>>>(
-            p, robust_mode, f2, d2, az, wt, u, v, w, gwt, nvis, newwt);
+            p, robust_mode, f2, d2, az, wt, u, v, w, gwt, nvis, newwt, &counts[7], ctx->d_status);
         SDE_CHECK_LAUNCH();
     }
     if (stats) {
