@@ -171,8 +171,9 @@ int64_t sde_ctx_launches(sde_ctx *ctx);
  * No counterpart in the reference (GRDH2D sums every visibility into its cell in REAL). */
 int sde_ctx_set_compensated(sde_ctx *ctx, int on);
 
-/* Polls after which a wait of one thread block for another gives up (look-back of the sorts and
- * scans), the call then returning SDE_ETIMEDOUT, or the next sde_ctx_sync where the call itself
+/* Polls after which a wait of one thread block for others gives up (the look-back of the sorts
+ * and scans, the exchange of maxima in the CLEANs' minor cycles but for sde_hogbom's grid-wide
+ * kernel), the call then returning SDE_ETIMEDOUT, or the next sde_ctx_sync where the call itself
  * does not wait (sde_weights without stats).  < 0, the default: about a second.  Small limits
  * let a program or a test see what becomes of a device that does not answer; nothing is written
  * outside the arrays, and the context can be used afterwards.  No counterpart in the reference. */

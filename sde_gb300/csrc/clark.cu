@@ -260,7 +260,7 @@ template <bool PSF_SMEM>
 __global__ void __launch_bounds__(CL_T, 1)
     k_clark_minor(const float *__restrict__ al, const int *__restrict__ pl, ClarkState *st,
                   const float *__restrict__ psf_g, int pw, float gain, int nsub, int bsub,
-                  float flux, float *cl, int *cx, int *cy, float *comp, int logw) {
+                  float flux, float *cl, int *cx, int *cy, float *comp, int logw, int limit) {
     constexpr int C = CL_CTAS, T = CL_T;
     extern __shared__ float spsf[];
     __shared__ __align__(16) ClusterMax<C> cm;
@@ -302,7 +302,13 @@ __global__ void __launch_bounds__(CL_T, 1)
     int isub = bsub, ansub = nsub;
     const int nabs = abs(nsub);
     unsigned long long wk = 0ull;
-    bool changed = true, ok = true, gave_up = false;
+    bool changed = true, ok = true, gave_up = false, last = false;  // last: the cycle ends
+    // (the last pass, isub > nabs: pix/pix2drcc.f:133-135)
+    auto stops = [&](unsigned long long gk) {
+        const float v = key_cand(gk).v;
+        return isub > nabs || (flux < 0.f && v < 0.f) || (nsub < 0 && v < 0.f) ||
+               fabsf(v) <= fmaxf(__fmul_rn(slim, smn), fabsf(flux)) || cluster_max_aborts(gk);
+    };
     for (int n = 0;; n++) {
         if (__any_sync(0xffffffffu, changed)) {
             // |v| compared by its bits: the order of the values, a NaN above all
@@ -321,25 +327,22 @@ __global__ void __launch_bounds__(CL_T, 1)
             changed = false;
         }
         if (lane == 0) skey[warp] = wk;
-        if (__syncthreads_or(!ok)) {  // some warp's wait gave up: the whole CTA leaves
-            gave_up = true;
-            break;
-        }
+        if (__syncthreads_or(!ok || last) && cluster_max_ends(&cm, n, ok, last, gave_up, skey, stops)) break;
         if (warp == 0) {
             const unsigned long long ck = warp_key_max(lane < T / 32 ? skey[lane] : 0ull);
             if (lane < C) cluster_max_send(&cm, n, (int)rank, lane, ck);
         }
         smn = __fadd_rn(smn, __fdiv_rn(1.0f, (float)isub));
-        const unsigned long long gk = cluster_max_wait(&cm, n, ok);
+        const unsigned long long gk = cluster_max_wait(&cm, n, ok, limit);
         if (!ok) continue;
         if (t == 0) cluster_max_rearm(&cm, n);
         const Cand g = key_cand(gk);
         maxres = g.v;
-        if (isub > nabs) break;  // pix/pix2drcc.f:133-135
-        if ((flux < 0.f && maxres < 0.f) || (nsub < 0 && maxres < 0.f) ||
-            fabsf(maxres) <= fmaxf(__fmul_rn(slim, smn), fabsf(flux))) {
-            ansub = isub - 1;
-            break;
+        if (stops(gk)) {
+            if (isub <= nabs) ansub = isub - 1;
+            gave_up = cluster_max_aborts(gk);
+            last = true;
+            continue;
         }
         const float pntsub = __fmul_rn(gain, maxres);
         tflux = __fadd_rn(tflux, pntsub);
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(256) k_clark_ext(const float *__restrict__ psf
 
 int launch_minor(const float *al, const int *pl, ClarkState *dst, const float *spsf, int pw,
                     const sde_clark_params *p, int riter, float *cl, int *cx, int *cy, float *comp, int w,
-                    cudaStream_t st) {
+                    int limit, cudaStream_t st) {
     const size_t sm_psf = sizeof(float) * (size_t)pw * pw;
     const bool in_smem = sm_psf <= 200u * 1024u;
     auto *k = in_smem ? &k_clark_minor<true> : &k_clark_minor<false>;
@@ -471,7 +474,7 @@ int launch_minor(const float *al, const int *pl, ClarkState *dst, const float *s
     int logw = 0;
     while ((1 << logw) < w) logw++;
     SDE_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, al, pl, dst, spsf, pw, p->gain, p->niter, riter, p->flux, cl, cx, cy,
-                                    comp, logw));
+                                    comp, logw, limit));
     return SDE_OK;
 }
 int fail(const char *m) {
@@ -579,7 +582,8 @@ extern "C" int sde_clark(sde_ctx *ctx, const float *dirty, const float *psf, int
         {
             KTimer kt(ctx, "clark_minor");
             // TFLUX carries over the cycles in *dst (img/imgcclea.f:251)
-            SDE_TRY(launch_minor(al, pl, dst, spsf, pw, p, riter, lcl, lcx, lcy, comp, w, st));
+            SDE_TRY(launch_minor(al, pl, dst, spsf, pw, p, riter, lcl, lcx, lcy, comp, w,
+                                 cm_spin(ctx->wait_limit), st));
         }
         SDE_TRY(clark_resid(ctx, comp, drt, xfr, mvis, pitch, resid, w, n));
         SDE_CUDA_TRY(cudaMemcpyAsync(&h, dst, sizeof h, cudaMemcpyDeviceToHost, st));

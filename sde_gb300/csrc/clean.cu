@@ -116,6 +116,7 @@ struct CleanArgs {
     Barrier *bar;
     int *status;     // [STATUS_TIMEOUT]
     float *out;      // [0] maxres [1] tflux [2] ansub (as int bits)
+    int limit;       // polls of k_hogbom_cluster's and k_hogbom_regs' waits, < 0 for their own
 };
 
 // SMEM: the CTA's slice of RES lives in shared memory for all iterations (dynamic shared
@@ -378,29 +379,36 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
     float tflux = A.tflux_in, maxres = 0.f;
     const int nabs = A.nsub < 0 ? -A.nsub : A.nsub;
     const uint32_t rnx = row_recip(A.nx);
-    int isub = A.bsub, stopped = 0;
-    bool ok = true;
+    const int spins = A.limit < 0 ? CM_SPIN : A.limit;
+    int isub = A.bsub, stopped = 0, nring = 0;
+    bool ok = true, gave_up = false, last = false;  // last: the cycle ends
+    // (a key of 0: no pixel is a number, so there is nothing to subtract)
+    auto stops = [&](unsigned long long gk) {
+        const float v = key_cand(gk).v;
+        return isub > nabs || (A.nsub < 0 && v < 0.0f) || fabsf(v) <= A.flux || gk == 0ull || cluster_max_aborts(gk);
+    };
     for (int n = 0;; n++) {
         const unsigned long long wk = best();
         if (lane == 0) skey[warp] = wk;
-        if (__syncthreads_or(!ok)) {  // some warp's wait gave up: the whole CTA leaves
-            if (t == 0) atomicExch(&A.status[STATUS_TIMEOUT], 1);
-            break;
-        }
+        if (__syncthreads_or(!ok || last) && cluster_max_ends(&cm, n, ok, last, gave_up, skey, stops)) break;
         if (warp == 0) {
             const unsigned long long ck = warp_key_max(lane < T / 32 ? skey[lane] : 0ull);
             if (lane < HC_CTAS) cluster_max_send(&cm, n, (int)rank, lane, ck);
         }
-        const unsigned long long gk = cluster_max_wait(&cm, n, ok);
+        if (nring == HC_RING && !gave_up) {  // (nring is the same in all warps until a wait runs out)
+            drain(HC_RING);
+            nring = 0;
+        }
+        const unsigned long long gk = cluster_max_wait(&cm, n, ok, spins);
         if (!ok) continue;
         if (t == 0) cluster_max_rearm(&cm, n);
         const Cand g = key_cand(gk);
         maxres = g.v;
-        if (isub > nabs) break;
-        // (a key of 0: no pixel is a number, so there is nothing to subtract)
-        if ((A.nsub < 0 && maxres < 0.0f) || fabsf(maxres) <= A.flux || gk == 0ull) {
-            stopped = 1;
-            break;
+        if (stops(gk)) {
+            stopped = isub <= nabs;
+            gave_up = cluster_max_aborts(gk);
+            last = true;
+            continue;
         }
         const float pntsub = __fmul_rn(A.gain, maxres);
         tflux = __fadd_rn(tflux, pntsub);
@@ -410,7 +418,6 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
         float p[PER];
 #pragma unroll
         for (int j = 0; j < PER; j++) p[j] = __ldg(p0 + rel[j]);
-        const int nring = (isub - A.bsub) % HC_RING;
         if (t == 0) {
             ring_idx[nring] = g.idx;
             ring_f[nring] = pntsub;
@@ -426,19 +433,23 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
             r[j] = __fsub_rn(r[j], A.box ? __fmul_rn(sub, A.box[min(base + j * T + t, npix - 1)]) : sub);
         }
         isub++;
-        if (nring == HC_RING - 1) drain(HC_RING);
+        nring++;
     }
-    drain((isub - A.bsub) % HC_RING);
+    if (gave_up) {
+        if (t == 0) atomicExch(&A.status[STATUS_TIMEOUT], 1);
+    } else {
+        drain(nring);
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int k = base + j * T + t;
-        if (k < npix) A.res[k] = r[j];
-    }
-    if (rank == 0 && t == 0) {
-        A.out[0] = maxres;
-        A.out[1] = tflux;
-        A.out[2] = __int_as_float(stopped ? isub - 1 : A.nsub);
-        A.out[3] = __int_as_float(stopped);
+        for (int j = 0; j < PER; j++) {
+            const int k = base + j * T + t;
+            if (k < npix) A.res[k] = r[j];
+        }
+        if (rank == 0 && t == 0) {
+            A.out[0] = maxres;
+            A.out[1] = tflux;
+            A.out[2] = __int_as_float(stopped ? isub - 1 : A.nsub);
+            A.out[3] = __int_as_float(stopped);
+        }
     }
     // no CTA leaves while another's stores to it may be in flight
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -486,6 +497,7 @@ __global__ void __launch_bounds__(HR_T, 1) k_hogbom_regs(CleanArgs A, unsigned l
     const int nj = mine > t ? (mine - t + HR_T - 1) / HR_T : 0;     // the thread's
     const int ncta = (mine + HR_T - 1) / HR_T;                      // the CTA's largest nj
     const int nbox = (nb + HR_SHARE - 1) / HR_SHARE;
+    const int spins = A.limit < 0 ? HR_SPIN : A.limit;
     const int wrap = A.pnx - A.nx;
     const uint32_t rnx = row_recip(A.nx);
     float r[HR_PER];
@@ -565,7 +577,7 @@ __global__ void __launch_bounds__(HR_T, 1) k_hogbom_regs(CleanArgs A, unsigned l
             const unsigned long long *row = slots + ((size_t)(blockIdx.x % nbox) * 2 + (n & 1)) * HR_MAXCTAS;
             unsigned long long best = 0ull;
             bool done = false;
-            for (int spin = 0; spin < HR_SPIN && !done; spin++) {
+            for (int spin = 0; spin < spins && !done; spin++) {
                 unsigned long long k[HR_MAXCTAS / 32];
 #pragma unroll
                 for (int b = 0; b < HR_MAXCTAS / 32; b++) {
@@ -911,7 +923,7 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
     A.cx = cx; A.cy = cy; A.nx = nx; A.ny = ny; A.pnx = pnx; A.pny = pny;
     A.pmpx = A.pmpy = 0; A.gain = gain; A.flux = flux; A.tflux_in = tflux_in;
     A.nsub = nsub; A.bsub = bsub; A.cancel = cancel_flag; A.bar = nullptr;
-    A.status = ctx->d_status; A.out = dout;
+    A.status = ctx->d_status; A.out = dout; A.limit = ctx->wait_limit;
     // PSF peak (pix/pix2drcl.f:73-80)
     int64_t *psf_ip;
     SDE_TRY(isamax_dev(ctx, psf, (int64_t)pnx * pny, &psf_ip));

@@ -33,6 +33,7 @@ __device__ __forceinline__ Cand key_cand(unsigned long long k) {
 }
 
 constexpr int CM_SPIN = 1 << 20;  // polls of a cluster wait before it gives up
+inline int cm_spin(int wait_limit) { return wait_limit < 0 ? CM_SPIN : wait_limit; }
 
 __device__ __forceinline__ uint32_t cl_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -42,6 +43,16 @@ struct ClusterMax {
     unsigned long long slot[2][C];
     unsigned long long bar[2];
 };
+
+// Waits that run out.  A warp whose wait of round n runs out takes note (ok = false) and goes to the
+// top of round n + 1.  Other warps of its CTA may have had the keys in time, so between a wait and
+// the top of the next round no warp takes a CTA-wide barrier or leaves the loop; at the top the CTA
+// votes.  There the warp waits once more, as long: the other CTAs' stores to this one must land
+// before it may leave, and their keys say whether round n was the last, where all stop as they
+// would have.  If not, the CTA sends CM_ABORT in place of its key, which is above every key (|value|
+// has no sign bit): all CTAs find it in the round's maximum and stop together, with no store on
+// its way.  Only when the second wait runs out as well does a CTA leave without the others.
+constexpr unsigned long long CM_ABORT = ~0ull;
 
 template <int C>
 __device__ __forceinline__ void cluster_max_init(ClusterMax<C> *m) {
@@ -72,23 +83,47 @@ __device__ __forceinline__ void cluster_max_send(ClusterMax<C> *m, int n, int ra
                  : "memory");
 }
 
-// Called by every thread: round n's keys of all CTAs, reduced; ok is cleared when the warp's
-// wait gave up.
+// The warp's wait for round n's keys of all CTAs.
 template <int C>
-__device__ __forceinline__ unsigned long long cluster_max_wait(ClusterMax<C> *m, int n, bool &ok) {
+__device__ __forceinline__ bool cluster_max_arrived(ClusterMax<C> *m, int n, int polls) {
     const uint32_t bar = cl_smem(&m->bar[n & 1]);
     const uint32_t parity = (uint32_t)(n >> 1) & 1u;
     uint32_t done = 0;
-    for (int spin = 0; spin < CM_SPIN && !done; spin++)
+    for (int spin = 0; spin < polls && !done; spin++)
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;"
             " selp.u32 %0, 1, 0, p; }"
             : "=r"(done)
             : "r"(bar), "r"(parity)
             : "memory");
+    return __all_sync(0xffffffffu, done);
+}
+template <int C>
+__device__ __forceinline__ unsigned long long cluster_max_keys(ClusterMax<C> *m, int n, bool ok) {
     const int lane = threadIdx.x & 31;
-    ok = __all_sync(0xffffffffu, done);
     return warp_key_max(ok && lane < C ? *(volatile unsigned long long *)&m->slot[n & 1][lane] : 0ull);
+}
+// Called by every thread: round n's keys of all CTAs, reduced; ok is cleared when they were not
+// there after `limit` polls.
+template <int C>
+__device__ __forceinline__ unsigned long long cluster_max_wait(ClusterMax<C> *m, int n, bool &ok, int limit) {
+    ok = cluster_max_arrived(m, n, limit);
+    return cluster_max_keys(m, n, ok);
+}
+__device__ __forceinline__ bool cluster_max_aborts(unsigned long long key) { return (long long)key < 0; }
+
+// At the top of round n, when some warp's wait ran out or found the end: whether the CTA leaves.
+// If not, CM_ABORT is its key of the round (one of skey's, which the first warp reduces).
+// stops(key): whether a round's maximum is the last (CM_ABORT is).
+template <int C, class F>
+__device__ __forceinline__ bool cluster_max_ends(ClusterMax<C> *m, int n, bool ok, bool last, bool &gave_up,
+                                                 unsigned long long *skey, F stops) {
+    gave_up = __syncthreads_or(!ok || gave_up);
+    if (!ok) last = !cluster_max_arrived(m, n - 1, CM_SPIN) || stops(cluster_max_keys(m, n - 1, true));
+    if (__syncthreads_or(last)) return true;
+    if (threadIdx.x == 0) skey[0] = CM_ABORT;
+    __syncthreads();
+    return false;
 }
 
 // One thread, after its CTA has passed round n's wait: the barrier's next phase expects C keys.
