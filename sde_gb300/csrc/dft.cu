@@ -366,6 +366,10 @@ int dft_rows(int ny) {
     return best;
 }
 
+// bytes of the bands' shares that sde_dft_vis keeps (all of them would be 33 GB for 64.7 million
+// visibilities of an 8192-row image)
+constexpr int64_t VIS_PART = 256 << 20;
+
 // the half pixel nearest a reference pixel
 double ref_half(double ref) { return 0.5 * rint(2.0 * ref); }
 
@@ -439,16 +443,22 @@ extern "C" int sde_dft_vis(sde_ctx *ctx, const float *image, int nx, int ny, dou
     k_dft_prep<<<(unsigned)ceil_div(nvis, (int64_t)256), 256, 0, st>>>(u, v, nullptr, wt, nvis, deltx, delty,
                                                                       refx - hx, refy - hy, nullptr, pv);
     SDE_CHECK_LAUNCH();
+    // the bands' shares of a slice of visibilities at a time: a slice of VIS_PART bytes is at least
+    // 524288 visibilities (64 bands of an 8192-row image), 27 CTAs an SM and band
     const int r = dft_rows(ny), nband = ceil_div(ny, 16 * r);
+    const int64_t slice = std::min<int64_t>(nvis, VIS_PART / (int64_t)sizeof(float2) / nband / DT * DT);
     float2 *part;
-    SDE_TRY(ctx_scratch(ctx, "dft_part", sizeof(float2) * (size_t)nband * (size_t)nvis, (void **)&part));
+    SDE_TRY(ctx_scratch(ctx, "dft_part", sizeof(float2) * (size_t)nband * (size_t)slice, (void **)&part));
     KTimer kt(ctx, "dft_vis");
     auto kern = r == 4 ? k_dft_vis<4> : r == 6 ? k_dft_vis<6> : k_dft_vis<8>;
-    kern<<<dim3((unsigned)ceil_div(nvis, (int64_t)DT), (unsigned)nband), DTHR, 0, st>>>(image, nx, ny, (float)hx,
-                                                                                       (float)hy, pv, nvis, part);
-    SDE_CHECK_LAUNCH();
-    k_dft_vis_sum<<<(unsigned)ceil_div(nvis, (int64_t)256), 256, 0, st>>>(part, nband, pv, nvis,
-                                                                         reinterpret_cast<float2 *>(vis));
-    SDE_CHECK_LAUNCH();
+    for (int64_t k0 = 0; k0 < nvis; k0 += slice) {
+        const int64_t n = std::min(slice, nvis - k0);
+        kern<<<dim3((unsigned)ceil_div(n, (int64_t)DT), (unsigned)nband), DTHR, 0, st>>>(
+            image, nx, ny, (float)hx, (float)hy, pv + k0, n, part);
+        SDE_CHECK_LAUNCH();
+        k_dft_vis_sum<<<(unsigned)ceil_div(n, (int64_t)256), 256, 0, st>>>(part, nband, pv + k0, n,
+                                                                           reinterpret_cast<float2 *>(vis) + k0);
+        SDE_CHECK_LAUNCH();
+    }
     return SDE_OK;
 }
