@@ -444,7 +444,7 @@ extern "C" int sde_dft_vis(sde_ctx *ctx, const float *image, int nx, int ny, dou
                                                                       refx - hx, refy - hy, nullptr, pv);
     SDE_CHECK_LAUNCH();
     // the bands' shares of a slice of visibilities at a time: a slice of VIS_PART bytes is at least
-    // 524288 visibilities (64 bands of an 8192-row image), 27 CTAs an SM and band
+    // 524288 visibilities (64 bands of an 8192-row image), 8192 CTAs a band
     const int r = dft_rows(ny), nband = ceil_div(ny, 16 * r);
     const int64_t slice = std::min<int64_t>(nvis, VIS_PART / (int64_t)sizeof(float2) / nband / DT * DT);
     float2 *part;
