@@ -258,12 +258,13 @@ __global__ void k_dft_reduce(const float2 *__restrict__ part, int nsplit, int64_
 // of 8 x 16 owns visibilities 2 tk + {0, 1} + 16 j (a quarter-warp's 16-byte reads are
 // contiguous) and rows R tr + {0..R-1}; a column's factors are made once for all rows of the
 // band, so a taller band makes fewer, and a band too tall for the image is padding: R is
-// chosen by dft_rows.  84 240 visibilities, 300 x 277: 0.65 ms (43 TFLOP/s);
+// chosen by dft_rows.  A single band's share is V_k itself: out is then the visibilities (the sum's
+// launch is 5 us of the 33 that 1000 visibilities of 16 x 16 take).  84 240 visibilities, 300 x 277: 0.65 ms (43 TFLOP/s);
 // 4 x 4 per thread over all rows with sincospif: 1.18 ms.
 template <int R>
 __global__ void __launch_bounds__(DTHR, R == 8 ? 2 : 3) k_dft_vis(const float *__restrict__ image, int nx, int ny,
                                                                   float rx, float ry, const DftVis *__restrict__ pv,
-                                                                  int64_t nvis, float2 *part) {
+                                                                  int64_t nvis, float2 *out) {
     constexpr int RB = 16 * R;
     __shared__ __align__(16) float2 ex[DK][DT];      // [column][visibility]
     __shared__ __align__(16) float img[DK][RB + 2];  // [column][row], padded: the row-wise fill has 2-way conflicts
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(DTHR, R == 8 ? 2 : 3) k_dft_vis(const float *_
             band.x += psum[g][t].x;
             band.y += psum[g][t].y;
         }
-        part[(size_t)blockIdx.y * nvis + v0 + t] = band;
+        if (gridDim.y > 1 || pv[v0 + t].w.z > 0.f) out[(size_t)blockIdx.y * nvis + v0 + t] = band;
     }
 }
 
@@ -446,9 +447,10 @@ extern "C" int sde_dft_vis(sde_ctx *ctx, const float *image, int nx, int ny, dou
     // the bands' shares of a slice of visibilities at a time: a slice of VIS_PART bytes is at least
     // 524288 visibilities (64 bands of an 8192-row image), 8192 CTAs a band
     const int r = dft_rows(ny), nband = ceil_div(ny, 16 * r);
-    const int64_t slice = std::min<int64_t>(nvis, VIS_PART / (int64_t)sizeof(float2) / nband / DT * DT);
-    float2 *part;
-    SDE_TRY(ctx_scratch(ctx, "dft_part", sizeof(float2) * (size_t)nband * (size_t)slice, (void **)&part));
+    const int64_t slice = nband == 1 ? nvis : std::min<int64_t>(nvis, VIS_PART / (int64_t)sizeof(float2) / nband / DT * DT);
+    float2 *out = reinterpret_cast<float2 *>(vis), *part = out;
+    if (nband > 1)
+        SDE_TRY(ctx_scratch(ctx, "dft_part", sizeof(float2) * (size_t)nband * (size_t)slice, (void **)&part));
     KTimer kt(ctx, "dft_vis");
     auto kern = r == 4 ? k_dft_vis<4> : r == 6 ? k_dft_vis<6> : k_dft_vis<8>;
     for (int64_t k0 = 0; k0 < nvis; k0 += slice) {
@@ -456,8 +458,8 @@ extern "C" int sde_dft_vis(sde_ctx *ctx, const float *image, int nx, int ny, dou
         kern<<<dim3((unsigned)ceil_div(n, (int64_t)DT), (unsigned)nband), DTHR, 0, st>>>(
             image, nx, ny, (float)hx, (float)hy, pv + k0, n, part);
         SDE_CHECK_LAUNCH();
-        k_dft_vis_sum<<<(unsigned)ceil_div(n, (int64_t)256), 256, 0, st>>>(part, nband, pv + k0, n,
-                                                                           reinterpret_cast<float2 *>(vis) + k0);
+        if (nband == 1) break;
+        k_dft_vis_sum<<<(unsigned)ceil_div(n, (int64_t)256), 256, 0, st>>>(part, nband, pv + k0, n, out + k0);
         SDE_CHECK_LAUNCH();
     }
     return SDE_OK;
