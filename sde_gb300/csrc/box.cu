@@ -47,6 +47,7 @@ __global__ void k_box_grid(const float2 *__restrict__ vis, const float *__restri
             vc = __fadd_rn(-vc, (float)vorigin);
         }
         if (psf) f = make_float2(1.f, 0.f);
+        if (fabsf(uc) >= 0x1p30f || fabsf(vc) >= 0x1p30f) continue;  // no integer's cell
         const int ug = (int)lroundf(uc) + 1, vg = (int)lroundf(vc);
         if (ug < 1 || ug > nu || vg < 1 || vg > nv) continue;
         float2 *cell = raw + (size_t)(vg - 1) * nu + (ug - 1);

@@ -122,8 +122,14 @@ GEOM_HD void dsincos(double x, double *s, double *c) {
 #endif
 }
 
-// Fortran NINT of a REAL (half away from zero).
-GEOM_HD int nint_r(float x) { return (int)roundf(x); }
+// Fortran NINT of a REAL (half away from zero); 0 for a NaN, as the device's conversion gives.
+GEOM_HD int nint_r(float x) {
+#ifdef __CUDA_ARCH__
+    return (int)roundf(x);
+#else
+    return x == x ? (int)roundf(x) : 0;
+#endif
+}
 
 // Fortran NINT of a DOUBLE: floor(x + 0.5), the negative side mirrored.  x + 0.5 cannot
 // round up to the next integer for the values it is given (cells >= 1/2 or offsets that
@@ -186,13 +192,28 @@ GEOM_HD DGeo degrid_cell_r(const GParams &p, float ucell, float vcell, bool conj
     return g;
 }
 
+// The same for cells of any size.  A cell of 2^30 or more, or an infinite one, is no integer that
+// the bound tests could take (adding SUPP to the largest wraps around): the point is off the grid.
+GEOM_HD DGeo degrid_cell_any(const GParams &p, float ucell, float vcell, bool conj, float rc, float rs) {
+    if (fabsf(ucell) >= 0x1p30f || fabsf(vcell) >= 0x1p30f) {
+        DGeo g;
+        g.nud = g.nvd = g.dui = g.dvi = 0;
+        g.valid = false;
+        g.conj = conj;
+        g.rc = rc;
+        g.rs = rs;
+        return g;
+    }
+    return degrid_cell_r(p, ucell, vcell, conj, rc, rs);
+}
+
 // GRDDEH2D's per-visibility geometry (grd/grddeh2d.f:92-118) from the rotated coordinates:
 // FP32 cell, the REAL rotation (rc, rs).
 GEOM_HD DGeo degrid_cell(const GParams &p, double ul, double vl, float rc, float rs) {
     const double pu = dmul((double)p.uscale, ul);
     const float ucell = d2f(dadd(pu, (double)p.uoffset));
     const float vcell = d2f(dadd(dmul((double)p.vscale, vl), (double)p.voffset));
-    return degrid_cell_r(p, ucell, vcell, pu > 0.0, rc, rs);
+    return degrid_cell_any(p, ucell, vcell, pu > 0.0, rc, rs);
 }
 
 // The rotation ULOCAL, VLOCAL, WLOCAL = SHIFT applied to (U, V, W) in DOUBLE (GRDDEH2D
@@ -232,8 +253,8 @@ GEOM_HD DGeo degrid_geom(const GParams &p, float u, float v, float w) {
 // shift): GRDDEH2D's REAL cell SNGL(USCALE*U) is the once-rounded REAL product (the DOUBLE
 // product of two REALs is exact), its phase is 0 (COS 1, SIN 0).
 GEOM_HD DGeo degrid_geom_fast(const GParams &p, float u, float v) {
-    return degrid_cell_r(p, fmul(p.uscale, u), fmul(p.vscale, v), dmul((double)p.uscale, (double)u) > 0.0,
-                         1.0f, 0.0f);
+    return degrid_cell_any(p, fmul(p.uscale, u), fmul(p.vscale, v), dmul((double)p.uscale, (double)u) > 0.0,
+                           1.0f, 0.0f);
 }
 
 // Both routines' geometry of one visibility.

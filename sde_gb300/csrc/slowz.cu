@@ -70,6 +70,7 @@ __global__ void k_h23_grid(const float2 *__restrict__ vis, const float *__restri
             wl = -wl;
         }
         if (g.psf) f = make_float2(1.f, 0.f);
+        if (fabsf(uc) >= 0x1p30f || fabsf(vc) >= 0x1p30f) continue;  // no integer's cell
         const int nuc = (int)lroundf(uc), nvc = (int)lroundf(vc);
         if (nuc + 2 * g.suppu > g.nu || nvc + g.suppv > g.nv || nvc - g.suppv < 1) continue;
         const int delui = (int)lroundf(__fmul_rn((float)g.osampu, __fsub_rn((float)nuc, uc)));
@@ -168,11 +169,12 @@ __global__ void k_deh23(float2 *vis, float *wt, const float *__restrict__ u, con
             vc = __fadd_rn(-vc, (float)g.vorigin);
             wl = -wl;
         }
-        const int nuc = (int)lroundf(uc), nvc = (int)lroundf(vc);
+        const bool off = fabsf(uc) >= 0x1p30f || fabsf(vc) >= 0x1p30f;  // no integer's cell
+        const int nuc = off ? 0 : (int)lroundf(uc), nvc = off ? 0 : (int)lroundf(vc);
         // VIS = 0 and WT negated before the bound tests: points outside the grid end so, and
         // are not counted as failed (grd/grddeh23.f:47-49, 74-76)
         wt[k] = -wk;
-        if (nuc + g.suppu > g.nu || nvc + g.suppv > g.nv || nvc - g.suppv < 1) {
+        if (off || nuc + g.suppu > g.nu || nvc + g.suppv > g.nv || nvc - g.suppv < 1) {
             vis[k] = make_float2(0.f, 0.f);
             continue;
         }
