@@ -299,17 +299,18 @@ __global__ void __launch_bounds__(CL_T, 1)
     const float slim = st->slim;
     const int pmpx = st->pmpx, pmpy = st->pmpy;
     float tflux = st->tflux, smn = 0.f, maxres = 0.f;
-    int isub = bsub, ansub = nsub;
     const int nabs = abs(nsub);
     unsigned long long wk = 0ull;
-    bool changed = true, ok = true, gave_up = false, last = false;  // last: the cycle ends
+    bool changed = true;
+    unsigned state = 0;
     // (the last pass, isub > nabs: pix/pix2drcc.f:133-135)
-    auto stops = [&](unsigned long long gk) {
+    auto stops = [&](unsigned long long gk, int n) {
         const float v = key_cand(gk).v;
-        return isub > nabs || (flux < 0.f && v < 0.f) || (nsub < 0 && v < 0.f) ||
+        return bsub + n > nabs || (flux < 0.f && v < 0.f) || (nsub < 0 && v < 0.f) ||
                fabsf(v) <= fmaxf(__fmul_rn(slim, smn), fabsf(flux)) || cluster_max_aborts(gk);
     };
-    for (int n = 0;; n++) {
+    int n = 0;
+    for (;; n++) {
         if (__any_sync(0xffffffffu, changed)) {
             // |v| compared by its bits: the order of the values, a NaN above all
             unsigned la = 0u, lo = 0u;
@@ -327,21 +328,24 @@ __global__ void __launch_bounds__(CL_T, 1)
             changed = false;
         }
         if (lane == 0) skey[warp] = wk;
-        if (__syncthreads_or(!ok || last) && cluster_max_ends(&cm, n, ok, last, gave_up, skey, stops)) break;
+        if (__syncthreads_or(state & (CM_LATE | CM_LAST)) && cluster_max_ends(&cm, n, state, skey, stops)) break;
         if (warp == 0) {
             const unsigned long long ck = warp_key_max(lane < T / 32 ? skey[lane] : 0ull);
             if (lane < C) cluster_max_send(&cm, n, (int)rank, lane, ck);
         }
+        const int isub = bsub + n;
         smn = __fadd_rn(smn, __fdiv_rn(1.0f, (float)isub));
+        bool ok;
         const unsigned long long gk = cluster_max_wait(&cm, n, ok, limit);
-        if (!ok) continue;
+        if (!ok) {
+            state |= CM_LATE;
+            continue;
+        }
         if (t == 0) cluster_max_rearm(&cm, n);
         const Cand g = key_cand(gk);
         maxres = g.v;
-        if (stops(gk)) {
-            if (isub <= nabs) ansub = isub - 1;
-            gave_up = cluster_max_aborts(gk);
-            last = true;
+        if (stops(gk, n)) {
+            state |= cluster_max_aborts(gk) ? CM_LAST | CM_GAVE_UP : CM_LAST;
             continue;
         }
         const float pntsub = __fmul_rn(gain, maxres);
@@ -368,16 +372,16 @@ __global__ void __launch_bounds__(CL_T, 1)
                 }
             }
         }
-        isub++;
     }
-    if (gave_up) {
+    if (state & CM_GAVE_UP) {
         if (t == 0) st->err = CL_ERR_WAIT;
     } else {
 #pragma unroll
         for (int j = 0; j < CL_PER; j++)
             if (mine >> j & 1u) comp[((size_t)((q[j] >> 16) - 1) << logw) + (q[j] & 0xFFFF) - 1] = c[j];
         if (rank == 0 && t == 0) {
-            st->aniter = ansub;
+            // the loop ends one round after the one that stopped it, at isub = bsub + n - 1
+            st->aniter = bsub + n - 1 <= nabs ? bsub + n - 2 : nsub;
             st->maxres = maxres;
             st->tflux = tflux;
         }

@@ -116,7 +116,7 @@ struct CleanArgs {
     Barrier *bar;
     int *status;     // [STATUS_TIMEOUT]
     float *out;      // [0] maxres [1] tflux [2] ansub (as int bits)
-    int limit;       // polls of k_hogbom_cluster's and k_hogbom_regs' waits, < 0 for their own
+    int limit;       // polls of k_hogbom_cluster's and k_hogbom_regs' waits
 };
 
 // SMEM: the CTA's slice of RES lives in shared memory for all iterations (dynamic shared
@@ -379,35 +379,34 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
     float tflux = A.tflux_in, maxres = 0.f;
     const int nabs = A.nsub < 0 ? -A.nsub : A.nsub;
     const uint32_t rnx = row_recip(A.nx);
-    const int spins = A.limit < 0 ? CM_SPIN : A.limit;
-    int isub = A.bsub, stopped = 0, nring = 0;
-    bool ok = true, gave_up = false, last = false;  // last: the cycle ends
+    unsigned state = 0;
     // (a key of 0: no pixel is a number, so there is nothing to subtract)
-    auto stops = [&](unsigned long long gk) {
+    auto stops = [&](unsigned long long gk, int n) {
         const float v = key_cand(gk).v;
-        return isub > nabs || (A.nsub < 0 && v < 0.0f) || fabsf(v) <= A.flux || gk == 0ull || cluster_max_aborts(gk);
+        return A.bsub + n > nabs || (A.nsub < 0 && v < 0.0f) || fabsf(v) <= A.flux || gk == 0ull || cluster_max_aborts(gk);
     };
-    for (int n = 0;; n++) {
+    int n = 0;  // rounds, and the components subtracted
+    for (;; n++) {
         const unsigned long long wk = best();
         if (lane == 0) skey[warp] = wk;
-        if (__syncthreads_or(!ok || last) && cluster_max_ends(&cm, n, ok, last, gave_up, skey, stops)) break;
+        if (__syncthreads_or(state & (CM_LATE | CM_LAST)) && cluster_max_ends(&cm, n, state, skey, stops)) break;
         if (warp == 0) {
             const unsigned long long ck = warp_key_max(lane < T / 32 ? skey[lane] : 0ull);
             if (lane < HC_CTAS) cluster_max_send(&cm, n, (int)rank, lane, ck);
         }
-        if (nring == HC_RING && !gave_up) {  // (nring is the same in all warps until a wait runs out)
-            drain(HC_RING);
-            nring = 0;
+        // (after a wait that ran out the ring may lack a component)
+        if (n > 0 && n % HC_RING == 0 && !(state & CM_GAVE_UP)) drain(HC_RING);
+        bool ok;
+        const unsigned long long gk = cluster_max_wait(&cm, n, ok, A.limit);
+        if (!ok) {
+            state |= CM_LATE;
+            continue;
         }
-        const unsigned long long gk = cluster_max_wait(&cm, n, ok, spins);
-        if (!ok) continue;
         if (t == 0) cluster_max_rearm(&cm, n);
         const Cand g = key_cand(gk);
         maxres = g.v;
-        if (stops(gk)) {
-            stopped = isub <= nabs;
-            gave_up = cluster_max_aborts(gk);
-            last = true;
+        if (stops(gk, n)) {
+            state |= cluster_max_aborts(gk) ? CM_LAST | CM_GAVE_UP : CM_LAST;
             continue;
         }
         const float pntsub = __fmul_rn(A.gain, maxres);
@@ -419,12 +418,13 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
 #pragma unroll
         for (int j = 0; j < PER; j++) p[j] = __ldg(p0 + rel[j]);
         if (t == 0) {
-            ring_idx[nring] = g.idx;
-            ring_f[nring] = pntsub;
+            ring_idx[n % HC_RING] = g.idx;
+            ring_f[n % HC_RING] = pntsub;
             if (rank == 0) {
-                A.cflux[isub - 1] = pntsub;
-                A.cx[isub - 1] = gx + 1;
-                A.cy[isub - 1] = gy + 1;
+                const int c = A.bsub + n - 1;
+                A.cflux[c] = pntsub;
+                A.cx[c] = gx + 1;
+                A.cy[c] = gy + 1;
             }
         }
 #pragma unroll
@@ -432,23 +432,23 @@ __global__ void __launch_bounds__(T, 1) k_hogbom_cluster(CleanArgs A, const int6
             const float sub = __fmul_rn(pntsub, p[j]);
             r[j] = __fsub_rn(r[j], A.box ? __fmul_rn(sub, A.box[min(base + j * T + t, npix - 1)]) : sub);
         }
-        isub++;
-        nring++;
     }
-    if (gave_up) {
+    if (state & CM_GAVE_UP) {
         if (t == 0) atomicExch(&A.status[STATUS_TIMEOUT], 1);
     } else {
-        drain(nring);
+        n--;  // the loop ends one round after the one that stopped it
+        drain(n % HC_RING);
 #pragma unroll
         for (int j = 0; j < PER; j++) {
             const int k = base + j * T + t;
             if (k < npix) A.res[k] = r[j];
         }
         if (rank == 0 && t == 0) {
+            const bool stopped = A.bsub + n <= nabs;
             A.out[0] = maxres;
             A.out[1] = tflux;
-            A.out[2] = __int_as_float(stopped ? isub - 1 : A.nsub);
-            A.out[3] = __int_as_float(stopped);
+            A.out[2] = __int_as_float(stopped ? A.bsub + n - 1 : A.nsub);
+            A.out[3] = __int_as_float(stopped ? 1 : 0);
         }
     }
     // no CTA leaves while another's stores to it may be in flight
@@ -497,7 +497,6 @@ __global__ void __launch_bounds__(HR_T, 1) k_hogbom_regs(CleanArgs A, unsigned l
     const int nj = mine > t ? (mine - t + HR_T - 1) / HR_T : 0;     // the thread's
     const int ncta = (mine + HR_T - 1) / HR_T;                      // the CTA's largest nj
     const int nbox = (nb + HR_SHARE - 1) / HR_SHARE;
-    const int spins = A.limit < 0 ? HR_SPIN : A.limit;
     const int wrap = A.pnx - A.nx;
     const uint32_t rnx = row_recip(A.nx);
     float r[HR_PER];
@@ -577,7 +576,7 @@ __global__ void __launch_bounds__(HR_T, 1) k_hogbom_regs(CleanArgs A, unsigned l
             const unsigned long long *row = slots + ((size_t)(blockIdx.x % nbox) * 2 + (n & 1)) * HR_MAXCTAS;
             unsigned long long best = 0ull;
             bool done = false;
-            for (int spin = 0; spin < spins && !done; spin++) {
+            for (int spin = 0; spin < A.limit && !done; spin++) {
                 unsigned long long k[HR_MAXCTAS / 32];
 #pragma unroll
                 for (int b = 0; b < HR_MAXCTAS / 32; b++) {
@@ -923,7 +922,7 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
     A.cx = cx; A.cy = cy; A.nx = nx; A.ny = ny; A.pnx = pnx; A.pny = pny;
     A.pmpx = A.pmpy = 0; A.gain = gain; A.flux = flux; A.tflux_in = tflux_in;
     A.nsub = nsub; A.bsub = bsub; A.cancel = cancel_flag; A.bar = nullptr;
-    A.status = ctx->d_status; A.out = dout; A.limit = ctx->wait_limit;
+    A.status = ctx->d_status; A.out = dout; A.limit = cm_spin(ctx->wait_limit);
     // PSF peak (pix/pix2drcl.f:73-80)
     int64_t *psf_ip;
     SDE_TRY(isamax_dev(ctx, psf, (int64_t)pnx * pny, &psf_ip));
@@ -943,6 +942,7 @@ int sde_hogbom(sde_ctx *ctx, const float *drt, const float *psf, const float *bo
     // a window that the registers hold, rows no shorter than a thread's step, the PSF covering it
     if (!cancel_flag && nx >= HR_T && ctx->num_sms <= HR_MAXCTAS &&
         (int64_t)nx * ny <= (int64_t)ctx->num_sms * HR_T * HR_PER && psf_covers(A.pmpx, A.pmpy, nx, ny, pnx, pny)) {
+        if (ctx->wait_limit < 0) A.limit = HR_SPIN;
         unsigned long long *slots;
         SDE_TRY(ctx_scratch(ctx, "cl_slots", HR_SLOTS * sizeof(*slots), (void **)&slots));
         SDE_CUDA_TRY(cudaMemsetAsync(slots, 0, HR_SLOTS * sizeof(*slots), ctx->stream));

@@ -44,7 +44,7 @@ struct ClusterMax {
     unsigned long long bar[2];
 };
 
-// Waits that run out.  A warp whose wait of round n runs out takes note (ok = false) and goes to the
+// Waits that run out.  A warp whose wait of round n runs out takes note (CM_LATE) and goes to the
 // top of round n + 1.  Other warps of its CTA may have had the keys in time, so between a wait and
 // the top of the next round no warp takes a CTA-wide barrier or leaves the loop; at the top the CTA
 // votes.  There the warp waits once more, as long: the other CTAs' stores to this one must land
@@ -52,6 +52,9 @@ struct ClusterMax {
 // would have.  If not, the CTA sends CM_ABORT in place of its key, which is above every key (|value|
 // has no sign bit): all CTAs find it in the round's maximum and stop together, with no store on
 // its way.  Only when the second wait runs out as well does a CTA leave without the others.
+// The states share one word and the loops count in rounds alone: a register each for a flag or a
+// counter cost 1-4 % of an iteration where the residual fills the registers.
+constexpr unsigned CM_LATE = 1, CM_LAST = 2, CM_GAVE_UP = 4;  // a warp's state: see above; the loop ends; failed
 constexpr unsigned long long CM_ABORT = ~0ull;
 
 template <int C>
@@ -114,13 +117,16 @@ __device__ __forceinline__ bool cluster_max_aborts(unsigned long long key) { ret
 
 // At the top of round n, when some warp's wait ran out or found the end: whether the CTA leaves.
 // If not, CM_ABORT is its key of the round (one of skey's, which the first warp reduces).
-// stops(key): whether a round's maximum is the last (CM_ABORT is).
+// stops(key, n): whether round n's maximum is the last (CM_ABORT is).
 template <int C, class F>
-__device__ __forceinline__ bool cluster_max_ends(ClusterMax<C> *m, int n, bool ok, bool last, bool &gave_up,
-                                                 unsigned long long *skey, F stops) {
-    gave_up = __syncthreads_or(!ok || gave_up);
-    if (!ok) last = !cluster_max_arrived(m, n - 1, CM_SPIN) || stops(cluster_max_keys(m, n - 1, true));
-    if (__syncthreads_or(last)) return true;
+__device__ __forceinline__ bool cluster_max_ends(ClusterMax<C> *m, int n, unsigned &state, unsigned long long *skey,
+                                                 F stops) {
+    if (__syncthreads_or(state & (CM_LATE | CM_GAVE_UP))) state |= CM_GAVE_UP;
+    if ((state & CM_LATE) &&
+        (!cluster_max_arrived(m, n - 1, CM_SPIN) || stops(cluster_max_keys(m, n - 1, true), n - 1)))
+        state |= CM_LAST;
+    state &= ~CM_LATE;
+    if (__syncthreads_or(state & CM_LAST)) return true;
     if (threadIdx.x == 0) skey[0] = CM_ABORT;
     __syncthreads();
     return false;
